@@ -7,13 +7,11 @@
 //
 // Per problem, in the CTA's scratch slot (or, for the factor and its row
 // lists, in shared memory when they fit the launch's staging space):
-//  * the supernodal factor in the reference's BCSC layout (column-major
-//    nrow x w blocks, D as diagonal + 2x2 sub-diagonal halves), the composed
-//    ordering perm/iperm and the row lists, renamed after Bunch-Kaufman
-//    pivoting as the reference's row_reordering does (without re-sorting the
-//    renamed rows: every consumer maps them through the target's row list).
-//    Once a supernode is factored, the unit lower triangle of its diagonal
-//    block is replaced by its inverse, which is all the solves need of it;
+//  * the supernodal factor, in blocks laid out for the kernels that read them
+//    (see "blocks" below), the composed ordering perm/iperm and the row lists,
+//    renamed after Bunch-Kaufman pivoting as the reference's row_reordering
+//    does (without re-sorting the renamed rows: every consumer maps them
+//    through the target's row list);
 //  * the active set as a per-constraint flag.  Hidden (inactive) constraint
 //    columns are width-1 supernodes whose entries read as zero; the
 //    reference's hidden-column tree edits (linear_solver_wrapper.cpp:770-907)
@@ -38,68 +36,113 @@ namespace nqg {
 
 namespace {
 
-// Up to 256 threads per CTA; the kernel's natural 128 registers leave 4 CTAs
-// of 128 threads per SM.  (Capping it at 80 registers for 6 CTAs per SM was
-// measured slower: 7-12 % on cold and FP64 batches, +2 % on warm ones.)
+// Up to 256 threads per CTA at 128 registers: 4 CTAs of 128 threads per SM.
+//
+// The kernel runs a whole solver, and its size is a cost of its own: with every
+// phase inlined where it is used and loops unrolled by the compiler it was 2 MB
+// of code, 16 times what an SM's instruction cache holds, and a tenth of all
+// issue slots waited for instructions.  So a phase is one function
+// (__noinline__), and loops are unrolled only where loads have to overlap
+// (#pragma unroll with a count; unroll 1 elsewhere): 0.3 MB.
 constexpr int BT_MAX_THREADS = 256;
-constexpr int WF_WARPS = 4;  // warps of the level-parallel factorization
+constexpr int WF_WARPS = BATCH_WF_WARPS;  // warps of the level-parallel factorization
 constexpr int MR_CAP = BATCH_MR_CAP;  // Krylov steps per restart held in shared memory
-
-template <class T> struct Ctx {
-  // pattern (read-only)
-  int n, meq, mineq, N, base, ns, nlev, nnzR, cmask_ok;
-  const int *__restrict__ super, *__restrict__ sparent, *__restrict__ col2sup, *__restrict__ lpi, *__restrict__ lpx;
-  const int *__restrict__ lvl_ptr, *__restrict__ lvl_sn, *__restrict__ lev;
-  const int *__restrict__ Rp, *__restrict__ Rj, *__restrict__ Rq, *__restrict__ ent;
-  const int *__restrict__ bt_ptr, *__restrict__ bt_var, *__restrict__ bt_q, *__restrict__ bt_rpos;
-  const int *__restrict__ sn_con, *__restrict__ con_sn, *__restrict__ eq_ptr, *__restrict__ eq_var,
-      *__restrict__ eq_q;
-  const int4 *__restrict__ snrec;  // 2 per supernode: {c0, w, nrow, value offset}, {row-list offset, pairs}
-  const int4 *__restrict__ prec;   // per pair: {descendant, lb, ub, descendant's row-list offset}
-  const int *__restrict__ con_ptr, *__restrict__ con_tgt;
-  const uint8_t *__restrict__ sn_big;  // per supernode: solved by a warp (wide or tall block)
-  // problem
-  const double *__restrict__ kv, *__restrict__ q, *__restrict__ bq, *__restrict__ dq;
-  const uint8_t *__restrict__ pert;
-  double reg, reg32;
-  // slot
-  T *L, *D;
-  int *ls, *perm, *iperm, *lperm, *alist, *vlist, *mlist;
-  uint8_t *mark, *piv;
-  double *Fv, *Rv;  // factorization / refinement values of K in CSR order
-  unsigned long long *cmask;  // per supernode: active constraint-column descendants (bit = pair - pair_mid)
-  double *rhs, *sol, *r, *w, *V, *tmp;
-  T *Z;
-  // shared memory
-  int *map;
-  T *xs, *B, *rowbuf, *Dsm, *Esm, *Binv;
-  int *lp;
-  // per-warp scratch of the level-parallel factorization (WF_WARPS warps):
-  // block wcap x rcap, D, E, local pivot order, Bunch-Kaufman multipliers
-  T *wB, *wD, *wE, *wwk;
-  int *wlp;
-  int wcap, rcap;  // widest / tallest supernode a warp takes (<= 32)
-  int wf;          // level-parallel factorization on
-  uint8_t *vis;  // per supernode: visible (structural, or the column of an active constraint)
-  uint8_t *act;  // per constraint: active
-  int *vlvl;     // visible supernodes of each level: vlist[vlvl[l] .. vlvl[l+1]),
-  int *vmid;     // the small ones (a thread each) before vmid[l], the big ones (a warp each) after
-  int *vfill;    // 2 * (nlev + 1) fill counters of build_vlist
-  int *nmark;    // length of mlist
-  double *red;   // 32 doubles
-  int *redi;     // 32 ints
-  int *status;   // device status bits of this problem
-  unsigned long long *cyc;  // per-phase SM cycles of this CTA (profiling), or null
-};
 
 // Counters of nqg_batch_get_profile.
 enum { PH_TOTAL, PH_INIT, PH_FACTOR, PH_PRECOND, PH_SPMV, PH_REFINE, PH_SELECT, PH_UPDATE, PH_SN, PH_ITER,
        PH_FWD_WIDE, PH_FWD_NARROW, PH_DIAG, PH_BWD, PH_GATHER, PH_INIT_FACTOR,
        PH_SN_ASSEMBLE, PH_SN_UPDATES, PH_SN_BK, PH_SN_ROWS, PH_SN_INVERSE, PH_SN_STORE, PH_RENAME, PH_N };
+struct GmresSmall {
+  double h[MR_CAP + 1][MR_CAP], cs[MR_CAP + 1], sn[MR_CAP + 1], g[MR_CAP + 1], y[MR_CAP + 1];
+  double scal[4];
+};
+
+// An array in the CTA's dynamic shared memory, by its offset: what is read
+// through it is known to be shared (a plain pointer kept in memory is not, and
+// costs a generic access; a generic atomic is compiled for both spaces).
+template <class T> struct Sh {
+  unsigned off;
+  __device__ __forceinline__ operator T *() const {
+    extern __shared__ __align__(16) unsigned char dsm[];
+    return reinterpret_cast<T *>(dsm + off);
+  }
+  __device__ __forceinline__ Sh at(int n) const { return {off + (unsigned)(n * (int)sizeof(T))}; }
+};
+
+// The problem that the CTA works on, at the start of its dynamic shared memory.
+template <class T> struct Ctx {
+  // pattern (read-only)
+  int n, meq, mineq, N, base, ns, nlev, nnzR, cmask_ok;
+  const int *__restrict__ super, *__restrict__ sparent, *__restrict__ col2sup, *__restrict__ lpi, *__restrict__ lpx;
+  const int *__restrict__ lev;
+  const int *__restrict__ Rp, *__restrict__ Rj, *__restrict__ Rq, *__restrict__ ent;
+  const int *__restrict__ bt_ptr, *__restrict__ bt_var, *__restrict__ bt_q, *__restrict__ bt_rpos;
+  const int *__restrict__ sn_con, *__restrict__ con_sn, *__restrict__ eq_ptr, *__restrict__ eq_var,
+      *__restrict__ eq_q;
+  const int4 *__restrict__ snrec;  // 2 per supernode: {c0, w, nrow, value offset}, {row-list offset, pairs}
+  // per pair (2): {descendant's first column, width << 16 | rows, its rows inside the target, row-list offset of
+  // the first of them}, {its value offset, its Y offset (width > 1), descendant, its index in the descendant's rows}
+  const int4 *__restrict__ prec;
+  const int *__restrict__ con_ptr, *__restrict__ con_tgt;
+  // solves: the single columns that may hide or are long, by level, then up to BATCH_SN_LONG rows / longer (so_seg:
+  // 2 nlev + 1 group starts); the others (so_e); the rows and columns of the wide supernodes (see ldlt_solve_smem)
+  const int *__restrict__ so_sn, *__restrict__ so_seg;
+  const int4 *__restrict__ so_rec, *__restrict__ so_e, *__restrict__ so_f, *__restrict__ so_b;
+  const int2 *__restrict__ so_g;  // groups of 32 targets of the single columns
+  const int *__restrict__ so_gj, *__restrict__ so_gs;  // their variables, their entries' columns
+  const int *__restrict__ gidx;   // per row-list position of a single column: its entry in G, or -1
+  int n1;  // length of so_sn
+  // problem
+  const double *__restrict__ kv, *__restrict__ q, *__restrict__ bq, *__restrict__ dq;
+  const uint8_t *__restrict__ pert;
+  double reg, reg32;
+  // slot
+  T *L, *D, *S, *G;  // G: the single columns' entries by target (see gather_singles)
+  T *Di;  // D^-1 of the wide supernodes: diagonal, then the 2x2 blocks' off-diagonals (N each)
+  int *ls, *perm, *iperm, *lperm, *alist, *mlist;
+  int4 *vrec;  // so_rec of the visible single columns
+  int *arow;   // rows of the active constraints
+  uint8_t *piv;
+  T *Fv;       // factorization values of K in CSR order
+  double *Rv;  // refinement values
+  unsigned long long *cmask;  // per supernode: active constraint-column descendants (bit = pair - pair_mid)
+  double *rhs, *sol, *r, *w, *V, *tmp;
+  T *Z;
+  // shared memory
+  Sh<int> map;
+  Sh<T> xs, xo;  // vectors of the solves, in the factor's order (xo shares the row map's memory)
+  Sh<T> B, rowbuf, Dsm, Esm, Binv;
+  Sh<int> lp;
+  // per-warp scratch of the level-parallel factorization (WF_WARPS warps,
+  // wstride values each): block wcap x rcap, wcap x wcap, D, E, D^-1; pivot orders
+  Sh<T> wB;
+  Sh<int> wlp;
+  int wstride;
+  int wcap, rcap;  // widest / tallest supernode a warp takes (<= 32)
+  int wf;          // level-parallel factorization on
+  Sh<uint8_t> vis;  // per supernode: visible (structural, or the column of an active constraint)
+  Sh<uint8_t> act;  // per constraint: active
+  Sh<int> vseg;     // starts of each level's two groups in vrec (2 nlev + 1), then the length of arow
+  Sh<int4> lvl;     // per level (3): the pattern's items of the solves (see BPat)
+  Sh<uint8_t> mark;  // per supernode: to be refactored
+  int nmark;    // > 0: edits wait for a refactorization; during one, the length of mlist
+  double red[32];
+  int redi[32];
+  int status;  // device status bits of this problem
+  int prof;    // per-phase SM cycles of this CTA are counted in cyc
+  unsigned long long cyc[PH_N];
+  GmresSmall gs;
+};
+static_assert(sizeof(Ctx<double>) <= BATCH_CTX_BYTES && sizeof(Ctx<float>) <= BATCH_CTX_BYTES, "context size");
+template <class T> __device__ __forceinline__ Ctx<T> &ctx() {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  return *reinterpret_cast<Ctx<T> *>(dsm);
+}
+
 static_assert(PH_N <= BATCH_PROFILE_COUNTERS, "profile counters");
-#define BQ_T0(c) const long long t0_ = (c).cyc ? clock64() : 0
+#define BQ_T0(c) const long long t0_ = (c).prof ? clock64() : 0
 #define BQ_T1(c, ph) \
-  if ((c).cyc && threadIdx.x == 0) (c).cyc[ph] += (unsigned long long)(clock64() - t0_)
+  if ((c).prof && threadIdx.x == 0) (c).cyc[ph] += (unsigned long long)(clock64() - t0_)
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_id() { return threadIdx.x >> 5; }
@@ -107,11 +150,13 @@ __device__ __forceinline__ int num_warps() { return blockDim.x >> 5; }
 
 template <class T> __device__ __forceinline__ bool visible(const Ctx<T> &c, int s) { return c.vis[s] != 0; }
 
-// Calls f(pair) for every descendant pair of s whose descendant is visible:
-// the structural ones, then the active constraint columns (bit mask, or a
-// scan when a supernode has more than 64 of them).
-template <class T, class F> __device__ __forceinline__ void for_visible_pairs(const Ctx<T> &c, int s, int pp, int pm,
-                                                                              int pe, F &&f) {
+// Calls f(pair) for every descendant pair of s (pairs [pp, pe), constraint
+// columns from pm) whose descendant is visible: the structural ones, then the
+// active constraint columns (bit mask, or a scan when a supernode has more
+// than 64 of them).
+template <class T, class F>
+__device__ __forceinline__ void for_visible_pairs(const Ctx<T> &c, int pp, int pm, int pe, int s, F &&f) {
+#pragma unroll 1
   for (int pq = pp; pq < pm; ++pq) f(pq);
   if (c.cmask_ok) {
     unsigned long long m = c.cmask[s];
@@ -121,8 +166,9 @@ template <class T, class F> __device__ __forceinline__ void for_visible_pairs(co
       f(pm + b);
     }
   } else {
+#pragma unroll 1
     for (int pq = pm; pq < pe; ++pq)
-      if (c.vis[c.prec[pq].x]) f(pq);
+      if (c.vis[c.prec[2 * pq + 1].z]) f(pq);
   }
 }
 
@@ -244,853 +290,1338 @@ template <class T> __device__ __forceinline__ double ref_val(const Ctx<T> &c, in
   return v;
 }
 
-// Panel rows [w, nr) of the supernode block B (ld nr): columns permuted by
-// the pivot order, solved with the unit lower L11^T, scaled by D^-1 (1x1:
-// times 1/d; 2x2: Cramer's rule, the arithmetic of blocked_2by2_solver,
-// Sym_BLAS.cpp:492-529).  Warp 0, one lane per row, rows staged in rowbuf
-// (w x 32).
-template <class T> __device__ void panel_rows_warp0(Ctx<T> &c, T *B, int nr, int w, bool permute) {
-  if (warp_id() != 0) return;
-  const int lane = lane_id();
-  T *rb = c.rowbuf;
-  const T *D = c.Dsm, *E = c.Esm;
-  for (int r0 = w; r0 < nr; r0 += 32) {
-    const int r = r0 + lane;
-    if (r < nr) {
-      for (int j = 0; j < w; ++j) rb[j * 32 + lane] = B[r + (size_t)(permute ? c.lp[j] : j) * nr];
-      for (int j = 0; j < w; ++j) {
-        T x = rb[j * 32 + lane];
-        for (int t = 0; t < j; ++t) x -= rb[t * 32 + lane] * B[j + (size_t)t * nr];
-        rb[j * 32 + lane] = x;
-      }
-      for (int j = 0; j < w; ++j) {
-        if (E[j] == T(0) || j + 1 >= w) {
-          B[r + (size_t)j * nr] = rb[j * 32 + lane] * (T(1) / D[j]);
-        } else {
-          const T e = E[j];
-          const T inv = T(1) / (D[j] * D[j + 1] - e * e);
-          const T x1 = rb[j * 32 + lane], x2 = rb[(j + 1) * 32 + lane];
-          B[r + (size_t)j * nr] = (x1 * D[j + 1] - x2 * e) * inv;
-          B[r + (size_t)(j + 1) * nr] = (x2 * D[j] - x1 * e) * inv;
-          ++j;
-        }
-      }
-    }
-  }
-  __syncwarp();
+// ---- blocks ------------------------------------------------------------------
+// A supernode of one column keeps [1/d; L21] in c.L.  Those of at most 32 rows
+// that never hide are stored 32 at a time, entry r of 32 neighbours (in the
+// order the solves take them) side by side, values and row list alike
+// (stride 32): a warp of the solves, a lane per supernode, reads them in whole
+// lines.  A wider supernode keeps in c.S, by rows of w4 = s_ld(w) values:
+//   R = [L11^-1; L21]   nrow rows, for the solves (their forward sums run along
+//                       a row, 16 bytes a load; the backward ones across rows,
+//                       a lane per column) and, from row w on, for the updates;
+//   Y = L21 D           m = nrow - w rows: an update is L21 Y^T, without a
+//                       pivot block in sight.
+__host__ __device__ __forceinline__ int s_ld(int w) { return (w + 3) & ~3; }
+// supernode record: rows, and the stride of its values and row list
+__device__ __forceinline__ int sn_rows(const int4 &r0) { return r0.z & 0xffff; }
+__device__ __forceinline__ int sn_stride(const int4 &r0) { return r0.z >> 16 ? 32 : 1; }
+
+// Four consecutive values from a multiple of four values into a block.
+[[maybe_unused]] __device__ __forceinline__ void load4(const float *p, float (&v)[4]) {
+  const float4 f = *reinterpret_cast<const float4 *>(p);
+  v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+}
+[[maybe_unused]] __device__ __forceinline__ void load4(const double *p, double (&v)[4]) {
+  const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
+  v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
 }
 
-// Subtracts descendant d's L D L^T restricted to target s (rows lb.. of d,
-// columns lb..ub) from the staged target block B.  One warp per pair; pairs
-// of different warps may hit the same entries, so the subtraction is atomic
-// (the summation order of a target entry varies between runs, as in the
-// reference's threaded factorization).
-template <class T> __device__ void sub_update_warp(Ctx<T> &c, int pq, int d, int c0, int w, int nr, const int *rows) {
-  const int lane = lane_id();
-  const int4 pr = c.prec[pq], d0 = c.snrec[2 * d];
-  const int lb = pr.y, ub = pr.z;
-  const int cd = d0.x, wd = d0.y, nrd = d0.z;
-  const int *rd = c.ls + pr.w;
-  const T *Ld = c.L + d0.w;
-  const T *Dd = c.D + cd, *Ed = c.D + c.N + cd;
-  const int m = nrd - lb, nc = ub - lb + 1;
-  T *B = c.B;
-  // lanes over the descendant's rows (each lane's target row found once),
-  // the target columns in turn; the products accumulate in the factor's
-  // precision, in the order of the descendant's columns
-  for (int i0 = 0; i0 < m; i0 += 32) {
-    const int i = i0 + lane;
-    int ti = -1;
-    if (i < m) {
-      const int ri = rd[lb + i];
-      ti = c.map[ri];
-      if (ti < 0 || ti >= nr || rows[ti] != ri) {
-        atomicOr(c.status, ST_BOUNDS);
-        ti = -1;
-      }
-    }
-    for (int jj = 0; jj < nc; ++jj) {
-      const int tj = rd[lb + jj] - c0;
-      if (tj < 0 || tj >= w) {
-        if (lane == 0) atomicOr(c.status, ST_BOUNDS);
-        continue;
-      }
-      if (ti < tj) continue;  // lower triangle of the target only (and rows out of bounds)
-      T acc = T(0);
-      for (int k = 0; k < wd; ++k) {
-        const T lik = Ld[lb + i + (size_t)k * nrd];
-        const T ek = Ed[k];
-        if (ek == T(0) || k + 1 >= wd) {
-          acc += lik * Dd[k] * Ld[lb + jj + (size_t)k * nrd];
-        } else {
-          // 2x2 block (k, k+1): (D L^T)_k,j = d1 L_jk + e L_j,k+1; (D L^T)_k+1,j = e L_jk + d2 L_j,k+1
-          const T ljk = Ld[lb + jj + (size_t)k * nrd], ljk1 = Ld[lb + jj + (size_t)(k + 1) * nrd];
-          const T lik1 = Ld[lb + i + (size_t)(k + 1) * nrd];
-          acc += lik * (Dd[k] * ljk + ek * ljk1) + lik1 * (ek * ljk + Dd[k + 1] * ljk1);
-          ++k;
-        }
-      }
-      atomicAdd(&B[ti + tj * nr], -acc);
-    }
-  }
-}
+constexpr int LD_BATCH = 8;  // loads in flight per lane
 
 // Warp-wide argmax of |value| with the smallest index winning ties (the
-// LAPACK idamax convention); every lane returns the winner.
-template <class T> __device__ __forceinline__ void warp_argmax(T &v, int &idx) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const T ov = __shfl_xor_sync(0xffffffffu, v, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    if (oi >= 0 && (idx < 0 || ov > v || (ov == v && oi < idx))) {
-      v = ov;
-      idx = oi;
-    }
-  }
+// LAPACK idamax convention) over the lanes that have one (idx >= 0, rising
+// with the lane); every lane returns the winner.  The bits of a non-negative
+// floating-point number order like an integer: two integer reductions and a
+// vote instead of a tree of compares (an FP64 compare holds the FP64 pipe of
+// the SM quarter for 64 cycles).
+[[maybe_unused]] __device__ __forceinline__ void warp_argmax(float &v, int &idx) {
+  const unsigned FULL = 0xffffffffu;
+  const unsigned key = idx >= 0 ? __float_as_uint(v) + 1u : 0u;
+  const unsigned best = __reduce_max_sync(FULL, key);
+  const unsigned who = __ballot_sync(FULL, best && key == best);
+  const int src = who ? __ffs(who) - 1 : 0;
+  v = __shfl_sync(FULL, v, src);
+  idx = best ? __shfl_sync(FULL, idx, src) : -1;
+}
+[[maybe_unused]] __device__ __forceinline__ void warp_argmax(double &v, int &idx) {
+  const unsigned FULL = 0xffffffffu;
+  const bool has = idx >= 0;
+  const unsigned hi = has ? (unsigned)__double2hiint(v) + 1u : 0u;
+  const unsigned bh = __reduce_max_sync(FULL, hi);
+  const bool top = has && hi == bh;
+  const unsigned lo = top ? (unsigned)__double2loint(v) : 0u;
+  const unsigned bl = __reduce_max_sync(FULL, lo);
+  const unsigned who = __ballot_sync(FULL, top && lo == bl);
+  const int src = who ? __ffs(who) - 1 : 0;
+  v = __shfl_sync(FULL, v, src);
+  idx = bh ? __shfl_sync(FULL, idx, src) : -1;
 }
 
-template <class T> __device__ __forceinline__ void s_flag_store(Ctx<T> &c, bool f) { c.redi[31] = f ? 1 : 0; }
+// Lanes (rows of 32, two rows deep) to one candidate each: the larger, the
+// smaller index on ties.
+template <class T> __device__ __forceinline__ void take_larger(T &v, int &i, T v2, int i2) {
+  if (i2 >= 0 && (i < 0 || v2 > v)) {
+    v = v2;
+    i = i2;
+  }
+}
 
 // Bunch-Kaufman (alpha = (1+sqrt(17))/8, the LAPACK dsytf2('L') pivot rule
 // and the reference's reorder_after_sytrf form: explicit interchanges, L with
 // unit diagonal, D / E the diagonal and 2x2 sub-diagonals, perm[m] = original
-// local column at position m) on a w <= 32 wide lower-stored block, by one
-// warp: the steps and the arithmetic of each entry are those of the CTA-wide
-// bk_factor.  wk holds the multipliers of a step (w - 1 of a 1x1, 2 (w - 2) of a
-// 2x2).  Returns whether
-// any interchange happened.
+// local column at position m) on a lower-stored block of at most 64 columns.
+// Every warp of the group finds the pivot by itself from the shared block (no
+// broadcast to wait for), and the trailing columns are dealt to the warps, a
+// lane per row.  wi of nw: this warp's place in the group that calls together;
+// nw = 1 synchronizes the warp only.  Returns whether any interchange happened.
+// A 22-column FP64 block took about 100k cycles by one warp whose lanes walked
+// their rows' columns one after another (w^2 / 2 multiply-adds of 64 cycles).
 template <class T>
-__device__ bool bk_factor_warp(T *a, int lda, int w, T *D, T *E, int *perm, int *status, T *wk) {
+__device__ __noinline__ bool bk_block(Sh<T> a_, int lda, int w, Sh<T> D_, Sh<T> E_, Sh<int> perm_, int wi, int nw) {
+  T *a = a_, *D = D_, *E = E_;
+  int *perm = perm_, *status = &ctx<T>().status;
+  const unsigned FULL = 0xffffffffu;
   const T alpha = (T)((1.0 + sqrt(17.0)) / 8.0);
   const int lane = lane_id();
+  auto sync = [&]() {
+    if (nw > 1) __syncthreads();
+    else __syncwarp();
+  };
   bool pivoted = false;
-  for (int m = lane; m < w; m += 32) perm[m] = m;
-  __syncwarp();
+  if (wi == 0)
+#pragma unroll 1
+    for (int m = lane; m < w; m += 32) perm[m] = m;
   int k = 0;
   while (k < w) {
-    const T absakk = tabs(a[k + (size_t)k * lda]);
-    T cv = T(-1);
-    int ci = -1;
-    for (int i = k + 1 + lane; i < w; i += 32) {
-      const T v = tabs(a[i + (size_t)k * lda]);
-      if (ci < 0 || v > cv) {
-        cv = v;
-        ci = i;
-      }
-    }
+    const T akk = a[k + k * lda], absakk = tabs(akk);
+    // rows k+1+lane and k+33+lane of column k
+    const int i0 = k + 1 + lane, i1 = i0 + 32;
+    T c0 = i0 < w ? a[i0 + k * lda] : T(0), c1 = i1 < w ? a[i1 + k * lda] : T(0);
+    T cv = tabs(c0);
+    int ci = i0 < w ? i0 : -1;
     warp_argmax(cv, ci);
+    if (w - k > 33) {
+      T v2 = tabs(c1);
+      int j2 = i1 < w ? i1 : -1;
+      warp_argmax(v2, j2);
+      take_larger(cv, ci, v2, j2);
+    }
     const T colmax = ci >= 0 ? cv : T(0);
     const int imax = ci;
     int kp = k, kstep = 1, zero = 0;
     if ((absakk >= colmax ? absakk : colmax) == T(0) || absakk != absakk) {
       zero = 1;
-    } else if (absakk >= alpha * colmax) {
-      kp = k;
-    } else {
+    } else if (!(absakk >= alpha * colmax)) {
       T rv = T(-1);
       int ri = -1;
-      for (int j = k + lane; j < w; j += 32) {
-        if (j == imax) continue;
-        const T v = j < imax ? tabs(a[imax + (size_t)j * lda]) : tabs(a[j + (size_t)imax * lda]);
-        if (ri < 0 || v > rv) {
-          rv = v;
-          ri = j;
-        }
+#pragma unroll 1
+      for (int b = k; b < w; b += 32) {
+        const int j = b + lane;
+        int jj = j < w && j != imax ? j : -1;
+        T v = jj < 0 ? T(0) : (j < imax ? tabs(a[imax + j * lda]) : tabs(a[j + imax * lda]));
+        warp_argmax(v, jj);
+        take_larger(rv, ri, v, jj);
       }
-      warp_argmax(rv, ri);
       const T rowmax = rv;
-      if (absakk >= alpha * colmax * (colmax / rowmax)) {
-        kp = k;
-      } else if (tabs(a[imax + (size_t)imax * lda]) >= alpha * rowmax) {
+      if (!(absakk >= alpha * colmax * (colmax / rowmax))) {
         kp = imax;
-      } else {
-        kp = imax;
-        kstep = 2;
+        if (!(tabs(a[imax + imax * lda]) >= alpha * rowmax)) kstep = 2;
       }
     }
     const int kk = k + kstep - 1;
-    if (zero && lane == 0) atomicOr(status, absakk == absakk ? ST_ZERO_PIVOT : ST_NONFINITE);
-    if (kp != kk) {  // symmetric interchange of kk and kp (kp > kk)
+    if (zero && wi == 0 && lane == 0) atomicOr(status, absakk == absakk ? ST_ZERO_PIVOT : ST_NONFINITE);
+    sync();
+    if (kp != kk) {  // symmetric interchange of kk and kp (kp > kk), by the first warp
       pivoted = true;
-      for (int i = kp + 1 + lane; i < w; i += 32) {
-        const T t = a[i + (size_t)kk * lda];
-        a[i + (size_t)kk * lda] = a[i + (size_t)kp * lda];
-        a[i + (size_t)kp * lda] = t;
-      }
-      for (int j = kk + 1 + lane; j < kp; j += 32) {
-        const T t = a[j + (size_t)kk * lda];
-        a[j + (size_t)kk * lda] = a[kp + (size_t)j * lda];
-        a[kp + (size_t)j * lda] = t;
-      }
-      const int ncols_left = kstep == 2 ? k + 1 : k;
-      for (int cc = lane; cc < ncols_left; cc += 32) {
-        const T t = a[kk + (size_t)cc * lda];
-        a[kk + (size_t)cc * lda] = a[kp + (size_t)cc * lda];
-        a[kp + (size_t)cc * lda] = t;
-      }
-      if (lane == 0) {
-        const T t = a[kk + (size_t)kk * lda];
-        a[kk + (size_t)kk * lda] = a[kp + (size_t)kp * lda];
-        a[kp + (size_t)kp * lda] = t;
-        const int pt = perm[kk];
-        perm[kk] = perm[kp];
-        perm[kp] = pt;
-      }
-    }
-    __syncwarp();
-    if (kstep == 1) {
-      if (!zero) {
-        const T r1 = T(1) / a[k + (size_t)k * lda];
-        // trailing update of the lower triangle: lane owns row i = k + 1 + lane
-        // (w <= 32) and walks its columns j <= i, independent updates; the
-        // multipliers r1 a_jk are staged once per column
-        for (int j = k + 1 + lane; j < w; j += 32) wk[j] = r1 * a[j + (size_t)k * lda];
-        __syncwarp();
-        {
-          const int i = k + 1 + lane;
-          if (i < w) {
-            const T aik = a[i + (size_t)k * lda];
-            for (int j = k + 1; j <= i; ++j) a[i + (size_t)j * lda] -= wk[j] * aik;
-          }
+      if (wi == 0) {
+#pragma unroll 1
+        for (int i = kp + 1 + lane; i < w; i += 32) {
+          const T t = a[i + kk * lda];
+          a[i + kk * lda] = a[i + kp * lda];
+          a[i + kp * lda] = t;
         }
-        __syncwarp();
-        for (int i = k + 1 + lane; i < w; i += 32) a[i + (size_t)k * lda] *= r1;
+#pragma unroll 1
+        for (int j = kk + 1 + lane; j < kp; j += 32) {
+          const T t = a[j + kk * lda];
+          a[j + kk * lda] = a[kp + j * lda];
+          a[kp + j * lda] = t;
+        }
+        const int ncols_left = kstep == 2 ? k + 1 : k;
+#pragma unroll 1
+        for (int cc = lane; cc < ncols_left; cc += 32) {
+          const T t = a[kk + cc * lda];
+          a[kk + cc * lda] = a[kp + cc * lda];
+          a[kp + cc * lda] = t;
+        }
+        if (lane == 0) {
+          const T t = a[kk + kk * lda];
+          a[kk + kk * lda] = a[kp + kp * lda];
+          a[kp + kp * lda] = t;
+          const int pt = perm[kk];
+          perm[kk] = perm[kp];
+          perm[kp] = pt;
+        }
       }
-      if (lane == 0) {
-        D[k] = a[k + (size_t)k * lda];
+      sync();
+    }
+    if (kstep == 1) {
+      const T d = kp != kk ? a[k + k * lda] : akk;
+      if (kp != kk) {
+        c0 = i0 < w ? a[i0 + k * lda] : T(0);
+        c1 = i1 < w ? a[i1 + k * lda] : T(0);
+      }
+      if (!zero) {
+        const T r1 = T(1) / d;
+        const T m0 = r1 * c0;  // multipliers, row i0 (and i1)
+        T m1 = T(0);
+        if (w - k > 33) m1 = r1 * c1;
+        // column j by warp (j - k - 1) mod nw: rows i >= j, four columns at a time
+#pragma unroll 1
+        for (int j = k + 1 + wi; j < w; j += 4 * nw) {
+          T v[4], mj[4];
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            const int jj = j + h * nw, q = jj - k - 1;
+            v[h] = i0 >= jj && i0 < w ? a[i0 + jj * lda] : T(0);
+            mj[h] = q < 32 ? __shfl_sync(FULL, m0, q & 31) : __shfl_sync(FULL, m1, q & 31);
+          }
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            const int jj = j + h * nw;
+            if (jj < w) v[h] -= mj[h] * c0;
+            if (i0 >= jj && i0 < w) a[i0 + jj * lda] = v[h];
+          }
+          if (w - k > 33)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+              const int jj = j + h * nw;
+              if (i1 >= jj && i1 < w) a[i1 + jj * lda] -= mj[h] * c1;
+            }
+        }
+        sync();  // every warp has read column k
+        if (wi == 0) {
+          if (i0 < w) a[i0 + k * lda] = m0;
+          if (i1 < w) a[i1 + k * lda] = m1;
+        }
+      }
+      if (wi == 0 && lane == 0) {
+        D[k] = d;
         E[k] = T(0);
       }
     } else {
       // 2x2 pivot on rows/cols k, k+1
-      T d21 = a[k + 1 + (size_t)k * lda];
-      const T d11 = a[k + 1 + (size_t)(k + 1) * lda] / d21;
-      const T d22 = a[k + (size_t)k * lda] / d21;
-      const T t = T(1) / (d11 * d22 - T(1));
-      d21 = t / d21;
-      const int m = w - k - 2;
-      for (int q = lane; q < m; q += 32) {
-        const int j = k + 2 + q;
-        const T ajk = a[j + (size_t)k * lda], ajk1 = a[j + (size_t)(k + 1) * lda];
-        wk[2 * q] = d21 * (d11 * ajk - ajk1);
-        wk[2 * q + 1] = d21 * (d22 * ajk1 - ajk);
+      const T a11 = a[k + k * lda], a21 = a[k + 1 + k * lda], a22 = a[k + 1 + (k + 1) * lda];
+      const T i21 = T(1) / a21;
+      const T d11 = a22 * i21, d22 = a11 * i21;
+      const T d21 = (T(1) / (d11 * d22 - T(1))) * i21;
+      const int p0 = k + 2 + lane, p1 = p0 + 32;
+      T x0 = T(0), y0 = T(0), x1 = T(0), y1 = T(0);
+      if (p0 < w) {
+        x0 = a[p0 + k * lda];
+        y0 = a[p0 + (k + 1) * lda];
       }
-      __syncwarp();
-      {
-        // lane owns row i = k + 2 + lane (w <= 32), independent updates over its columns
-        const int i = k + 2 + lane;
-        if (i < w) {
-          const T aik = a[i + (size_t)k * lda], aik1 = a[i + (size_t)(k + 1) * lda];
-          for (int q = 0; q <= i - k - 2; ++q)
-            a[i + (size_t)(k + 2 + q) * lda] -= aik * wk[2 * q] + aik1 * wk[2 * q + 1];
+      if (p1 < w) {
+        x1 = a[p1 + k * lda];
+        y1 = a[p1 + (k + 1) * lda];
+      }
+      const T u0 = d21 * (d11 * x0 - y0), v0 = d21 * (d22 * y0 - x0);
+      T u1 = T(0), v1 = T(0);
+      if (w - k > 34) {
+        u1 = d21 * (d11 * x1 - y1);
+        v1 = d21 * (d22 * y1 - x1);
+      }
+#pragma unroll 2
+      for (int j = k + 2 + wi; j < w; j += nw) {
+        const int q = j - k - 2;
+        const T uj = q < 32 ? __shfl_sync(FULL, u0, q & 31) : __shfl_sync(FULL, u1, q & 31);
+        const T vj = q < 32 ? __shfl_sync(FULL, v0, q & 31) : __shfl_sync(FULL, v1, q & 31);
+        if (p0 >= j && p0 < w) a[p0 + j * lda] -= x0 * uj + y0 * vj;
+        if (w - k > 34 && p1 >= j && p1 < w) a[p1 + j * lda] -= x1 * uj + y1 * vj;
+      }
+      sync();
+      if (wi == 0) {
+        if (p0 < w) {
+          a[p0 + k * lda] = u0;
+          a[p0 + (k + 1) * lda] = v0;
+        }
+        if (p1 < w) {
+          a[p1 + k * lda] = u1;
+          a[p1 + (k + 1) * lda] = v1;
+        }
+        if (lane == 0) {
+          D[k] = a11;
+          D[k + 1] = a22;
+          E[k] = a21;
+          E[k + 1] = T(0);
+          a[k + 1 + k * lda] = T(0);
         }
       }
-      __syncwarp();
-      for (int q = lane; q < m; q += 32) {
-        const int j = k + 2 + q;
-        a[j + (size_t)k * lda] = wk[2 * q];
-        a[j + (size_t)(k + 1) * lda] = wk[2 * q + 1];
-      }
-      __syncwarp();
-      if (lane == 0) {
-        D[k] = a[k + (size_t)k * lda];
-        D[k + 1] = a[k + 1 + (size_t)(k + 1) * lda];
-        E[k] = a[k + 1 + (size_t)k * lda];
-        E[k + 1] = T(0);
-        a[k + 1 + (size_t)k * lda] = T(0);
-      }
     }
-    __syncwarp();
+    sync();
     k += kstep;
   }
-  for (int m = lane; m < w; m += 32) a[m + (size_t)m * lda] = T(1);
-  __syncwarp();
+  if (wi == 0)
+#pragma unroll 1
+    for (int m = lane; m < w; m += 32) a[m + m * lda] = T(1);
+  sync();
   return pivoted;
 }
 
-// ---- factorization of one supernode (CTA scope) ------------------------------
+// D^-1 of a block as diagonal and 2x2 off-diagonal: entry m of both (D, E: the
+// w diagonals and 2x2 sub-diagonals; 2x2 pivots by Cramer's rule, the
+// arithmetic of blocked_2by2_solver, Sym_BLAS.cpp:492-529).
+template <class T>
+__device__ __forceinline__ void d_inverse(const T *D, const T *E, int w, int m, T &inv, T &off) {
+  const bool first = m + 1 < w && E[m] != T(0), second = m > 0 && E[m - 1] != T(0);
+  off = T(0);
+  if (first || second) {
+    const int k = second ? m - 1 : m;
+    const T e = E[k], det = T(1) / (D[k] * D[k + 1] - e * e);
+    inv = det * D[second ? k : k + 1];
+    if (first) off = -e * det;
+  } else {
+    inv = T(1) / D[m];
+  }
+}
+
+[[maybe_unused]] __device__ __forceinline__ bool finite_bits(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+[[maybe_unused]] __device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+template <class T> __device__ __forceinline__ void check_finite(Ctx<T> &c, T v) {
+  if (!finite_bits(v)) atomicOr(&c.status, ST_NONFINITE);
+}
+
+// Updates of target s from its visible descendants: the staged target block
+// B (nr x w, rows found by pos(row)) loses L_d[rows] Y_d[rows in s]^T of every
+// one (single columns: Y = d L).  Entries of a pair go to lanes one each, so
+// that all lanes work whatever the pair's shape; small pairs are dealt to the
+// warps in turn, large ones shared by all of them (wi of nw warps call).
+// Pairs of different warps may hit the same entry: the subtraction is atomic
+// when nw > 1 (the summation order varies between runs, as in the
+// reference's threaded factorization).
+template <class T, class F>
+__device__ __forceinline__ void sn_updates(Ctx<T> &c, int s, int c0, int w, int nr, int pp, int pm, int pe, T *B,
+                                           int wi, int nw, F &&pos) {
+  const int lane = lane_id();
+  int t = 0;
+  for_visible_pairs(c, pp, pm, pe, s, [&](int pq) {
+    const int4 ra = c.prec[2 * pq], rb = c.prec[2 * pq + 1];
+    const int wd = (int)((unsigned)ra.y >> 16), nc = ra.z, md = (ra.y & 0xffff) - rb.w;
+    const int total = md * nc;
+    int e0 = lane, step = 32;
+    if (nw > 1) {
+      if (total <= 128) {
+        if (t++ % nw != wi) return;
+      } else {
+        e0 += 32 * wi;
+        step *= nw;
+      }
+    }
+    // wd 0, 1: a single column (stride 32, 1)
+    const int st = wd == 0 ? 32 : 1, ld = s_ld(wd);
+    const int *rd = c.ls + ra.w;  // descendant's rows from its first one inside s
+    const T *Li = (wd < 2 ? c.L : c.S) + rb.x;  // its L21 from that row
+    const T *Yj = c.S + rb.y;                   // its Y from that row (wd > 1)
+    const T d1 = wd < 2 ? c.D[ra.x] : T(0);
+#pragma unroll 1
+    for (int eb = e0 - lane; eb < total; eb += step) {
+      const int e = eb + lane;
+      const int jj = e / md, i = e - jj * md;
+      int ti = -1, tj = 0;
+      if (e < total) {
+        tj = rd[jj * st] - c0;
+        ti = pos(rd[i * st]);
+        if (ti < 0 || tj < 0 || tj >= w) {
+          atomicOr(&c.status, ST_BOUNDS);
+          ti = -1;
+        }
+      }
+      if (e >= total || ti < tj) continue;  // lower triangle of the target only
+      T acc = T(0);
+      if (wd < 2) {
+        acc = Li[i * st] * (d1 * Li[jj * st]);
+      } else {
+        const T *li = Li + i * ld, *yj = Yj + jj * ld;
+#pragma unroll 2
+        for (int k0 = 0; k0 < wd; k0 += 4) {
+          T l[4], y[4];
+          load4(li + k0, l);
+          load4(yj + k0, y);
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (k0 + q < wd) acc += l[q] * y[q];
+        }
+      }
+      if (nw > 1) atomicAdd(&B[ti + tj * nr], -acc);
+      else B[ti + tj * nr] -= acc;
+    }
+    if (nw == 1) __syncwarp();
+  });
+}
+
+// ---- factorization of one single-column supernode (warp scope) ----------------
+// The left-looking step of the reference (Serial_update_ldl.cpp:62-190) for a
+// column of at most 32 rows, a lane per row: most supernodes of a KKT tree.
+// Warp wi has 32 values of the row scratch and byte wi of every word of the row map.
+template <class T> __device__ __noinline__ void factor_single(Ctx<T> &, int s, int wi) {
+  Ctx<T> &c = ctx<T>();
+  T *b = c.rowbuf + 32 * wi;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = lane_id();
+  if (c.prof && lane == 0) atomicAdd(&c.cyc[PH_SN], 1ull);
+  const int4 r0 = c.snrec[2 * s], r1 = c.snrec[2 * s + 1];
+  const int c0 = r0.x, nr = sn_rows(r0), ss = sn_stride(r0);
+  const int *rows = c.ls + r1.x;
+  uint8_t *map8 = Sh<uint8_t>{c.map.off};
+  const int myrow = lane < nr ? rows[lane * ss] : -1;
+  if (lane < nr) map8[4 * myrow + wi] = (uint8_t)lane;
+  b[lane] = T(0);
+  __syncwarp();
+  // every lane calls; -1: not in the row list
+  auto find = [&](int r) {
+    const int p = r >= 0 ? map8[4 * r + wi] & 31 : 0;
+    return __shfl_sync(FULL, myrow, p) == r && p < nr ? p : -1;
+  };
+  const int j = c.perm[c0], qb = c.Rp[j], qe = c.Rp[j + 1];
+#pragma unroll 1
+  for (int q0 = qb; q0 < qe; q0 += 32) {
+    const int qq = q0 + lane;
+    const int oi = qq < qe ? c.iperm[c.Rj[qq]] : -1;
+    const T v = qq < qe ? c.Fv[qq] : T(0);
+    const int p = find(oi);
+    if (oi >= c0) {
+      if (p < 0) atomicOr(&c.status, ST_BOUNDS);  // not in the row list: corrupted structure
+      else b[p] = v;
+    }
+  }
+  __syncwarp();
+  for_visible_pairs(c, r1.y, r1.z, r1.w, s, [&](int pq) {
+    const int4 ra = c.prec[2 * pq], rb = c.prec[2 * pq + 1];
+    const int wd = (int)((unsigned)ra.y >> 16), md = (ra.y & 0xffff) - rb.w;
+    const int st = wd == 0 ? 32 : 1, ld = s_ld(wd);
+    const int *rd = c.ls + ra.w;
+    const T *Li = (wd < 2 ? c.L : c.S) + rb.x, *y = c.S + rb.y;
+#pragma unroll 1
+    for (int i0 = 0; i0 < md; i0 += 32) {
+      const int i = i0 + lane;
+      const int p = find(i < md ? rd[i * st] : -1);
+      if (i < md) {
+        T acc = T(0);
+        if (wd < 2) {
+          acc = Li[i * st] * (c.D[ra.x] * Li[0]);
+        } else {
+#pragma unroll 1
+          for (int k = 0; k < wd; ++k) acc += Li[i * ld + k] * y[k];
+        }
+        if (p < 0) atomicOr(&c.status, ST_BOUNDS);
+        else b[p] -= acc;
+      }
+    }
+    __syncwarp();
+  });
+  const T v = b[lane], d = __shfl_sync(FULL, v, 0);
+  const T inv = T(1) / d;
+  if (lane == 0 && !(tabs(d) > T(0))) atomicOr(&c.status, d == T(0) ? ST_ZERO_PIVOT : ST_NONFINITE);
+  if (lane < nr) {
+    const T l = lane ? v * inv : inv;
+    check_finite(c, l);
+    c.L[r0.w + lane * ss] = l;
+    const int g = ss == 32 ? c.gidx[r1.x + lane * 32] : -1;
+    if (g >= 0) c.G[g] = l;
+  }
+  if (lane == 0) {
+    c.D[c0] = d;
+    c.lperm[c0] = 0;
+    c.piv[s] = 0;
+  }
+  __syncwarp();
+}
+
+// ---- factorization of one supernode -------------------------------------------
 // Left-looking step of the reference (Serial_update_ldl.cpp:62-190): scatter
 // the matrix columns, subtract every visible descendant's L D L^T restricted
-// to the supernode, Bunch-Kaufman on the diagonal block, permute / solve /
-// scale the rows below.
-template <class T> __device__ void factor_sn(Ctx<T> &c, int s) {
+// to the supernode, Bunch-Kaufman on the diagonal block, then the rows below
+// permuted and solved with the unit L11^T.  The rows of the identity go along
+// (their solutions are the columns of L11^-1).  The blocks stay in factored
+// form: A11^-1 and L21 L11^-1 as such would make every solve a single product,
+// but pivots as small as the 1e-9 regularization leave them with errors that
+// the refinement then needs three times the steps for (measured).
+//
+// wi of nw warps call with the same scratch: the whole CTA (nw > 1, barriers)
+// or one warp (nw = 1).  B: nr x w, I: w x w, dv: 2 w values (D^-1).
+template <class T, bool CTA, class F>
+__device__ __forceinline__ void sn_finish(Ctx<T> &c, int s, int c0, int w, int nr, const int4 &r0, T *B, T *I, T *D,
+                                          T *E, int *lp, T *dv, bool pivoted, int tid, int nt, F &&lap) {
+  auto sync = [&]() {
+    if (CTA) __syncthreads();
+    else __syncwarp();
+  };
+  const int m = nr - w;
+  // a lane keeps its row: R of them, the other index over nt / R
+  int R = 32;
+  while (R < nt && R < nr) R *= 2;
+  const int rr = tid & (R - 1), cq = tid / R, cs = nt / R;
+  if (pivoted) {  // columns of the rows below into pivot order (cycles, in place)
+#pragma unroll 1
+    for (int r = w + tid; r < nr; r += nt) {
+      T *br = B + r;
+#pragma unroll 1
+      for (int j0 = 0; j0 < w; ++j0) {
+        int q = lp[j0], g = 0;
+        while (q > j0 && g++ < w) q = lp[q];
+        if (q != j0 || lp[j0] == j0) continue;  // the smallest index of a cycle turns it
+        const T first = br[j0 * nr];
+        int j = j0;
+#pragma unroll 1
+        for (g = 0; g < w; ++g) {
+          const int src = lp[j];
+          br[j * nr] = src == j0 ? first : br[src * nr];
+          if (src == j0) break;
+          j = src;
+        }
+      }
+    }
+  }
+#pragma unroll 1
+  for (int j = cq; j < w; j += cs)
+#pragma unroll 1
+    for (int r = rr; r < w; r += R) I[r + j * w] = r == j ? T(1) : T(0);
+  if (tid < w) {
+    T inv, off;
+    d_inverse(D, E, w, tid, inv, off);
+    dv[tid] = inv;
+    dv[w + tid] = off;
+  }
+#pragma unroll 1
+  for (int k = tid + nt; k < w; k += nt) {
+    T inv, off;
+    d_inverse(D, E, w, k, inv, off);
+    dv[k] = inv;
+    dv[w + k] = off;
+  }
+  sync();
+  // V L11^T = [I; A21]: column j is final, the later ones lose x_j L11(t, j)
+  // (each entry receives its terms in increasing j, as in the substitution)
+#pragma unroll 1
+  for (int j = 0; j + 1 < w; ++j) {
+    const T *Lj = B + j * nr;
+#pragma unroll 1
+    for (int r = rr; r < nr; r += R) {
+      if (r < w && r > j) continue;  // still zero
+      T *vr = r < w ? I + r : B + r;
+      const int ld = r < w ? w : nr;
+      const T xj = vr[j * ld];
+      int t = j + 1 + cq;
+#pragma unroll 1
+      for (; t + 3 * cs < w; t += 4 * cs) {
+        const T l0 = Lj[t], l1 = Lj[t + cs], l2 = Lj[t + 2 * cs], l3 = Lj[t + 3 * cs];
+        const T v0 = vr[t * ld], v1 = vr[(t + cs) * ld], v2 = vr[(t + 2 * cs) * ld], v3 = vr[(t + 3 * cs) * ld];
+        vr[t * ld] = v0 - xj * l0;
+        vr[(t + cs) * ld] = v1 - xj * l1;
+        vr[(t + 2 * cs) * ld] = v2 - xj * l2;
+        vr[(t + 3 * cs) * ld] = v3 - xj * l3;
+      }
+#pragma unroll 1
+      for (; t < w; t += cs) vr[t * ld] -= xj * Lj[t];
+    }
+    if (CTA && cs > 1) __syncthreads();
+    // a row's columns all belong to its lane otherwise
+  }
+  sync();
+  lap(PH_SN_ROWS);
+  // out: L11^-1 by rows (I(r, k) = L11^-1(k, r)), Y as it stands, L21 = Y D^-1
+  const int w4 = s_ld(w);
+  T *Rb = c.S + r0.w, *Yb = Rb + nr * w4;
+#pragma unroll 1
+  for (int e = tid; e < w * w4; e += nt) {
+    const int i = e / w4, j = e - i * w4;
+    const T v = j < w ? I[j + i * w] : T(0);
+    check_finite(c, v);
+    Rb[e] = v;
+  }
+#pragma unroll 1
+  for (int e = tid; e < m * w4; e += nt) {
+    const int r = w + e / w4, j = e % w4;
+    T y = T(0), v = T(0);
+    if (j < w) {
+      y = B[r + j * nr];
+      v = y * dv[j];
+      if (dv[w + j] != T(0)) v += dv[w + j] * B[r + (j + 1) * nr];
+      if (j > 0 && dv[w + j - 1] != T(0)) v += dv[w + j - 1] * B[r + (j - 1) * nr];
+      check_finite(c, v);
+    }
+    Yb[e] = y;
+    Rb[w * w4 + e] = v;
+  }
+#pragma unroll 1
+  for (int k = tid; k < w; k += nt) {
+    check_finite(c, dv[k]);
+    c.D[c0 + k] = D[k];
+    c.Di[c0 + k] = dv[k];
+    c.Di[c.N + c0 + k] = dv[w + k];
+    c.lperm[c0 + k] = lp[k];
+  }
+  if (tid == 0) c.piv[s] = pivoted ? 1 : 0;
+  sync();
+  lap(PH_SN_STORE);
+}
+
+// By the whole CTA.
+template <class T> __device__ __noinline__ void factor_sn(Ctx<T> &, int s) {
+  Ctx<T> &c = ctx<T>();
   const int tid = threadIdx.x, nt = blockDim.x;
-  if (c.cyc && tid == 0) c.cyc[PH_SN] += 1;
+  if (c.prof && tid == 0) c.cyc[PH_SN] += 1;
   const int4 r0 = c.snrec[2 * s], r1 = c.snrec[2 * s + 1];
-  const int c0 = r0.x, w = r0.y, nr = r0.z;
+  const int c0 = r0.x, w = r0.y, nr = sn_rows(r0);
   const int *rows = c.ls + r1.x;
   T *B = c.B;
-  long long tq = c.cyc ? clock64() : 0;
+  long long tq = c.prof ? clock64() : 0;
   auto lap = [&](int ph) {
-    if (c.cyc && tid == 0) {
+    if (c.prof && tid == 0) {
       const long long now = clock64();
       c.cyc[ph] += (unsigned long long)(now - tq);
       tq = now;
     }
   };
+#pragma unroll 1
   for (int p = tid; p < nr; p += nt) c.map[rows[p]] = p;
+#pragma unroll 1
   for (int e = tid; e < nr * w; e += nt) B[e] = T(0);
   __syncthreads();
   // matrix columns (symmetric neighbours of the original column, ordered >=
   // the column): g threads per column, all columns at once
   const int g = w < nt ? nt / w : 1;
+#pragma unroll 1
   for (int t = tid; t < w * g; t += nt) {
     const int m = t % w, k0 = t / w;
     const int col = c0 + m;
     const int j = c.perm[col];
+#pragma unroll 1
     for (int qq = c.Rp[j] + k0; qq < c.Rp[j + 1]; qq += g) {
       const int oi = c.iperm[c.Rj[qq]];
       if (oi < col) continue;
       const int pos = c.map[oi];
       if (pos < 0 || pos >= nr || rows[pos] != oi) {  // not in the row list: corrupted structure
-        atomicOr(c.status, ST_BOUNDS);
+        atomicOr(&c.status, ST_BOUNDS);
         continue;
       }
-      B[pos + m * nr] = T(c.Fv[qq]);
+      B[pos + m * nr] = c.Fv[qq];
     }
   }
   __syncthreads();
   lap(PH_SN_ASSEMBLE);
-  // descendant updates: descendants that never hide, then the active
-  // constraint columns; warp wi takes every num_warps()-th of them
-  {
-    int t = 0;
-    const int wi = warp_id(), nw = num_warps();
-    for_visible_pairs(c, s, r1.y, r1.z, r1.w, [&](int pq) {
-      if (t++ % nw == wi) sub_update_warp(c, pq, c.prec[pq].x, c0, w, nr, rows);
-    });
-  }
+  sn_updates(c, s, c0, w, nr, r1.y, r1.z, r1.w, B, warp_id(), num_warps(), [&](int r) {
+    const int p = c.map[r];
+    return p >= 0 && p < nr && rows[p] == r ? p : -1;
+  });
   __syncthreads();
   lap(PH_SN_UPDATES);
-  // Bunch-Kaufman on the diagonal block (one warp up to 32 columns), then the rows below
-  bool pivoted = false;
-  if (w <= 32) {
-    if (warp_id() == 0) {
-      const bool pv = bk_factor_warp<T>(B, nr, w, c.Dsm, c.Esm, c.lp, c.status, c.rowbuf);
-      if (lane_id() == 0) s_flag_store(c, pv);
+  if (w == 1) {  // a column of more than 32 rows
+    const T d = B[0], inv = T(1) / d;
+    if (tid == 0) {
+      if (!(tabs(d) > T(0))) atomicOr(&c.status, d == T(0) ? ST_ZERO_PIVOT : ST_NONFINITE);
+      c.D[c0] = d;
+      c.lperm[c0] = 0;
+      c.piv[s] = 0;
+    }
+#pragma unroll 1
+    for (int r = tid; r < nr; r += nt) {
+      const T l = r ? B[r] * inv : inv;
+      check_finite(c, l);
+      c.L[r0.w + r] = l;
     }
     __syncthreads();
-    pivoted = c.redi[31] != 0;
-    __syncthreads();
-  } else {
-    bk_factor<T>(B, nr, w, c.Dsm, c.Esm, c.lp, c.status, &pivoted);
+    lap(PH_SN_STORE);
+    return;
   }
+  bool pivoted = false;
+  if (w <= 64) pivoted = bk_block<T>(c.B, nr, w, c.Dsm, c.Esm, c.lp, warp_id(), num_warps());
+  else bk_factor<T>(B, nr, w, c.Dsm, c.Esm, c.lp, &c.status, &pivoted);
   __syncthreads();
   lap(PH_SN_BK);
-  if (nr > w) panel_rows_warp0(c, B, nr, w, pivoted);
-  __syncthreads();
-  lap(PH_SN_ROWS);
-  // The solves apply the diagonal block through the inverse of its unit
-  // lower triangle (one product instead of w dependent steps); nothing else
-  // reads L11 once the rows below are solved, so the inverse replaces it.
-  // Column j of the inverse by thread j: X[i][j] = -sum_{j<=k<i} L[i][k] X[k][j].
-  for (int j = tid; j < w; j += nt) {
-    T *X = c.Binv;
-    X[j + j * w] = T(1);
-    for (int i = j + 1; i < w; ++i) {
-      T acc = B[i + (size_t)j * nr];
-      for (int k = j + 1; k < i; ++k) acc += B[i + (size_t)k * nr] * X[k + j * w];
-      X[i + j * w] = -acc;
-    }
-  }
-  __syncthreads();
-  for (int e = tid; e < w * w; e += nt) {
-    const int i = e % w, j = e / w;
-    if (i > j) B[i + (size_t)j * nr] = c.Binv[i + j * w];
-  }
-  __syncthreads();
-  lap(PH_SN_INVERSE);
-  T *Ls = c.L + r0.w;
-  for (int e = tid; e < nr * w; e += nt) {
-    T v = B[e];
-    if (!(v == v) || isinf((double)v)) atomicOr(c.status, ST_NONFINITE);
-    Ls[e] = v;
-  }
-  for (int m = tid; m < w; m += nt) {
-    c.D[c0 + m] = c.Dsm[m];
-    c.D[c.N + c0 + m] = c.Esm[m];
-    c.lperm[c0 + m] = c.lp[m];
-  }
-  if (tid == 0) c.piv[s] = pivoted ? 1 : 0;
-  __syncthreads();
-  lap(PH_SN_STORE);
+  sn_finish<T, true>(c, s, c0, w, nr, r0, B, c.Binv, c.Dsm, c.Esm, c.lp, c.rowbuf, pivoted, tid, nt, lap);
 }
 
-// ---- factorization of one supernode (warp scope) -----------------------------
-// The steps and the per-entry arithmetic of factor_sn for a supernode of at
-// most wcap columns and rcap rows (both <= 32), by warp wi in its own
-// scratch: target rows found by a search of the row list held one per lane,
-// descendant updates applied in list order (no atomics), the rows below
-// permuted in place along the cycles of the pivot order, and the inverse of
-// the unit L11 formed in the block's upper triangle (zero otherwise) before
-// it replaces L11.
-template <class T> __device__ void factor_sn_warp(Ctx<T> &c, int s, int wi) {
-  const unsigned FULL = 0xffffffffu;
+// By warp wi alone, in its own scratch: a supernode of at most wcap columns
+// and rcap rows (both <= 32).
+template <class T> __device__ __noinline__ void factor_sn_warp(Ctx<T> &, int s, int wi) {
+  Ctx<T> &c = ctx<T>();
   const int lane = lane_id();
-  if (c.cyc && lane == 0) atomicAdd(&c.cyc[PH_SN], 1ull);
+  if (c.prof && lane == 0) atomicAdd(&c.cyc[PH_SN], 1ull);
   const int4 r0 = c.snrec[2 * s], r1 = c.snrec[2 * s + 1];
-  const int c0 = r0.x, w = r0.y, nr = r0.z;
+  const int c0 = r0.x, w = r0.y, nr = sn_rows(r0);
   const int *rows = c.ls + r1.x;
-  T *B = c.wB + (size_t)wi * c.wcap * c.rcap;
-  T *Dw = c.wD + wi * c.wcap, *Ew = c.wE + wi * c.wcap, *wk = c.wwk + wi * 64;
-  int *lpw = c.wlp + wi * c.wcap;
+  const Sh<T> sB = c.wB.at(wi * c.wstride), sD = sB.at(c.wcap * (c.rcap + c.wcap)), sE = sD.at(c.wcap);
+  const Sh<int> slp = c.wlp.at(wi * c.wcap);
+  T *B = sB, *I = B + c.wcap * c.rcap, *Dw = sD, *Ew = sE, *dv = Ew + c.wcap;
+  int *lpw = slp;
+  uint8_t *map8 = Sh<uint8_t>{c.map.off};
   const int myrow = lane < nr ? rows[lane] : -1;
-  // position of row r in the row list, -1 when absent (every lane calls)
-  auto find = [&](int r) {
-    int pos = -1;
-    for (int k = 0; k < nr; ++k)
-      if (__shfl_sync(FULL, myrow, k) == r) pos = k;
-    return pos;
-  };
+  if (lane < nr) map8[4 * myrow + wi] = (uint8_t)lane;
+#pragma unroll 1
   for (int e = lane; e < nr * w; e += 32) B[e] = T(0);
   __syncwarp();
-  // matrix columns (entries of rows >= the column)
+  // matrix columns (entries of rows >= the column), one lane per entry
+#pragma unroll 1
   for (int m = 0; m < w; ++m) {
     const int col = c0 + m, j = c.perm[col];
     const int qb = c.Rp[j], qe = c.Rp[j + 1];
-    for (int q0 = qb; q0 < qe; q0 += 32) {
-      const int qq = q0 + lane;
-      const int oi = qq < qe ? c.iperm[c.Rj[qq]] : -1;
-      const int pos = find(oi);
-      if (qq < qe && oi >= col) {
-        if (pos < 0) atomicOr(c.status, ST_BOUNDS);  // not in the row list: corrupted structure
-        else B[pos + m * nr] = T(c.Fv[qq]);
-      }
+#pragma unroll 1
+    for (int qq = qb + lane; qq < qe; qq += 32) {
+      const int oi = c.iperm[c.Rj[qq]];
+      if (oi < col) continue;
+      const int p = map8[4 * oi + wi];
+      if (p >= nr || rows[p] != oi) atomicOr(&c.status, ST_BOUNDS);  // not in the row list: corrupted structure
+      else B[p + m * nr] = c.Fv[qq];
     }
   }
   __syncwarp();
-  // descendant updates (sub_update_warp's arithmetic, one pair after another)
-  for_visible_pairs(c, s, r1.y, r1.z, r1.w, [&](int pq) {
-    const int4 pr = c.prec[pq], d0 = c.snrec[2 * pr.x];
-    const int lb = pr.y, ub = pr.z;
-    const int cd = d0.x, wd = d0.y, nrd = d0.z;
-    const int *rd = c.ls + pr.w;
-    const T *Ld = c.L + d0.w;
-    const T *Dd = c.D + cd, *Ed = c.D + c.N + cd;
-    const int md = nrd - lb, nc = ub - lb + 1;
-    for (int i0 = 0; i0 < md; i0 += 32) {
-      const int i = i0 + lane;
-      const int ri = i < md ? rd[lb + i] : -1;
-      int ti = find(ri);
-      if (i < md && ti < 0) atomicOr(c.status, ST_BOUNDS);
-      for (int jj = 0; jj < nc; ++jj) {
-        const int tj = rd[lb + jj] - c0;
-        if (tj < 0 || tj >= w) {
-          if (lane == 0) atomicOr(c.status, ST_BOUNDS);
-          continue;
-        }
-        if (ti < tj) continue;  // lower triangle of the target only (and absent rows)
-        T acc = T(0);
-        for (int k = 0; k < wd; ++k) {
-          const T lik = Ld[lb + i + (size_t)k * nrd];
-          const T ek = Ed[k];
-          if (ek == T(0) || k + 1 >= wd) {
-            acc += lik * Dd[k] * Ld[lb + jj + (size_t)k * nrd];
-          } else {
-            const T ljk = Ld[lb + jj + (size_t)k * nrd], ljk1 = Ld[lb + jj + (size_t)(k + 1) * nrd];
-            const T lik1 = Ld[lb + i + (size_t)(k + 1) * nrd];
-            acc += lik * (Dd[k] * ljk + ek * ljk1) + lik1 * (ek * ljk + Dd[k + 1] * ljk1);
-            ++k;
-          }
-        }
-        B[ti + tj * nr] -= acc;
-      }
-    }
-    __syncwarp();
+  sn_updates(c, s, c0, w, nr, r1.y, r1.z, r1.w, B, 0, 1, [&](int r) {
+    const int p = map8[4 * r + wi];
+    return p < nr && rows[p] == r ? p : -1;
   });
-  const bool pivoted = bk_factor_warp<T>(B, nr, w, Dw, Ew, lpw, c.status, wk);
-  // rows below: lane owns row r; new column j takes old column lpw[j]
-  // (cycles of the pivot order, in place), solve with the unit L11^T, scale
-  // by D^-1 (panel_rows_warp0's arithmetic)
-  for (int rb0 = w; rb0 < nr; rb0 += 32) {
-    const int r = rb0 + lane;
-    if (r < nr) {
-      T *br = B + r;
-      if (pivoted) {
-        unsigned done = 0u;
-        for (int j0 = 0; j0 < w; ++j0) {
-          if ((done >> j0) & 1u) continue;
-          const T first = br[(size_t)j0 * nr];
-          int j = j0;
-          for (int guard = 0; guard < w; ++guard) {
-            done |= 1u << j;
-            const int src = lpw[j];
-            if (src == j0 || src < 0 || src >= w) {
-              br[(size_t)j * nr] = first;
-              break;
-            }
-            br[(size_t)j * nr] = br[(size_t)src * nr];
-            j = src;
-          }
-        }
-      }
-      for (int j = 0; j < w; ++j) {
-        T x = br[(size_t)j * nr];
-        for (int t = 0; t < j; ++t) x -= br[(size_t)t * nr] * B[j + (size_t)t * nr];
-        br[(size_t)j * nr] = x;
-      }
-      for (int j = 0; j < w; ++j) {
-        if (Ew[j] == T(0) || j + 1 >= w) {
-          br[(size_t)j * nr] = br[(size_t)j * nr] * (T(1) / Dw[j]);
-        } else {
-          const T e = Ew[j];
-          const T inv = T(1) / (Dw[j] * Dw[j + 1] - e * e);
-          const T x1 = br[(size_t)j * nr], x2 = br[(size_t)(j + 1) * nr];
-          br[(size_t)j * nr] = (x1 * Dw[j + 1] - x2 * e) * inv;
-          br[(size_t)(j + 1) * nr] = (x2 * Dw[j] - x1 * e) * inv;
-          ++j;
-        }
-      }
-    }
-  }
-  __syncwarp();
-  // inverse of the unit L11: X(i, j), i > j, at B[j + i nr] (lane j owns row j
-  // of the upper triangle), then moved below the diagonal
-  if (lane < w) {
-    const int j = lane;
-    for (int i = j + 1; i < w; ++i) {
-      T acc = B[i + (size_t)j * nr];
-      for (int k = j + 1; k < i; ++k) acc += B[i + (size_t)k * nr] * B[j + (size_t)k * nr];
-      B[j + (size_t)i * nr] = -acc;
-    }
-  }
-  __syncwarp();
-  for (int e = lane; e < w * w; e += 32) {
-    const int i = e % w, j = e / w;
-    if (i > j) B[i + (size_t)j * nr] = B[j + (size_t)i * nr];
-  }
-  __syncwarp();
-  for (int e = lane; e < w * w; e += 32) {
-    const int i = e % w, j = e / w;
-    if (i > j) B[j + (size_t)i * nr] = T(0);
-  }
-  __syncwarp();
-  T *Ls = c.L + r0.w;
-  for (int e = lane; e < nr * w; e += 32) {
-    const T v = B[e];
-    if (!(v == v) || isinf((double)v)) atomicOr(c.status, ST_NONFINITE);
-    Ls[e] = v;
-  }
-  for (int m = lane; m < w; m += 32) {
-    c.D[c0 + m] = Dw[m];
-    c.D[c.N + c0 + m] = Ew[m];
-    c.lperm[c0 + m] = lpw[m];
-  }
-  if (lane == 0) c.piv[s] = pivoted ? 1 : 0;
-  __syncwarp();
+  const bool pivoted = bk_block<T>(sB, nr, w, sD, sE, slp, 0, 1);
+  sn_finish<T, false>(c, s, c0, w, nr, r0, B, I, Dw, Ew, lpw, dv, pivoted, lane, 32, [](int) {});
 }
 
 // Factor the supernodes of mlist (ascending ids: children before parents,
 // the reference's order of mod_indices), then fold the pivots into the row
 // lists of the descendants (row_reordering, Sym_BLAS.cpp:327-490) and into
 // the ordering (reorder_matrix, linear_solver_wrapper.cpp:1432-1460).
-// Level-parallel form: supernodes of one level of the tree are independent
-// (each reads only descendants on lower levels and writes only itself), so
-// per level the first WF_WARPS warps take the marked supernodes that fit a
-// warp, in turn by their rank among the level's marked supernodes, and the
-// CTA factors the rest one at a time.  A refactorization of one or two paths
-// to the root (at most 2 nlev supernodes, the active-set iterations) keeps
-// the CTA path throughout: its supernodes are the widest, with the most
-// descendant updates, which the CTA path spreads over every warp.
-template <class T> __device__ void factor_marked(Ctx<T> &c) {
-  const int m = *c.nmark;
-  if (c.wf && m > 2 * c.nlev) {
-    const unsigned FULL = 0xffffffffu;
-    const int wi = warp_id(), lane = lane_id(), nwf = min(num_warps(), WF_WARPS);
-    auto fits = [&](int s) { return c.snrec[2 * s].y <= c.wcap && c.snrec[2 * s].z <= c.rcap; };
+// Supernodes of one level of the tree are independent (each reads only
+// descendants on lower levels and writes only itself), so a long list goes
+// level by level: single columns a warp each, wider ones a warp each where
+// there are enough of them to keep the warps busy (and the launch has the
+// scratch), else one after another by the CTA.  A short list (the one or two
+// paths to the root of an active-set step) runs through in order.
+template <class T> __device__ __noinline__ void factor_marked(Ctx<T> &) {
+  Ctx<T> &c = ctx<T>();
+  const int m = c.nmark;
+  const unsigned FULL = 0xffffffffu;
+  const int wi = warp_id(), lane = lane_id(), nwf = min(num_warps(), WF_WARPS);
+  // 0: a single column a warp takes, 1: a wide one that fits a warp, 2: the rest
+  auto kind = [&](int s) {
+    const int w = c.snrec[2 * s].y, nr = sn_rows(c.snrec[2 * s]);
+    if (w == 1 && nr <= 32) return 0;
+    return w > 1 && w <= c.wcap && nr <= c.rcap ? 1 : 2;
+  };
+  if (m > 2 * c.nlev) {
+#pragma unroll 1
     for (int l = 0; l < c.nlev; ++l) {
       // every warp counts the level's supernodes the same way (uniform over the CTA)
-      int nfit = 0;
-      bool big = false;
+      int n1 = 0, nw1 = 0, n2 = 0;
+#pragma unroll 1
       for (int t0 = 0; t0 < m; t0 += 32) {
-        const int t = t0 + lane;
-        const int s = t < m ? c.mlist[t] : -1;
-        const bool at = s >= 0 && c.lev[s] == l;
-        nfit += __popc(__ballot_sync(FULL, at && fits(s)));
-        big = big || __any_sync(FULL, at && !fits(s));
+        const int s = t0 + lane < m ? c.mlist[t0 + lane] : -1;
+        const int k = s >= 0 && c.lev[s] == l ? kind(s) : -1;
+        n1 += __popc(__ballot_sync(FULL, k == 0));
+        nw1 += __popc(__ballot_sync(FULL, k == 1));
+        n2 += __popc(__ballot_sync(FULL, k == 2));
       }
-      if (nfit > 0 && wi < nwf) {
+      const bool warps = c.wf && nw1 >= 2;
+      if (n1 + (warps ? nw1 : 0) > 0) {
         int seen = 0;
+#pragma unroll 1
         for (int t0 = 0; t0 < m; t0 += 32) {
-          const int t = t0 + lane;
-          const int s = t < m ? c.mlist[t] : -1;
-          unsigned bal = __ballot_sync(FULL, s >= 0 && c.lev[s] == l && fits(s));
+          const int s = t0 + lane < m ? c.mlist[t0 + lane] : -1;
+          const int k = s >= 0 && c.lev[s] == l ? kind(s) : -1;
+          unsigned bal = __ballot_sync(FULL, k == 0 || (k == 1 && warps));
           while (bal) {
             const int b = __ffs(bal) - 1;
             bal &= bal - 1u;
-            const int sb = __shfl_sync(FULL, s, b);
-            if (seen++ % nwf == wi) factor_sn_warp(c, sb, wi);
+            const int sb_ = __shfl_sync(FULL, s, b), kb = __shfl_sync(FULL, k, b);
+            if (seen++ % nwf == wi) {
+              if (kb == 0) factor_single(c, sb_, wi);
+              else factor_sn_warp(c, sb_, wi);
+            }
           }
         }
+        __syncthreads();
       }
-      if (nfit > 0) __syncthreads();
-      if (big)
+      if (n2 + (warps ? 0 : nw1) > 0)
+#pragma unroll 1
         for (int t = 0; t < m; ++t) {
           const int s = c.mlist[t];
-          if (c.lev[s] == l && !fits(s)) factor_sn(c, s);
+          if (c.lev[s] != l) continue;
+          const int k = kind(s);
+          if (k == 2 || (k == 1 && !warps)) factor_sn(c, s);
         }
     }
   } else {
-    for (int t = 0; t < m; ++t) factor_sn(c, c.mlist[t]);
+#pragma unroll 1
+    for (int t = 0; t < m; ++t) {
+      const int s = c.mlist[t];
+      if (kind(s) == 0) {
+        if (wi == 0) factor_single(c, s, 0);
+        __syncthreads();
+      } else {
+        factor_sn(c, s);
+      }
+    }
   }
   BQ_T0(c);
   // renaming: rows of descendants that fall into a pivoted supernode
+#pragma unroll 1
   for (int t = 0; t < m; ++t) {
     const int s = c.mlist[t];
     if (!c.piv[s]) continue;
     const int4 r0 = c.snrec[2 * s], r1 = c.snrec[2 * s + 1];
     const int c0 = r0.x, w = r0.y;
-    // inverse of the local pivot order: old local position -> new position
-    for (int q = threadIdx.x; q < w; q += blockDim.x) c.lp[c.lperm[c0 + q]] = q;
-    __syncthreads();
-    for (int pq = r1.y; pq < r1.w; ++pq) {
-      const int4 pr = c.prec[pq];
-      int *rd = c.ls + pr.w;
-      for (int i = pr.y + threadIdx.x; i <= pr.z; i += blockDim.x) {
-        const int o = rd[i] - c0;
-        if (o >= 0 && o < w) rd[i] = c0 + c.lp[o];
-        else atomicOr(c.status, ST_BOUNDS);
-      }
-    }
+    // inverse of the local pivot order: old local position -> new position;
     // composed ordering: new position q holds the column that was at lperm[q]
     // (old values staged in the free row map)
-    for (int q = threadIdx.x; q < w; q += blockDim.x) c.map[q] = c.perm[c0 + c.lperm[c0 + q]];
+#pragma unroll 1
+    for (int q = threadIdx.x; q < w; q += blockDim.x) {
+      const int o = c.lperm[c0 + q];
+      c.lp[o] = q;
+      c.map[q] = c.perm[c0 + o];
+    }
     __syncthreads();
-    for (int q = threadIdx.x; q < w; q += blockDim.x) c.perm[c0 + q] = c.map[q];
-    __syncthreads();
-    for (int q = threadIdx.x; q < w; q += blockDim.x) c.iperm[c.perm[c0 + q]] = c0 + q;
+#pragma unroll 1
+    for (int q = threadIdx.x; q < w; q += blockDim.x) {
+      const int j = c.map[q];
+      c.perm[c0 + q] = j;
+      c.iperm[j] = c0 + q;
+    }
+#pragma unroll 1
+    for (int pq = r1.y + threadIdx.x; pq < r1.w; pq += blockDim.x) {  // a pair per thread
+      const int4 ra = c.prec[2 * pq];
+      const int st = (unsigned)ra.y >> 16 ? 1 : 32;
+      int *rd = c.ls + ra.w;
+#pragma unroll 1
+      for (int i = 0; i < ra.z; ++i) {
+        const int o = rd[i * st] - c0;
+        if (o >= 0 && o < w) rd[i * st] = c0 + c.lp[o];
+        else atomicOr(&c.status, ST_BOUNDS);
+      }
+    }
     __syncthreads();
   }
+#pragma unroll 1
   for (int t = threadIdx.x; t < m; t += blockDim.x) c.mark[c.mlist[t]] = 0;
   __syncthreads();
-  if (threadIdx.x == 0) *c.nmark = 0;
+  if (threadIdx.x == 0) c.nmark = 0;
   __syncthreads();
   BQ_T1(c, PH_RENAME);
 }
 
-// ---- triangular solves (factor order, vector in shared memory) ---------------
-// Forward step of one supernode (reference H2LeveledBlockedLsolve,
-// Triangular_BCSC.cpp:378-446): x_s <- L11^-1 x_s through the stored inverse,
-// then the rows below push -L21 x_s into their (ancestor) entries; pushes of
-// supernodes of the same level may meet, so they are atomic, as in the
-// reference's threaded solve (:435).  Wide levels: a thread per supernode,
-// narrow levels: a warp per supernode.
-template <class T> __device__ void fwd_thread(Ctx<T> &c, int s) {
-  T *x = c.xs;
-  const int4 r0 = c.snrec[2 * s], r1 = c.snrec[2 * s + 1];
-  const int c0 = r0.x, w = r0.y, nr = r0.z;
-  const T *Ls = c.L + r0.w;
-  const int *rows = c.ls + r1.x;
-  for (int i = w - 1; i > 0; --i) {  // bottom-up: row i reads x_j, j < i, not yet replaced
-    T acc = x[c0 + i];
-    for (int j = 0; j < i; ++j) acc += Ls[i + (size_t)j * nr] * x[c0 + j];
-    x[c0 + i] = acc;
-  }
-#pragma unroll 4
-  for (int r = w; r < nr; ++r) {
-    T y = T(0);
-    for (int k = 0; k < w; ++k) y += Ls[r + (size_t)k * nr] * x[c0 + k];
-    const int rr = rows[r];
-    if ((unsigned)rr < (unsigned)c.N) atomicAdd(&x[rr], -y);
-  }
+// ---- triangular solves (factor order, vectors in shared memory) ----------------
+// Forward (reference H2LeveledBlockedLsolve, Triangular_BCSC.cpp:378-446):
+// t_s = L11^-1 x_s, then the rows below lose L21 t_s (pushes of supernodes of
+// the same level may meet, so they are atomic, as in the reference's threaded
+// solve, :435).  Backward (:534-600): v_s = D^-1 t_s - L21^T x(rows below),
+// x_s = L11^-T v_s.  Two vectors, xs and xo, take turns, so that all rows
+// (columns) of a level's supernodes can be formed at once: xs holds the
+// accumulated right hand side, then v; xo holds t, then the solution.  Single
+// columns need no t: theirs is x_s.
+//
+// What bounds them: latency (a chain of row index, factor entry and push per
+// level, 16 warps on an SM that issue one instruction in 16 cycles each), the
+// instructions of a step, the lines that a warp's loads touch, and in FP64
+// operations (a multiply-add holds the FP64 pipe of its SM quarter for 64
+// cycles whatever the number of lanes at work).  So
+//  * the rows (columns) of all wide supernodes of a level form one list (so_f,
+//    so_b, in the pattern), dealt to the threads with as many lanes to a row
+//    as keep the CTA full;
+//  * a step issues its first loads, which no other step writes, before the
+//    barrier that it has to wait for, and no load stands under a condition:
+//    places beyond the end read a valid entry with a zero factor (a branch per
+//    term made every load wait for the one before: 230k cycles per
+//    application of horizon-50 MPC, FP32, 4 CTAs per SM);
+//  * where a level has many single columns, their targets gather (so_g: the
+//    factor entries once more, by target) instead of the columns pushing: an
+//    FP32 atomic of shared memory takes 88 cycles for every lane that meets
+//    another on its entry, an FP64 one 140.
+template <class T> __device__ __forceinline__ void push(const Ctx<T> &c, int rr, T y) {
+  if (y != T(0)) atomicAdd(&c.xs[min((unsigned)rr, (unsigned)c.N - 1u)], -y);
 }
 
-template <class T> __device__ void fwd_warp(Ctx<T> &c, int s) {
-  T *x = c.xs;
-  const int lane = lane_id();
-  const int4 r0 = c.snrec[2 * s], r1 = c.snrec[2 * s + 1];
-  const int c0 = r0.x, w = r0.y, nr = r0.z;
-  const T *Ls = c.L + r0.w;
-  const int *rows = c.ls + r1.x;
-  // x_s <- L11^-1 x_s: lanes form rows of the product, then write; chunks
-  // of 32 rows from the bottom (a chunk reads only rows above it)
-  for (int i0 = ((w - 1) / 32) * 32; i0 >= 0; i0 -= 32) {
-    const int i = i0 + lane;
-    T acc = T(0);
-    if (i < w) {
-      acc = x[c0 + i];
-      for (int j = 0; j < i; ++j) acc += Ls[i + (size_t)j * nr] * x[c0 + j];
-    }
-    __syncwarp();
-    if (i < w) x[c0 + i] = acc;
-    __syncwarp();
-  }
-  for (int r = w + lane; r < nr; r += 32) {
-    T y = T(0);
-    for (int k = 0; k < w; ++k) y += Ls[r + (size_t)k * nr] * x[c0 + k];
-    const int rr = rows[r];
-    if ((unsigned)rr < (unsigned)c.N) atomicAdd(&x[rr], -y);
-  }
-  __syncwarp();
-}
-
-// Backward (Triangular_BCSC.cpp:534-600): x1 -= L21^T x(rows below), then
-// x1 <- L11^-T x1 through the stored inverse.
-template <class T> __device__ void bwd_thread(Ctx<T> &c, int s) {
-  T *x = c.xs;
-  const int4 r0 = c.snrec[2 * s], r1 = c.snrec[2 * s + 1];
-  const int c0 = r0.x, w = r0.y, nr = r0.z;
-  const int *rows = c.ls + r1.x;
-  const T *Ls = c.L + r0.w;
-  for (int j = 0; j < w; ++j) {
-    T acc = T(0);
-#pragma unroll 4
-    for (int r = w; r < nr; ++r) {
-      const int rr = rows[r];
-      if ((unsigned)rr < (unsigned)c.N) acc += Ls[r + (size_t)j * nr] * x[rr];
-    }
-    x[c0 + j] -= acc;
-  }
-  // top-down: entry j reads x_i, i > j, not yet replaced
-  for (int j = 0; j + 1 < w; ++j) {
-    T acc = x[c0 + j];
-    for (int i = j + 1; i < w; ++i) acc += Ls[i + (size_t)j * nr] * x[c0 + i];
-    x[c0 + j] = acc;
-  }
-}
-
-template <class T> __device__ void bwd_warp(Ctx<T> &c, int s) {
-  T *x = c.xs;
-  const int lane = lane_id();
-  const int4 r0 = c.snrec[2 * s], r1 = c.snrec[2 * s + 1];
-  const int c0 = r0.x, w = r0.y, nr = r0.z;
-  const int *rows = c.ls + r1.x;
-  const T *Ls = c.L + r0.w;
-  for (int j = 0; j < w; ++j) {
-    T acc = T(0);
-    for (int r = w + lane; r < nr; r += 32) {
-      const int rr = rows[r];
-      if ((unsigned)rr < (unsigned)c.N) acc += Ls[r + (size_t)j * nr] * x[rr];
+// Four rows below of a single column (entry r0 on, stride st), zeros beyond the end.
+template <class T> struct Single4 {
+  T l[4];
+  int rr[4];
+  __device__ __forceinline__ void load(const Ctx<T> &c, const int4 &v, int r0, int st) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = min(r0 + q, v.y - 1);
+      l[q] = c.L[v.z + r * st];
+      rr[q] = c.ls[v.w + r * st];
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane == 0) x[c0 + j] -= acc;
+    for (int q = 0; q < 4; ++q)
+      if (r0 + q >= v.y) l[q] = T(0);
   }
-  __syncwarp();
-  // x_s <- L11^-T x_s: lanes form entries of the product, chunks of 32 from the top
-  for (int j0 = 0; j0 < w; j0 += 32) {
-    const int j = j0 + lane;
+};
+template <class T> __device__ __noinline__ void fwd_single(Ctx<T> &, const int4 v, int st) {
+  Ctx<T> &c = ctx<T>();
+  const T t = c.xs[v.x];
+#pragma unroll 1
+  for (int r0 = 1; r0 < v.y; r0 += 4) {
+    Single4<T> b;
+    b.load(c, v, r0, st);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) push(c, b.rr[q], b.l[q] * t);
+  }
+}
+// b: the first four rows, loaded
+template <class T> __device__ __forceinline__ void bwd_single(Ctx<T> &c, const int4 &v, Single4<T> &b, T dinv, int st) {
+  T acc = dinv * c.xs[v.x];
+#pragma unroll 1
+  for (int r0 = 1; r0 < v.y;) {
+    T x[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = c.xo[min((unsigned)b.rr[q], (unsigned)c.N - 1u)];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc -= b.l[q] * x[q];
+    r0 += 4;
+    if (r0 < v.y) b.load(c, v, r0, st);
+  }
+  c.xo[v.x] = acc;
+}
+// Single columns of constraints and long ones: few are visible at a time.
+template <class T> __device__ __noinline__ void fwd_listed(Ctx<T> &, int a, int m, int e) {
+  Ctx<T> &c = ctx<T>();
+#pragma unroll 1
+  for (int q = a + threadIdx.x; q < m; q += blockDim.x) fwd_single(c, c.vrec[q], 1);
+#pragma unroll 1
+  for (int q = m + warp_id(); q < e; q += num_warps()) {
+    const int4 v = c.vrec[q];
+    const T t = c.xs[v.x];
+#pragma unroll 4
+    for (int r = 1 + lane_id(); r < v.y; r += 32) push(c, c.ls[v.w + r], c.L[v.z + r] * t);
+  }
+}
+template <class T> __device__ __noinline__ void bwd_listed(Ctx<T> &, int a, int m, int e) {
+  Ctx<T> &c = ctx<T>();
+#pragma unroll 1
+  for (int q = a + threadIdx.x; q < m; q += blockDim.x) {
+    const int4 v = c.vrec[q];
+    Single4<T> b;
+    b.load(c, v, 1, 1);
+    bwd_single(c, v, b, c.L[v.z], 1);
+  }
+#pragma unroll 1
+  for (int q = m + warp_id(); q < e; q += num_warps()) {
+    const int4 v = c.vrec[q];
     T acc = T(0);
-    if (j < w) {
-      acc = x[c0 + j];
-      for (int i = j + 1; i < w; ++i) acc += Ls[i + (size_t)j * nr] * x[c0 + i];
-    }
-    __syncwarp();
-    if (j < w) x[c0 + j] = acc;
-    __syncwarp();
+#pragma unroll 4
+    for (int r = 1 + lane_id(); r < v.y; r += 32)
+      acc += c.L[v.z + r] * c.xo[min((unsigned)c.ls[v.w + r], (unsigned)c.N - 1u)];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane_id() == 0) c.xo[v.x] = c.L[v.z] * c.xs[v.x] - acc;
   }
 }
 
-// x <- (L D L^T)^-1 x on the visible part, in the factor's order.  Per
-// level, small supernodes take a thread each and big ones a warp each, in
-// the same pass (supernodes of one level are independent).
-template <class T> __device__ void ldlt_solve_smem(Ctx<T> &c) {
-  const int nw = num_warps();
+// The targets of a level's single columns: x_j loses the sum of its entries
+// times the columns' x.  g: first group of 32 targets, n of them;
+// `alone`: no other thread pushes meanwhile.
+template <class T> __device__ __noinline__ void gather_singles(Ctx<T> &, int g0, int n, bool alone) {
+  Ctx<T> &c = ctx<T>();
+#pragma unroll 1
+  for (int g = g0 + warp_id(); g < g0 + n; g += num_warps()) {
+    const int2 gr = c.so_g[g];  // first entry, entries per lane (a multiple of 4)
+    const int j = c.so_gj[32 * g + lane_id()];  // variable, -1 beyond the end
+    const int pos = c.iperm[max(j, 0)];
+    T acc = T(0);
+#pragma unroll 1
+    for (int k = 0; k < gr.y; k += 4) {
+      const int e = gr.x + 32 * k + lane_id();
+      T l[4], x[4];
+      int src[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        src[q] = c.so_gs[e + 32 * q];
+        l[q] = c.G[e + 32 * q];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) x[q] = c.xs[src[q]];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc += l[q] * x[q];
+    }
+    if (j >= 0) {
+      if (alone) c.xs[pos] -= acc;
+      else atomicAdd(&c.xs[pos], -acc);
+    }
+  }
+}
+
+// Sum over the G = 2^lg neighbouring lanes that share an item.
+template <class T> __device__ __forceinline__ T lanes_sum(T v, int lg) {
+#pragma unroll 1
+  for (int o = 1 << lg >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Sum of a block's row with x[0 ..] (zeros follow its terms up to a multiple
+// of four): lane g of G takes every G-th group of four, from k0 = 4 g; p: its
+// first two groups, loaded.
+template <class T> struct RowTerms {
+  T p[2][4];
+  __device__ __forceinline__ void load(const T *row, int k0, int terms, int lg) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = k0 + (4 << lg) * h;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) p[h][q] = T(0);
+      if (k < terms) load4(row + k, p[h]);
+    }
+  }
+  __device__ __forceinline__ T sum(const T *row, const T *x, int terms, int k0, int lg) {
+    T acc = T(0);
+    const int last = terms - 1;
+#pragma unroll 1
+    for (; k0 < terms;) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int k = k0 + (4 << lg) * h;
+        if (h == 1 && k >= terms) break;
+        T v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = x[min(k + q, last)];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc += p[h][q] * v[q];
+      }
+      k0 += 8 << lg;
+      if (k0 < terms) load(row, k0, terms, lg);
+    }
+    return acc;
+  }
+};
+// Sum down a block's column (stride ld, terms terms): lane g of G takes every
+// G-th row from r0 = g; p: its first four, loaded (zeros beyond the end).
+template <class T> struct ColTerms {
+  T p[4];
+  __device__ __forceinline__ void load(const T *col, int r0, int ld, int terms, int lg) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = r0 + (q << lg);
+      p[q] = T(0);
+      if (r < terms) p[q] = col[r * ld];
+    }
+  }
+};
+
+// xo <- (L D L^T)^-1 xs on the visible part, in the factor's order (xs is
+// overwritten).  The caller's writes to xs and xo need no barrier before;
+// one follows the last step.
+template <class T> __device__ __noinline__ void ldlt_solve_smem(Ctx<T> &) {
+  Ctx<T> &c = ctx<T>();
+  const int tid = threadIdx.x, nt = blockDim.x, lane = lane_id();
+  const T *const S = c.S;
+  const int *const ls = c.ls;
+  T *const xs = c.xs, *const xo = c.xo;
+  const int nlev = c.nlev;
+  const unsigned top = (unsigned)c.N - 1u;
   {
     BQ_T0(c);
-    for (int l = 0; l < c.nlev; ++l) {
-      const int a = c.vlvl[l], m = c.vmid[l], b = c.vlvl[l + 1];
-      for (int q = a + threadIdx.x; q < m; q += blockDim.x) fwd_thread(c, c.vlist[q]);
-      for (int q = m + warp_id(); q < b; q += nw) fwd_warp(c, c.vlist[q]);
-      __syncthreads();
+#pragma unroll 1
+    for (int l = 0; l < nlev; ++l) {
+      const int a = c.vseg[2 * l], m = c.vseg[2 * l + 1], e = c.vseg[2 * l + 2];
+      const int4 lf = c.lvl[3 * l], lb = c.lvl[3 * l + 1], lg_ = c.lvl[3 * l + 2];
+      const int n1 = lf.y >> 5, lg1 = lf.y & 31, n2 = lf.w >> 5, lg2 = lf.w & 31, es = lb.z, en = lb.w;
+      if (a == e && n1 == 0 && en == 0) continue;
+      // t of the wide supernodes (an item: a row of L11^-1), then the single columns
+      if (n1 > 0) {
+        int t = tid, it = t >> lg1, k0 = 4 * (t & ((1 << lg1) - 1));
+        int4 v = c.so_f[lf.x + min(it, n1 - 1)];  // {row in S, first column, terms, row-list position}
+        RowTerms<T> rt;
+        rt.load(S + v.x, k0, v.z, lg1);
+        __syncthreads();
+#pragma unroll 1
+        for (; t - lane < n1 << lg1;) {
+          const T y = lanes_sum(rt.sum(S + v.x, xs + v.y, v.z, k0, lg1), lg1);
+          if (k0 == 0 && it < n1) xo[v.y + v.z - 1] = y;
+          t += nt;
+          if (t - lane >= n1 << lg1) break;
+          it = t >> lg1;
+          v = c.so_f[lf.x + min(it, n1 - 1)];
+          rt.load(S + v.x, k0, v.z, lg1);
+        }
+      } else {
+        __syncthreads();
+      }
+      if (lg_.y > 0) {
+        gather_singles(c, lg_.x, lg_.y, a == e);
+      } else {
+#pragma unroll 1
+        for (int q = tid; q < en; q += nt) fwd_single(c, c.so_e[es + q], 32);
+      }
+      if (a != e) fwd_listed(c, a, m, e);
+      if (n1 > 0) {
+        // pushes of the wide ones (an item: a row of L21)
+        int t = tid, it = t >> lg2, k0 = 4 * (t & ((1 << lg2) - 1));
+        int4 v = make_int4(0, 0, 0, 0);
+        RowTerms<T> rt;
+        int rr = 0;
+        if (n2 > 0) {
+          v = c.so_f[lf.z + min(it, n2 - 1)];
+          rt.load(S + v.x, k0, v.z, lg2);
+          rr = ls[v.w];
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (; t - lane < n2 << lg2;) {
+          const T y = lanes_sum(rt.sum(S + v.x, xo + v.y, v.z, k0, lg2), lg2);
+          if (k0 == 0 && it < n2) push(c, rr, y);
+          t += nt;
+          if (t - lane >= n2 << lg2) break;
+          it = t >> lg2;
+          v = c.so_f[lf.z + min(it, n2 - 1)];
+          rt.load(S + v.x, k0, v.z, lg2);
+          rr = ls[v.w];
+        }
+      }
     }
     BQ_T1(c, PH_FWD_WIDE);
   }
-  {
-    BQ_T0(c);
-    // D solve: 1x1 by division, 2x2 by Cramer's rule (blocked_2by2_solver, Sym_BLAS.cpp:492-529)
-    for (int i = threadIdx.x; i < c.N; i += blockDim.x) {
-      if (!visible(c, c.col2sup[i])) continue;
-      if (i > 0 && c.D[c.N + i - 1] != T(0)) continue;  // second column of a 2x2 block
-      const T e = i + 1 < c.N ? c.D[c.N + i] : T(0);
-      if (e == T(0)) {
-        c.xs[i] = c.xs[i] / c.D[i];
-      } else {
-        const T d1 = c.D[i], d2 = c.D[i + 1];
-        const T inv = T(1) / (d1 * d2 - e * e);
-        const T x1 = c.xs[i], x2 = c.xs[i + 1];
-        c.xs[i] = (x1 * d2 - x2 * e) * inv;
-        c.xs[i + 1] = (x2 * d1 - x1 * e) * inv;
+  BQ_T0(c);
+#pragma unroll 1
+  for (int l = nlev - 1; l >= 0; --l) {
+    const int a = c.vseg[2 * l], m = c.vseg[2 * l + 1], e = c.vseg[2 * l + 2];
+    const int4 lb = c.lvl[3 * l + 1];
+    const int n = lb.y >> 5, lg = lb.y & 31, es = lb.z, en = lb.w;
+    if (a == e && n == 0 && en == 0) continue;
+    const int g = tid & ((1 << lg) - 1), total = n << lg;
+    // an item: a column {its first entry in L21, c0 << 16 | w, place in the block << 16 | rows below, row-list offset}
+    int4 v0 = make_int4(0, 0, 0, 0);
+    if (n > 0) {
+      int t = tid, it = t >> lg;
+      int4 v = c.so_b[lb.x + min(it, n - 1)];
+      v0 = v;
+      ColTerms<T> ct;
+      int rr[4];
+      T d, db, dbm;
+      auto load = [&]() {
+        const int ld = s_ld(v.y & 0xffff), mm = v.z & 0xffff, j = (int)((unsigned)v.z >> 16);
+        const int cj = (int)((unsigned)v.y >> 16) + j;
+        ct.load(S + v.x, g, ld, mm, lg);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) rr[q] = ls[v.w + max(min(g + (q << lg), mm - 1), -1)];
+        d = c.Di[cj];
+        db = c.Di[c.N + cj];
+        dbm = c.Di[c.N + cj - (j > 0 ? 1 : 0)];
+        if (j == 0) dbm = T(0);
+      };
+      load();
+      __syncthreads();
+#pragma unroll 1
+      for (; t - lane < total;) {
+        const int ld = s_ld(v.y & 0xffff), mm = v.z & 0xffff, j = (int)((unsigned)v.z >> 16);
+        const int cj = (int)((unsigned)v.y >> 16) + j;
+        T y = T(0);
+#pragma unroll 1
+        for (int r0 = g; r0 < mm;) {
+          T x[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) x[q] = xo[min((unsigned)rr[q], top)];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) y += ct.p[q] * x[q];
+          r0 += 4 << lg;
+          if (r0 < mm) {
+            ct.load(S + v.x, r0, ld, mm, lg);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) rr[q] = ls[v.w + min(r0 + (q << lg), mm - 1)];
+          }
+        }
+        y = lanes_sum(y, lg);
+        const T u = d * xo[cj] + db * xo[cj + (db != T(0) ? 1 : 0)] + dbm * xo[cj - (dbm != T(0) ? 1 : 0)] - y;
+        if (g == 0 && it < n) xs[cj] = u;
+        t += nt;
+        if (t - lane >= total) break;
+        it = t >> lg;
+        v = c.so_b[lb.x + min(it, n - 1)];
+        load();
+      }
+    } else {
+      __syncthreads();
+    }
+#pragma unroll 1
+    for (int q = tid; q < en; q += nt) {
+      const int4 v = c.so_e[es + q];
+      Single4<T> b;
+      b.load(c, v, 1, 32);
+      bwd_single(c, v, b, c.L[v.z], 32);
+    }
+    if (a != e) bwd_listed(c, a, m, e);
+    if (n > 0) {
+      // x_j = v_j + sum over i > j of L11^-1(i, j) v_i: the rows j + 1 .. w of the column
+      int t = tid, it = t >> lg;
+      int4 v = v0;
+      ColTerms<T> ct;
+      int terms, ld, cj;
+      const T *col;
+      auto load = [&]() {
+        const int w = v.y & 0xffff, j = (int)((unsigned)v.z >> 16);
+        cj = (int)((unsigned)v.y >> 16) + j;
+        ld = s_ld(w);
+        terms = w - 1 - j;
+        col = S + v.x - terms * ld;  // L21's first row is row w
+        ct.load(col, g, ld, terms, lg);
+      };
+      load();
+      __syncthreads();
+#pragma unroll 1
+      for (; t - lane < total;) {
+        T y = T(0);
+#pragma unroll 1
+        for (int r0 = g; r0 < terms;) {
+          T x[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) x[q] = xs[cj + min(1 + r0 + (q << lg), terms)];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) y += ct.p[q] * x[q];
+          r0 += 4 << lg;
+          if (r0 < terms) ct.load(col, r0, ld, terms, lg);
+        }
+        y = lanes_sum(y, lg);
+        if (g == 0 && it < n) xo[cj] = xs[cj] + y;
+        t += nt;
+        if (t - lane >= total) break;
+        it = t >> lg;
+        v = c.so_b[lb.x + min(it, n - 1)];
+        load();
       }
     }
-    __syncthreads();
-    BQ_T1(c, PH_DIAG);
   }
-  BQ_T0(c);
-  for (int l = c.nlev - 1; l >= 0; --l) {
-    const int a = c.vlvl[l], m = c.vmid[l], b = c.vlvl[l + 1];
-    for (int q = a + threadIdx.x; q < m; q += blockDim.x) bwd_thread(c, c.vlist[q]);
-    for (int q = m + warp_id(); q < b; q += nw) bwd_warp(c, c.vlist[q]);
-    __syncthreads();
-  }
+  __syncthreads();
   BQ_T1(c, PH_BWD);
 }
 
-// Visible supernodes grouped by level (after every change of the active set):
-// per level the small ones, then the big ones.
-template <class T> __device__ void build_vlist(Ctx<T> &c) {
-  const int L1 = c.nlev + 1;
-  for (int l = threadIdx.x; l < 2 * L1; l += blockDim.x) c.vfill[l] = 0;
+// The visible single columns' records, compacted from the pattern's order (by
+// level, then short / long) after every change of the active set, where each
+// level's two groups start, and the rows of the active constraints.  Each
+// warp counts, then writes, its own stretch of the order.
+template <class T> __device__ __noinline__ void build_vlist(Ctx<T> &) {
+  Ctx<T> &c = ctx<T>();
+  const int lane = lane_id(), wi = warp_id(), nw = num_warps(), ns = c.n1;
+  const int per = ((ns + nw - 1) / nw + 31) / 32 * 32;
+  const int t0 = min(wi * per, ns), t1 = min(t0 + per, ns);
+  int cnt = 0;  // visible ones, and constraint columns among them (high half)
+#pragma unroll 1
+  for (int t = t0 + lane; t < t1; t += 32) {
+    const int s = c.so_sn[t];
+    if (c.vis[s]) cnt += c.sn_con[s] >= 0 ? 0x10001 : 1;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+  if (lane == 0) c.redi[wi] = cnt;
   __syncthreads();
-  for (int s = threadIdx.x; s < c.ns; s += blockDim.x)
-    if (c.vis[s]) atomicAdd(&c.vfill[c.lev[s] + (c.sn_big[s] ? L1 : 0)], 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int l = 0; l < c.nlev; ++l) {
-      c.vlvl[l] = acc;
-      acc += c.vfill[l];
-      c.vmid[l] = acc;
-      acc += c.vfill[L1 + l];
-      c.vfill[l] = c.vlvl[l];     // next free position of the small ones
-      c.vfill[L1 + l] = c.vmid[l];  // and of the big ones
-    }
-    c.vlvl[c.nlev] = acc;
+  int before = 0, total = 0;
+#pragma unroll 1
+  for (int k = 0; k < nw; ++k) {
+    if (k < wi) before += c.redi[k];
+    total += c.redi[k];
+  }
+  int pos = before & 0xffff, pcon = before >> 16;
+  const unsigned below = (1u << lane) - 1u;
+#pragma unroll 1
+  for (int tb = t0; tb < t1; tb += 32) {
+    const int t = tb + lane;
+    const int s = t < t1 ? c.so_sn[t] : 0;
+    const bool v = t < t1 && c.vis[s] != 0;
+    const int k = v ? c.sn_con[s] : -1;
+    const unsigned bal = __ballot_sync(0xffffffffu, v), bcon = __ballot_sync(0xffffffffu, k >= 0);
+    const int p = pos + __popc(bal & below);
+    if (t < t1) c.map[t] = p;  // records before position t (the row map is free here)
+    if (v) c.vrec[p] = c.so_rec[t];
+    if (k >= 0) c.arow[pcon + __popc(bcon & below)] = c.base + k;
+    pos += __popc(bal);
+    pcon += __popc(bcon);
   }
   __syncthreads();
-  for (int s = threadIdx.x; s < c.ns; s += blockDim.x)
-    if (c.vis[s]) c.vlist[atomicAdd(&c.vfill[c.lev[s] + (c.sn_big[s] ? L1 : 0)], 1)] = s;
+#pragma unroll 1
+  for (int k = threadIdx.x; k <= 2 * c.nlev; k += blockDim.x) {
+    const int t = c.so_seg[k];
+    c.vseg[k] = t < ns ? c.map[t] : total & 0xffff;
+  }
+  if (threadIdx.x == 0) c.vseg[2 * c.nlev + 1] = total >> 16;
   __syncthreads();
 }
 
-// out = M^-1 v (original numbering; hidden rows give zero).  Vectors in
-// global memory, the solve in shared memory.
-template <class T, class VI, class VO> __device__ void precond(Ctx<T> &c, const VI *v, VO *out) {
+// Rows of K that take part: the structural ones, then the active
+// constraints (c.arow, kept by build_vlist).  Everything below runs over
+// them alone: the hidden rows of a small batch QP outnumber them (900 of
+// 1650 at horizon 50), and FP64 operations are what the vectors cost.
+template <class T> __device__ __forceinline__ int vis_rows(const Ctx<T> &c) { return c.base + c.vseg[2 * c.nlev + 1]; }
+template <class T> __device__ __forceinline__ int vis_row(const Ctx<T> &c, int t) {
+  return t < c.base ? t : c.arow[t - c.base];
+}
+// f(i) for every hidden row i
+template <class T, class F> __device__ __forceinline__ void hidden_rows(const Ctx<T> &c, F &&f) {
+#pragma unroll 1
+  for (int k = threadIdx.x; k < c.mineq; k += blockDim.x)
+    if (!c.act[k]) f(c.base + k);
+}
+
+// out(i, M^-1 v) over the visible rows (original numbering), v(i) the right
+// hand side; the solve runs in shared memory.  Both permutations go through
+// iperm, so that the global side is read and written in order.  Ends with a
+// barrier.  Cycles per application of horizon-50 MPC with 4 CTAs on the SM,
+// against one thread or warp per supernode walking its entries: FP32 458k ->
+// 126k, FP64 969k -> 248k; 2048 cold QPs (FP32) 121 -> 46 ms, 1024 (FP64)
+// 92 -> 32 ms.
+template <class T, class VI, class VO> __device__ void precond(Ctx<T> &c, VI &&v, VO &&out) {
   BQ_T0(c);
-  const long long tg0 = c.cyc ? clock64() : 0;
-  for (int i = threadIdx.x; i < c.N; i += blockDim.x) c.xs[i] = visible(c, c.col2sup[i]) ? T(v[c.perm[i]]) : T(0);
-  __syncthreads();
-  if (c.cyc && threadIdx.x == 0) c.cyc[PH_GATHER] += (unsigned long long)(clock64() - tg0);
+  const long long tg0 = c.prof ? clock64() : 0;
+  const int M = vis_rows(c);
+#pragma unroll 4
+  for (int t = threadIdx.x; t < M; t += blockDim.x) {
+    const int i = vis_row(c, t);
+    c.xs[c.iperm[i]] = T(v(i));
+  }
+  hidden_rows(c, [&](int i) { c.xo[c.iperm[i]] = T(0); });  // read by the products with hidden rows' zeros
+  if (c.prof && threadIdx.x == 0) c.cyc[PH_GATHER] += (unsigned long long)(clock64() - tg0);
   ldlt_solve_smem(c);
-  const long long tg1 = c.cyc ? clock64() : 0;
-  for (int i = threadIdx.x; i < c.N; i += blockDim.x) out[c.perm[i]] = VO(c.xs[i]);
+  const long long tg1 = c.prof ? clock64() : 0;
+#pragma unroll 4
+  for (int t = threadIdx.x; t < M; t += blockDim.x) {
+    const int i = vis_row(c, t);
+    out(i, c.xo[c.iperm[i]]);
+  }
   __syncthreads();
-  if (c.cyc && threadIdx.x == 0) c.cyc[PH_GATHER] += (unsigned long long)(clock64() - tg1);
+  if (c.prof && threadIdx.x == 0) c.cyc[PH_GATHER] += (unsigned long long)(clock64() - tg1);
   BQ_T1(c, PH_PRECOND);
 }
 
-// y = K x with the refinement values (original numbering).
-template <class T> __device__ void spmv_ref(const Ctx<T> &c, const double *x, double *y) {
-  BQ_T0(c);
-  for (int i = threadIdx.x; i < c.N; i += blockDim.x) {
-    double acc = 0.0;
-    for (int qq = c.Rp[i]; qq < c.Rp[i + 1]; ++qq) acc += c.Rv[qq] * x[c.Rj[qq]];
-    y[i] = acc;
+// Row i of K x with the refinement values (original numbering).  Entries of
+// hidden constraints are zeros and skipped by their bits: the columns there
+// hold no value of this problem.
+template <class T> __device__ __forceinline__ double spmv_row(const Ctx<T> &c, const double *x, int i) {
+  double acc = 0.0;
+  const int q1 = c.Rp[i + 1];
+#pragma unroll 1
+  for (int q0 = c.Rp[i]; q0 < q1; q0 += 4) {
+    double v[4], u[4];
+    int j[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int q = min(q0 + e, q1 - 1);
+      v[e] = c.Rv[q];
+      j[e] = c.Rj[q];
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) u[e] = x[j[e]];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (q0 + e < q1 && __double_as_longlong(v[e]) << 1) acc += v[e] * u[e];
   }
-  __syncthreads();
-  BQ_T1(c, PH_SPMV);
+  return acc;
 }
 
-template <class T> __device__ double dot(const Ctx<T> &c, const double *a, const double *b) {
-  double s = 0.0;
-  for (int i = threadIdx.x; i < c.N; i += blockDim.x) s += a[i] * b[i];
-  return block_sum(s, c.red);
+// Block-wide sums of K values in a fixed order (the same inputs give the
+// same bits on every run).  `par` alternates between two halves of red, so
+// one barrier per call is enough; every thread adds the warps' sums itself.
+template <int K> __device__ __forceinline__ void block_sums(double (&v)[K], double *red, int &par) {
+  static_assert(K <= 2, "two halves of 16 doubles, up to 8 warps");
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < K; ++q) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+  double *h = red + 16 * par;
+  par ^= 1;
+  if (lane_id() == 0)
+#pragma unroll
+    for (int q = 0; q < K; ++q) h[q * 8 + warp_id()] = v[q];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    v[q] = h[q * 8];
+#pragma unroll 1
+    for (int t = 1; t < num_warps(); ++t) v[q] += h[q * 8 + t];
+  }
 }
 
 // ---- refinement (reference pmgmres_ldlt_auto, src/gmres/mgmres.cpp:1015-1211)
-struct GmresSmall {
-  double h[MR_CAP + 1][MR_CAP], cs[MR_CAP + 1], sn[MR_CAP + 1], g[MR_CAP + 1], y[MR_CAP + 1];
-  double scal[4];
-};
 
 // Solves K x = b (x holds the preconditioned solution on entry).  flexible:
 // right-preconditioned FGMRES with stored directions Z (Saad 1993) -- the
@@ -1098,92 +1629,180 @@ struct GmresSmall {
 // left-preconditioned GMRES.  adaptive: stop once the residual estimate is
 // below rtol * ||b||; else the reference's rule (rho <= tol_rel * rho0 and
 // rho <= tol_abs).  Returns the Krylov steps taken.
+//
+// The vectors are a few hundred FP64 entries in L2: what they cost is FP64
+// operations and block-wide sums.  So a pass forms all it can of the next
+// step (residual and its norm, K z with its norm and first projection, each
+// projection with the next one), vectors are scaled by a reciprocal (an FP64
+// division takes nine multiply-adds) and only if a further step reads them.
+// A row belongs to the same thread in every pass, so barriers stand only
+// where a product with K or a solve crosses rows.
 template <class T>
 __device__ int refine(Ctx<T> &c, const double *b, double *x, int itr_max, int mr, bool flexible, bool adaptive,
-                      double rtol, double tol_abs, double tol_rel, GmresSmall &gs) {
+                      double rtol, double tol_abs, double tol_rel) {
   if (itr_max <= 0 || mr <= 0) return 0;
   mr = min(mr, MR_CAP);
-  const int N = c.N;
+  GmresSmall &gs = c.gs;
+  const int N = c.N, M = vis_rows(c), tid = threadIdx.x, nt = blockDim.x;
   const double delta = 1.0e-03;
   double *r = c.r, *V = c.V;
   double rho = 0.0, rho_tol = 0.0, stop_abs = tol_abs;
-  int used = 0;
+  int used = 0, par = 0;
+  __syncthreads();  // red is free
   if (adaptive) {
-    const double nb = sqrt(dot(c, b, b));
-    stop_abs = rtol * nb;
+    double s[1] = {0.0};
+#pragma unroll 1
+    for (int t = tid; t < M; t += nt) {
+      const double v = b[vis_row(c, t)];
+      s[0] += v * v;
+    }
+    block_sums<1>(s, c.red, par);
+    stop_abs = rtol * sqrt(s[0]);
   }
+#pragma unroll 1
   for (int itr = 0; itr < itr_max; ++itr) {
-    spmv_ref(c, x, r);
-    for (int i = threadIdx.x; i < N; i += blockDim.x) r[i] = b[i] - r[i];
-    __syncthreads();
-    if (!flexible) precond(c, r, r);
-    rho = sqrt(dot(c, r, r));
+    double s1[1] = {0.0};
+    {
+      BQ_T0(c);
+#pragma unroll 1
+      for (int t = tid; t < M; t += nt) {
+        const int i = vis_row(c, t);
+        const double v = b[i] - spmv_row(c, x, i);
+        r[i] = v;
+        if (flexible) s1[0] += v * v;
+      }
+      BQ_T1(c, PH_SPMV);
+    }
+    if (!flexible) {
+      __syncthreads();
+      precond(c, [&](int i) { return r[i]; }, [&](int i, T v) {
+        const double u = (double)v;
+        r[i] = u;
+        s1[0] += u * u;
+      });
+    }
+    block_sums<1>(s1, c.red, par);
+    rho = sqrt(s1[0]);
     if (adaptive ? rho <= stop_abs : rho < tol_abs) return used;
     if (itr == 0) rho_tol = rho * tol_rel;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) V[i] = r[i] / rho;
-    if (threadIdx.x == 0) {
-      gs.g[0] = rho;
-      for (int i = 1; i <= mr; ++i) gs.g[i] = 0.0;
-      for (int i = 0; i <= mr; ++i)
-        for (int j = 0; j < mr; ++j) gs.h[i][j] = 0.0;
+    double scale = 1.0 / rho;  // of the newest basis vector, applied when a step reads it
+#pragma unroll 1
+    for (int t = tid; t < M; t += nt) {
+      const int i = vis_row(c, t);
+      V[i] = r[i] * scale;
     }
-    __syncthreads();
+    if (tid == 0) {
+      gs.g[0] = rho;
+#pragma unroll 1
+      for (int i = 1; i <= mr; ++i) gs.g[i] = 0.0;
+    }
     int k_copy = 0;
     bool stop = false;
+#pragma unroll 1
     for (int k = 0; k < mr; ++k) {
       k_copy = k;
       double *vk = V + (size_t)k * N, *vk1 = V + (size_t)(k + 1) * N;
+      double s[2] = {0.0, 0.0};  // |K z|^2 and its product with V_0
       if (flexible) {
         T *zk = c.Z + (size_t)k * N;
-        precond(c, vk, zk);
-        // A z_k in FP64 (z widened)
-        for (int i = threadIdx.x; i < N; i += blockDim.x) c.w[i] = (double)zk[i];
-        __syncthreads();
-        spmv_ref(c, c.w, vk1);
+        double *w = c.w;
+        precond(c, [&](int i) { return vk[i]; }, [&](int i, T v) {
+          zk[i] = v;
+          w[i] = (double)v;  // widened for K z in FP64
+        });
+        BQ_T0(c);
+#pragma unroll 1
+        for (int t = tid; t < M; t += nt) {
+          const int i = vis_row(c, t);
+          const double v = spmv_row(c, w, i);
+          vk1[i] = v;
+          s[0] += v * v;
+          s[1] += v * V[i];
+        }
+        BQ_T1(c, PH_SPMV);
       } else {
-        spmv_ref(c, vk, vk1);
-        precond(c, vk1, vk1);
-      }
-      const double av = sqrt(dot(c, vk1, vk1));
-      for (int j = 0; j <= k; ++j) {
-        const double hj = dot(c, vk1, V + (size_t)j * N);
-        for (int i = threadIdx.x; i < N; i += blockDim.x) vk1[i] -= hj * V[(size_t)j * N + i];
-        if (threadIdx.x == 0) gs.h[j][k] = hj;
         __syncthreads();
-      }
-      double hk1 = sqrt(dot(c, vk1, vk1));
-      if ((av + delta * hk1) == av) {
-        for (int j = 0; j <= k; ++j) {
-          const double ht = dot(c, vk1, V + (size_t)j * N);
-          for (int i = threadIdx.x; i < N; i += blockDim.x) vk1[i] -= ht * V[(size_t)j * N + i];
-          if (threadIdx.x == 0) gs.h[j][k] += ht;
-          __syncthreads();
-        }
-        hk1 = sqrt(dot(c, vk1, vk1));
-      }
-      if (hk1 != 0.0)
-        for (int i = threadIdx.x; i < N; i += blockDim.x) vk1[i] = vk1[i] / hk1;
-      if (threadIdx.x == 0) {
-        gs.h[k + 1][k] = hk1;
-        if (0 < k) {
-          for (int j = 0; j < k; ++j) {  // previous Givens rotations
-            const double g1 = gs.cs[j] * gs.h[j][k] - gs.sn[j] * gs.h[j + 1][k];
-            const double g2 = gs.sn[j] * gs.h[j][k] + gs.cs[j] * gs.h[j + 1][k];
-            gs.h[j][k] = g1;
-            gs.h[j + 1][k] = g2;
+        {
+          BQ_T0(c);
+#pragma unroll 1
+          for (int t = tid; t < M; t += nt) {
+            const int i = vis_row(c, t);
+            vk1[i] = spmv_row(c, vk, i);
           }
+          BQ_T1(c, PH_SPMV);
         }
-        const double mu = sqrt(gs.h[k][k] * gs.h[k][k] + gs.h[k + 1][k] * gs.h[k + 1][k]);
+        precond(c, [&](int i) { return vk1[i]; }, [&](int i, T v) {
+          const double u = (double)v;
+          vk1[i] = u;
+          s[0] += u * u;
+          s[1] += u * V[i];
+        });
+      }
+      block_sums<2>(s, c.red, par);
+      const double av = sqrt(s[0]);
+      double hj = s[1], hk1 = 0.0;
+#pragma unroll 1
+      for (int j = 0; j <= k; ++j) {  // modified Gram-Schmidt, each pass forming the next product
+        const double *vj = V + (size_t)j * N, *vn = V + (size_t)(j + 1) * N;
+        if (tid == 0) gs.h[j][k] = hj;
+        double p[1] = {0.0};
+#pragma unroll 1
+        for (int t = tid; t < M; t += nt) {
+          const int i = vis_row(c, t);
+          const double v = vk1[i] - hj * vj[i];
+          vk1[i] = v;
+          p[0] += j < k ? v * vn[i] : v * v;
+        }
+        block_sums<1>(p, c.red, par);
+        hj = p[0];
+      }
+      hk1 = sqrt(hj);
+      if ((av + delta * hk1) == av) {  // reorthogonalisation
+#pragma unroll 1
+        for (int j = 0; j <= k; ++j) {
+          const double *vj = V + (size_t)j * N;
+          double p[1] = {0.0};
+#pragma unroll 1
+          for (int t = tid; t < M; t += nt) {
+            const int i = vis_row(c, t);
+            p[0] += vk1[i] * vj[i];
+          }
+          block_sums<1>(p, c.red, par);
+#pragma unroll 1
+          for (int t = tid; t < M; t += nt) {
+            const int i = vis_row(c, t);
+            vk1[i] -= p[0] * vj[i];
+          }
+          if (tid == 0) gs.h[j][k] += p[0];
+        }
+        double p[1] = {0.0};
+#pragma unroll 1
+        for (int t = tid; t < M; t += nt) {
+          const double v = vk1[vis_row(c, t)];
+          p[0] += v * v;
+        }
+        block_sums<1>(p, c.red, par);
+        hk1 = sqrt(p[0]);
+      }
+      if (tid == 0) {
+        double hk = hk1;
+#pragma unroll 1
+        for (int j = 0; j < k; ++j) {  // previous Givens rotations
+          const double g1 = gs.cs[j] * gs.h[j][k] - gs.sn[j] * gs.h[j + 1][k];
+          const double g2 = gs.sn[j] * gs.h[j][k] + gs.cs[j] * gs.h[j + 1][k];
+          gs.h[j][k] = g1;
+          gs.h[j + 1][k] = g2;
+        }
+        const double h0 = gs.h[k][k], mu = sqrt(h0 * h0 + hk * hk);
         gs.scal[0] = mu;
         if (mu != 0.0) {
-          gs.cs[k] = gs.h[k][k] / mu;
-          gs.sn[k] = -gs.h[k + 1][k] / mu;
-          gs.h[k][k] = gs.cs[k] * gs.h[k][k] - gs.sn[k] * gs.h[k + 1][k];
-          gs.h[k + 1][k] = 0.0;
-          const double g1 = gs.cs[k] * gs.g[k] - gs.sn[k] * gs.g[k + 1];
-          const double g2 = gs.sn[k] * gs.g[k] + gs.cs[k] * gs.g[k + 1];
-          gs.g[k] = g1;
-          gs.g[k + 1] = g2;
+          const double im = 1.0 / mu, cs = h0 * im, sn = -hk * im;
+          gs.cs[k] = cs;
+          gs.sn[k] = sn;
+          gs.h[k][k] = cs * h0 - sn * hk;
+          const double g0 = gs.g[k], gk1 = gs.g[k + 1];
+          gs.g[k] = cs * g0 - sn * gk1;
+          gs.g[k + 1] = sn * g0 + cs * gk1;
         }
       }
       __syncthreads();
@@ -1192,23 +1811,34 @@ __device__ int refine(Ctx<T> &c, const double *b, double *x, int itr_max, int mr
       used++;
       stop = adaptive ? rho <= stop_abs : (rho <= rho_tol && rho <= tol_abs);
       if (stop) break;
+      if (k + 1 < mr && hk1 != 0.0) {
+        scale = 1.0 / hk1;
+#pragma unroll 1
+        for (int t = tid; t < M; t += nt) vk1[vis_row(c, t)] *= scale;
+      }
     }
     const int k = k_copy;
     if (gs.h[k][k] == 0.0) return used;
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
       gs.y[k] = gs.g[k] / gs.h[k][k];
+#pragma unroll 1
       for (int i = k - 1; 0 <= i; i--) {
         double yi = gs.g[i];
+#pragma unroll 1
         for (int j = i + 1; j < k + 1; j++) yi = yi - gs.h[i][j] * gs.y[j];
         gs.y[i] = yi / gs.h[i][i];
       }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+#pragma unroll 1
+    for (int t = tid; t < M; t += nt) {
+      const int i = vis_row(c, t);
       double acc = 0.0;
       if (flexible)
+#pragma unroll 1
         for (int j = 0; j <= k; ++j) acc += (double)c.Z[(size_t)j * N + i] * gs.y[j];
       else
+#pragma unroll 1
         for (int j = 0; j <= k; ++j) acc += V[(size_t)j * N + i] * gs.y[j];
       x[i] += acc;
     }
@@ -1218,147 +1848,185 @@ __device__ int refine(Ctx<T> &c, const double *b, double *x, int itr_max, int mr
   return used;
 }
 
+// x = M^-1 b, then refine; hidden rows of x are zero.  Returns the Krylov steps.
+template <class T>
+__device__ __noinline__ int solve_refined(Ctx<T> &, const double *b, double *x, int itr_max, int mr, bool flexible, bool adaptive,
+                             double rtol, double tol_abs, double tol_rel) {
+  Ctx<T> &c = ctx<T>();
+  hidden_rows(c, [&](int i) { x[i] = 0.0; });
+  precond(c, [&](int i) { return b[i]; }, [&](int i, T v) { x[i] = (double)v; });
+  return refine(c, b, x, itr_max, mr, flexible, adaptive, rtol, tol_abs, tol_rel);
+}
+
 // ---- NASOQ on one problem ------------------------------------------------------
 // Marks the supernodes on the elimination-tree path from supernode s to the
-// root and appends them to mlist (the reference marks the visible ones of its
-// edited tree, which are a subset; refactoring an unchanged supernode
-// reproduces it).  Thread 0 only.
+// root for the next refactorization (the reference marks the visible ones of
+// its edited tree, which are a subset; refactoring an unchanged supernode
+// reproduces it).  A marked supernode's path is marked, or being marked by
+// another thread, already.
 template <class T> __device__ void mark_path(Ctx<T> &c, int s) {
-  for (; s >= 0; s = c.sparent[s])
-    if (!c.mark[s]) {
-      c.mark[s] = 1;
-      c.mlist[(*c.nmark)++] = s;
-    }
+  while (s >= 0 && !c.mark[s]) {
+    c.mark[s] = 1;
+    s = c.sparent[s];
+  }
 }
 
 // KKT edit of constraint k (reference edit_kkt -> add_del_matrix_qp,
 // linear_solver_wrapper.cpp:1020-1137): the constraint's entries become
 // visible / hidden in both value copies and in the descendant masks of its
 // targets, and the paths of its column and of its variables are marked for
-// the next partial refactorization.  Thread 0 only.
-template <class T> __device__ void edit_constraint(Ctx<T> &c, int k, bool add) {
+// the next partial refactorization.  One thread per constraint; several may
+// edit different constraints at once.
+template <class T> __device__ __noinline__ void edit_constraint(Ctx<T> &, int k, bool add) {
+  Ctx<T> &c = ctx<T>();
   c.act[k] = add ? 1 : 0;
   c.vis[c.con_sn[k]] = add ? 1 : 0;
+  c.nmark = 1;  // edits wait for a refactorization
+#pragma unroll 1
   for (int e = c.bt_ptr[k]; e < c.bt_ptr[k + 1]; ++e) {
     const int qq = c.bt_rpos[e];
     const double v = add ? c.kv[c.bt_q[e]] : 0.0;
-    c.Fv[qq] = v;
+    c.Fv[qq] = T(v);
     c.Rv[qq] = v;
   }
   const int row = c.base + k;
+#pragma unroll 1
   for (int qq = c.Rp[row]; qq < c.Rp[row + 1]; ++qq)
     if (c.Rj[qq] != row) {
       const double v = add ? c.kv[c.Rq[qq]] : 0.0;
-      c.Fv[qq] = v;
+      c.Fv[qq] = T(v);
       c.Rv[qq] = v;
     }
+#pragma unroll 1
   for (int e = c.con_ptr[k]; e < c.con_ptr[k + 1]; ++e) {
     const int tg = c.con_tgt[2 * e], bit = c.con_tgt[2 * e + 1];
     if (bit < 64) {
-      if (add) c.cmask[tg] |= 1ull << bit;
-      else c.cmask[tg] &= ~(1ull << bit);
+      if (add) atomicOr(c.cmask + tg, 1ull << bit);
+      else atomicAnd(c.cmask + tg, ~(1ull << bit));
     }
   }
   mark_path(c, c.con_sn[k]);
+#pragma unroll 1
   for (int e = c.bt_ptr[k]; e < c.bt_ptr[k + 1]; ++e) mark_path(c, c.col2sup[c.iperm[c.bt_var[e]]]);
 }
 
-// Marks every supernode (visible ones only when `only_visible`), in
-// ascending order.
-template <class T> __device__ void mark_all(Ctx<T> &c, bool only_visible) {
-  int base = 0;
-  for (int q0 = 0; q0 < c.ns; q0 += blockDim.x) {
-    const int q = q0 + threadIdx.x;
-    const int f = (q < c.ns && (!only_visible || c.vis[q])) ? 1 : 0;
-    if (q < c.ns) c.mark[q] = (uint8_t)f;
-    const unsigned bal = __ballot_sync(0xffffffffu, f);
-    const int wpre = __popc(bal & ((1u << lane_id()) - 1u));
-    if (lane_id() == 0) c.redi[warp_id()] = __popc(bal);
-    __syncthreads();
-    int before = 0, total = 0;
-    for (int t = 0; t < num_warps(); ++t) {
-      if (t < warp_id()) before += c.redi[t];
-      total += c.redi[t];
-    }
-    if (f) c.mlist[base + before + wpre] = q;
-    base += total;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *c.nmark = base;
+// Every visible supernode is to be factored.
+template <class T> __device__ void mark_visible(Ctx<T> &c) {
+#pragma unroll 1
+  for (int s = threadIdx.x; s < c.ns; s += blockDim.x) c.mark[s] = c.vis[s];
   __syncthreads();
 }
 
-// Sorts mlist ascending (children before parents).  Thread 0; the lists of
-// partial refactorizations are a few tree paths long.
-template <class T> __device__ void sort_mlist(Ctx<T> &c) {
-  if (threadIdx.x == 0) {
-    const int m = *c.nmark;
-    for (int i = 1; i < m; ++i) {
-      const int v = c.mlist[i];
-      int j = i - 1;
-      while (j >= 0 && c.mlist[j] > v) {
-        c.mlist[j + 1] = c.mlist[j];
-        --j;
-      }
-      c.mlist[j + 1] = v;
-    }
-  }
+// mlist = the marked supernodes in ascending order (children before parents).
+// Each warp counts, then writes, its own stretch.
+template <class T> __device__ __noinline__ void collect_marked(Ctx<T> &) {
+  Ctx<T> &c = ctx<T>();
+  const int lane = lane_id(), wi = warp_id(), nw = num_warps(), ns = c.ns;
+  const int per = ((ns + nw - 1) / nw + 31) / 32 * 32;
+  const int t0 = min(wi * per, ns), t1 = min(t0 + per, ns);
+  int cnt = 0;
+#pragma unroll 1
+  for (int t = t0 + lane; t < t1; t += 32) cnt += c.mark[t] ? 1 : 0;
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if (lane == 0) c.redi[wi] = cnt;
   __syncthreads();
+  int pos = 0, total = 0;
+#pragma unroll 1
+  for (int k = 0; k < nw; ++k) {
+    if (k < wi) pos += c.redi[k];
+    total += c.redi[k];
+  }
+#pragma unroll 1
+  for (int tb = t0; tb < t1; tb += 32) {
+    const int t = tb + lane;
+    const bool v = t < t1 && c.mark[t] != 0;
+    const unsigned bal = __ballot_sync(0xffffffffu, v);
+    if (v) c.mlist[pos + __popc(bal & ((1u << lane) - 1u))] = t;
+    pos += __popc(bal);
+  }
+  if (threadIdx.x == 0) c.nmark = total;
+  __syncthreads();
+}
+
+// The marked supernodes factored again, and the solves' lists brought up to date.
+template <class T> __device__ __noinline__ void refactor(Ctx<T> &) {
+  Ctx<T> &c = ctx<T>();
+  collect_marked(c);
+  factor_marked(c);
+  build_vlist(c);
 }
 
 // Slot state of a problem whose group shares one factorization: the factor,
 // its pivoting state and both value copies of K with every inequality
 // hidden, copied from the group's base slot; visibility likewise.
-template <class T> __device__ void copy_base(Ctx<T> &c, const unsigned char *bs, const BSlot &L, const BPat &pt) {
+template <class T> __device__ __noinline__ void copy_base(Ctx<T> &, const unsigned char *bs, const BSlot &L, const BPat &pt) {
+  Ctx<T> &c = ctx<T>();
   const int tid = threadIdx.x, nt = blockDim.x, N = c.N;
   const T *bL = reinterpret_cast<const T *>(bs + L.o_L);
   const T *bD = reinterpret_cast<const T *>(bs + L.o_D);
+  const T *bS = reinterpret_cast<const T *>(bs + L.o_S);
+  const T *bG = reinterpret_cast<const T *>(bs + L.o_G);
   const int *bls = reinterpret_cast<const int *>(bs + L.o_ls);
   const int *bperm = reinterpret_cast<const int *>(bs + L.o_perm);
   const int *biperm = reinterpret_cast<const int *>(bs + L.o_iperm);
   const int *blperm = reinterpret_cast<const int *>(bs + L.o_lperm);
-  const double *bF = reinterpret_cast<const double *>(bs + L.o_Fv);
+  const T *bF = reinterpret_cast<const T *>(bs + L.o_Fv);
   const double *bR = reinterpret_cast<const double *>(bs + L.o_Rv);
   const unsigned long long *bmask = reinterpret_cast<const unsigned long long *>(bs + L.o_cmask);
-  for (int i = tid; i < pt.xsize; i += nt) c.L[i] = bL[i];
-  for (int i = tid; i < 2 * N; i += nt) c.D[i] = bD[i];
-  for (int i = tid; i < pt.ssize; i += nt) c.ls[i] = bls[i];
+#pragma unroll 4
+  for (int i = tid; i < pt.lsize; i += nt) c.L[i] = bL[i];
+#pragma unroll 4
+  for (int i = tid; i < pt.sbsize; i += nt) c.S[i] = bS[i];
+#pragma unroll 4
+  for (int i = tid; i < pt.gsize; i += nt) c.G[i] = bG[i];
+#pragma unroll 4
+  for (int i = tid; i < pt.rsize; i += nt) c.ls[i] = bls[i];
+#pragma unroll 4
   for (int i = tid; i < N; i += nt) {
+#pragma unroll 1
+    for (int k = 0; k < 3; ++k) c.D[k * N + i] = bD[k * N + i];
     c.perm[i] = bperm[i];
     c.iperm[i] = biperm[i];
     c.lperm[i] = blperm[i];
   }
+#pragma unroll 4
   for (int i = tid; i < c.nnzR; i += nt) {
     c.Fv[i] = bF[i];
     c.Rv[i] = bR[i];
   }
+#pragma unroll 4
   for (int s = tid; s < c.ns; s += nt) {
     c.piv[s] = bs[L.o_piv + s];
     c.cmask[s] = bmask[s];
     c.mark[s] = 0;
     c.vis[s] = c.sn_con[s] < 0 ? 1 : 0;
   }
-  if (tid == 0) *c.nmark = 0;
+  if (tid == 0) c.nmark = 0;
   __syncthreads();
 }
 
 // Visibility, descendant masks and both value copies of K from the active set.
-template <class T> __device__ void load_state(Ctx<T> &c) {
+template <class T> __device__ __noinline__ void load_state(Ctx<T> &) {
+  Ctx<T> &c = ctx<T>();
+#pragma unroll 1
   for (int s = threadIdx.x; s < c.ns; s += blockDim.x) {
     const int k = c.sn_con[s];
     c.vis[s] = (k < 0 || c.act[k]) ? 1 : 0;
     c.cmask[s] = 0ull;
   }
   __syncthreads();
+#pragma unroll 1
   for (int k = threadIdx.x; k < c.mineq; k += blockDim.x)
     if (c.act[k])
+#pragma unroll 1
       for (int e = c.con_ptr[k]; e < c.con_ptr[k + 1]; ++e) {
         const int bit = c.con_tgt[2 * e + 1];
         if (bit < 64) atomicOr(c.cmask + c.con_tgt[2 * e], 1ull << bit);
       }
+#pragma unroll 1
   for (int qq = threadIdx.x; qq < c.nnzR; qq += blockDim.x) {
     const int vq = c.Rq[qq];
-    c.Fv[qq] = fact_val(c, vq);
+    c.Fv[qq] = T(fact_val(c, vq));
     c.Rv[qq] = ref_val(c, vq);
   }
   __syncthreads();
@@ -1367,74 +2035,46 @@ template <class T> __device__ void load_state(Ctx<T> &c) {
 }  // namespace
 
 template <class T>
-__global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double red[32];
-  __shared__ int redi[32];
-  __shared__ int s_status, s_prob;
-  __shared__ GmresSmall gs;
+__global__ void __launch_bounds__(BT_MAX_THREADS, 2) k_nasoq_batch(BArgs a) {
+  __shared__ int s_prob;
   __shared__ int s_int[8];
   __shared__ double s_dbl[8];
-  __shared__ int s_nmark;
-  __shared__ Ctx<T> sc;  // the problem's context, read by every thread
-  __shared__ unsigned long long s_cyc[PH_N];
+  Ctx<T> &c = ctx<T>();
+  double *red = c.red;
+  int *redi = c.redi;
   const int tid = threadIdx.x, nt = blockDim.x;
-  if (tid < PH_N) s_cyc[tid] = 0;
+  if (tid < PH_N) c.cyc[tid] = 0;
   // shared-memory carve-up (sizes from the largest pattern of the batch)
-  auto up16 = [](size_t v) { return (v + 15) / 16 * 16; };
-  unsigned char *sp = smem;
-  int *map = reinterpret_cast<int *>(sp);
-  sp += up16((size_t)a.N_max * sizeof(int));
-  T *xs = reinterpret_cast<T *>(sp);
-  sp += up16((size_t)a.N_max * sizeof(T));
-  T *Bm = reinterpret_cast<T *>(sp);
-  sp += up16((size_t)a.nr_max * a.w_max * sizeof(T));
-  T *rowbuf = reinterpret_cast<T *>(sp);
-  sp += up16((size_t)a.w_max * 32 * sizeof(T));
-  T *Dsm = reinterpret_cast<T *>(sp);
-  sp += up16((size_t)a.w_max * sizeof(T));
-  T *Esm = reinterpret_cast<T *>(sp);
-  sp += up16((size_t)a.w_max * sizeof(T));
-  int *lp = reinterpret_cast<int *>(sp);
-  sp += up16((size_t)a.w_max * sizeof(int));
-  T *Binv = reinterpret_cast<T *>(sp);
-  sp += up16((size_t)a.w_max * a.w_max * sizeof(T));
-  int *vlvl = reinterpret_cast<int *>(sp);
-  sp += up16((size_t)(a.nlev_max + 1) * sizeof(int));
-  int *vmid = reinterpret_cast<int *>(sp);
-  sp += up16((size_t)(a.nlev_max + 1) * sizeof(int));
-  int *vfill = reinterpret_cast<int *>(sp);
-  sp += up16((size_t)2 * (a.nlev_max + 1) * sizeof(int));
-  uint8_t *vis = sp;
-  sp += up16((size_t)a.ns_max);
-  uint8_t *act = sp;
-  sp += up16((size_t)a.mi_max);
-  const int wcap = min(a.w_max, 32), rcap = min(a.nr_max, 32);
-  T *wB = nullptr, *wD = nullptr, *wE = nullptr, *wwk = nullptr;
-  int *wlp = nullptr;
-  if (a.warp_factor) {
-    wB = reinterpret_cast<T *>(sp);
-    sp += up16((size_t)WF_WARPS * wcap * rcap * sizeof(T));
-    wD = reinterpret_cast<T *>(sp);
-    sp += up16((size_t)WF_WARPS * wcap * sizeof(T));
-    wE = reinterpret_cast<T *>(sp);
-    sp += up16((size_t)WF_WARPS * wcap * sizeof(T));
-    wlp = reinterpret_cast<int *>(sp);
-    sp += up16((size_t)WF_WARPS * wcap * sizeof(int));
-    wwk = reinterpret_cast<T *>(sp);
-    sp += up16((size_t)WF_WARPS * 64 * sizeof(T));
-  }
-  unsigned char *stage = sp;  // the factor and row lists of a problem that fits
+  unsigned sp = BATCH_CTX_BYTES;
+  auto take = [&](size_t bytes) {
+    const unsigned o = sp;
+    sp += (unsigned)((bytes + 15) / 16 * 16);
+    return o;
+  };
+  const unsigned o_map = take((size_t)a.N_max * sizeof(T));  // the row map of a factorization, xo of the solves
+  const unsigned o_xs = take((size_t)a.N_max * sizeof(T));
+  const unsigned o_rowbuf = take(batch_rowbuf(a) * sizeof(T));
+  const unsigned o_D = take((size_t)a.w_max * sizeof(T)), o_E = take((size_t)a.w_max * sizeof(T));
+  const unsigned o_lp = take((size_t)a.w_max * sizeof(int));
+  const unsigned o_lvl = take((size_t)3 * a.nlev_max * sizeof(int4));
+  const unsigned o_vseg = take((size_t)(2 * a.nlev_max + 2) * sizeof(int));
+  const unsigned o_vis = take((size_t)a.ns_max), o_mark = take((size_t)a.ns_max), o_act = take((size_t)a.mi_max);
+  // blocks of the factorization: the CTA's, or one set per warp in the same memory
+  const int wcap = a.warp_factor ? min(a.w_max, 32) : 0, rcap = a.warp_factor ? min(a.nr_max, 32) : 0;
+  const int wstride = wcap * (rcap + wcap + 4);
+  const unsigned o_B = take(batch_block_bytes(a, sizeof(T)));
+  unsigned char *stage = Sh<unsigned char>{sp};  // the factor and row lists of a problem that fits
 
   unsigned char *const own_slot = a.slots + (size_t)blockIdx.x * a.slot.bytes;
   const bool build_bases = a.mode == 1;
+#pragma unroll 1
   for (;;) {
     if (tid == 0) {
       const int qi = atomicAdd(a.head, 1);
       if (build_bases) s_prob = qi < a.nbase ? qi : -1;  // a group
       else s_prob = qi < a.nprob ? a.order[qi] : -1;
-      s_status = 0;
-      s_nmark = 0;
+      c.status = 0;
+      c.nmark = 0;
     }
     __syncthreads();
     if (s_prob < 0) break;
@@ -1445,7 +2085,6 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
     unsigned char *const slot = build_bases ? a.bases + (size_t)grp * a.slot.bytes : own_slot;
     const BProb &P = a.probs[pi];
     const BPat &pt = a.pats[P.pat];
-    Ctx<T> &c = sc;
     if (tid == 0) {
       const int *ip = a.ipool;
       c.n = pt.n;
@@ -1462,8 +2101,6 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       c.col2sup = ip + pt.o_col2sup;
       c.lpi = ip + pt.o_lpi;
       c.lpx = ip + pt.o_lpx;
-      c.lvl_ptr = ip + pt.o_lvl_ptr;
-      c.lvl_sn = ip + pt.o_lvl_sn;
       c.lev = ip + pt.o_lev;
       c.Rp = ip + pt.o_Rp;
       c.Rj = ip + pt.o_Rj;
@@ -1482,7 +2119,18 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       c.prec = reinterpret_cast<const int4 *>(ip + pt.o_prec);
       c.con_ptr = ip + pt.o_con_ptr;
       c.con_tgt = ip + pt.o_con_tgt;
-      c.sn_big = reinterpret_cast<const uint8_t *>(ip + pt.o_sn_big);
+      c.so_sn = ip + pt.o_so_sn;
+      c.so_seg = ip + pt.o_so_seg;
+      c.so_rec = reinterpret_cast<const int4 *>(ip + pt.o_so_rec);
+      c.so_e = reinterpret_cast<const int4 *>(ip + pt.o_so_e);
+      c.so_f = reinterpret_cast<const int4 *>(ip + pt.o_so_f);
+      c.so_b = reinterpret_cast<const int4 *>(ip + pt.o_so_b);
+      c.so_g = reinterpret_cast<const int2 *>(ip + pt.o_so_g);
+      c.so_gj = ip + pt.o_so_gj;
+      c.so_gs = ip + pt.o_so_gs;
+      c.gidx = ip + pt.o_gidx;
+      c.G = reinterpret_cast<T *>(slot + a.slot.o_G);
+      c.n1 = pt.n1;
       c.kv = a.dpool + P.o_kv;
       c.q = a.dpool + P.o_q;
       c.bq = a.dpool + P.o_b;
@@ -1491,24 +2139,29 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       c.reg = P.reg;
       c.reg32 = P.reg32;
       // the factor and the row lists live in shared memory when they fit
-      const size_t lbytes = ((size_t)pt.xsize * sizeof(T) + 15) / 16 * 16;
-      if (!build_bases && lbytes + (size_t)pt.ssize * sizeof(int) <= (size_t)a.stage_bytes) {
-        c.L = reinterpret_cast<T *>(stage);
-        c.ls = reinterpret_cast<int *>(stage + lbytes);
+      const size_t lbytes = ((size_t)pt.lsize * sizeof(T) + 15) / 16 * 16, sbytes = (size_t)pt.sbsize * sizeof(T);
+      if (!build_bases && lbytes + sbytes + (size_t)pt.rsize * sizeof(int) <= (size_t)a.stage_bytes) {
+        c.S = reinterpret_cast<T *>(stage);
+        c.L = reinterpret_cast<T *>(stage + sbytes);
+        c.ls = reinterpret_cast<int *>(stage + sbytes + lbytes);
       } else {
         c.L = reinterpret_cast<T *>(slot + a.slot.o_L);
+        c.S = reinterpret_cast<T *>(slot + a.slot.o_S);
         c.ls = reinterpret_cast<int *>(slot + a.slot.o_ls);
       }
       c.D = reinterpret_cast<T *>(slot + a.slot.o_D);
+      c.Di = c.D + c.N;
       c.perm = reinterpret_cast<int *>(slot + a.slot.o_perm);
       c.iperm = reinterpret_cast<int *>(slot + a.slot.o_iperm);
       c.lperm = reinterpret_cast<int *>(slot + a.slot.o_lperm);
-      c.mark = slot + a.slot.o_mark;
+      c.mark.off = o_mark;
+      c.lvl.off = o_lvl;
       c.piv = slot + a.slot.o_piv;
       c.alist = reinterpret_cast<int *>(slot + a.slot.o_alist);
-      c.vlist = reinterpret_cast<int *>(slot + a.slot.o_vlist);
+      c.vrec = reinterpret_cast<int4 *>(slot + a.slot.o_vrec);
+      c.arow = reinterpret_cast<int *>(slot + a.slot.o_arow);
       c.mlist = reinterpret_cast<int *>(slot + a.slot.o_mlist);
-      c.Fv = reinterpret_cast<double *>(slot + a.slot.o_Fv);
+      c.Fv = reinterpret_cast<T *>(slot + a.slot.o_Fv);
       c.Rv = reinterpret_cast<double *>(slot + a.slot.o_Rv);
       c.cmask = reinterpret_cast<unsigned long long *>(slot + a.slot.o_cmask);
       c.rhs = reinterpret_cast<double *>(slot + a.slot.o_rhs);
@@ -1518,32 +2171,25 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       c.V = reinterpret_cast<double *>(slot + a.slot.o_V);
       c.Z = reinterpret_cast<T *>(slot + a.slot.o_Z);
       c.tmp = reinterpret_cast<double *>(slot + a.slot.o_tmp);
-      c.map = map;
-      c.xs = xs;
-      c.B = Bm;
-      c.rowbuf = rowbuf;
-      c.Dsm = Dsm;
-      c.Esm = Esm;
-      c.Binv = Binv;
-      c.lp = lp;
-      c.wB = wB;
-      c.wD = wD;
-      c.wE = wE;
-      c.wlp = wlp;
-      c.wwk = wwk;
+      c.map.off = o_map;
+      c.xs.off = o_xs;
+      c.xo.off = o_map;
+      c.B.off = o_B;
+      c.rowbuf.off = o_rowbuf;
+      c.Dsm.off = o_D;
+      c.Esm.off = o_E;
+      c.Binv.off = o_B + (unsigned)(a.b_max * (int)sizeof(T));
+      c.lp.off = o_lp;
+      c.wB.off = o_B;
+      c.wstride = wstride;
+      c.wlp.off = o_B + (unsigned)(WF_WARPS * wstride * (int)sizeof(T));
       c.wcap = wcap;
       c.rcap = rcap;
       c.wf = a.warp_factor ? 1 : 0;
-      c.vis = vis;
-      c.act = act;
-      c.vlvl = vlvl;
-      c.vmid = vmid;
-      c.vfill = vfill;
-      c.nmark = &s_nmark;
-      c.red = red;
-      c.redi = redi;
-      c.status = &s_status;
-      c.cyc = a.prof ? s_cyc : nullptr;
+      c.vis.off = o_vis;
+      c.act.off = o_act;
+      c.vseg.off = o_vseg;
+      c.prof = a.prof ? 1 : 0;
     }
     __syncthreads();
     const long long tp0 = clock64();
@@ -1558,27 +2204,37 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
     // ---- set-up: pattern state into the slot (a problem of a group starts
     // from the group's factorization instead, below)
     if (build_bases || P.base < 0) {
+#pragma unroll 1
       for (int i = tid; i < N; i += nt) {
         const int p0 = ip[pt.o_perm0 + i];
         c.perm[i] = p0;
         c.iperm[p0] = i;
-        c.D[i] = T(0);
-        c.D[N + i] = T(0);
+#pragma unroll 1
+        for (int k = 0; k < 3; ++k) c.D[k * N + i] = T(0);
       }
-      for (int i = tid; i < pt.ssize; i += nt) c.ls[i] = ip[pt.o_ls0 + i];
-      for (int i = tid; i < pt.xsize; i += nt) c.L[i] = T(0);
+#pragma unroll 1
+      for (int i = tid; i < pt.rsize; i += nt) c.ls[i] = ip[pt.o_ls0 + i];
+#pragma unroll 1
+      for (int i = tid; i < pt.lsize; i += nt) c.L[i] = T(0);
+#pragma unroll 1
+      for (int i = tid; i < pt.sbsize; i += nt) c.S[i] = T(0);
+#pragma unroll 1
+      for (int i = tid; i < pt.gsize; i += nt) c.G[i] = T(0);
+#pragma unroll 1
       for (int s = tid; s < c.ns; s += nt) {
         c.mark[s] = 0;
         c.piv[s] = 0;
       }
     }
+#pragma unroll 1
     for (int k = tid; k < mineq; k += nt) c.act[k] = 0;
+#pragma unroll 1
+    for (int l = tid; l < 3 * c.nlev; l += nt) c.lvl[l] = reinterpret_cast<const int4 *>(ip + pt.o_lvl)[l];
     __syncthreads();
     if (build_bases) {  // every inequality hidden: the cold start's factorization
       load_state(c);
-      build_vlist(c);
-      mark_all(c, true);
-      factor_marked(c);
+      mark_visible(c);
+      refactor(c);
       continue;
     }
     const unsigned char *const bslot = P.base >= 0 ? a.bases + (size_t)P.base * a.slot.bytes : nullptr;
@@ -1587,6 +2243,7 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
     // the equality-constrained solution on it (below)
     const bool warm = P.ws_n >= 0;
     if (warm) {
+#pragma unroll 1
       for (int t = tid; t < P.ws_n; t += nt) {
         const int k = as_out[t];
         if (k >= 0 && k < mineq) c.act[k] = 1;
@@ -1600,30 +2257,27 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
     // and is skipped by the solves.  After the first warm round, dropped
     // constraints are hidden by the partial refactorization of their paths.
     bool cold = !warm, full = true;
+#pragma unroll 1
     for (int round = 0; round < 5; ++round) {
-      const long long tf0 = c.cyc ? clock64() : 0;
+      const long long tf0 = c.prof ? clock64() : 0;
       if (full && bslot) {
         // the group's cold factorization, then the active rows made visible
         // by partial refactorization of their paths
         copy_base(c, bslot, a.slot, pt);
-        if (tid == 0)
-          for (int k = 0; k < mineq; ++k)
-            if (c.act[k]) edit_constraint(c, k, true);
+#pragma unroll 1
+        for (int k = tid; k < mineq; k += nt)
+          if (c.act[k]) edit_constraint(c, k, true);
         __syncthreads();
-        sort_mlist(c);
-        factor_marked(c);
-        build_vlist(c);
+        refactor(c);
       } else if (full) {
         load_state(c);
-        build_vlist(c);
-        mark_all(c, true);
-        factor_marked(c);
+        mark_visible(c);
+        refactor(c);
       } else {
-        sort_mlist(c);
-        factor_marked(c);
-        build_vlist(c);
+        refactor(c);
       }
-      if (c.cyc && tid == 0) c.cyc[PH_INIT_FACTOR] += (unsigned long long)(clock64() - tf0);
+      if (c.prof && tid == 0) c.cyc[PH_INIT_FACTOR] += (unsigned long long)(clock64() - tf0);
+#pragma unroll 1
       for (int i = tid; i < N; i += nt) {
         double v = 0.0;
         if (i < n) v = -c.q[i];
@@ -1632,69 +2286,73 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
         c.rhs[i] = v;
       }
       __syncthreads();
-      precond(c, c.rhs, c.sol);
       solves++;
-      steps += refine(c, c.rhs, c.sol, P.outer, P.inner, flexible, adaptive, a.refine_tol, P.tol_abs, P.tol_rel, gs);
+      steps += solve_refined(c, c.rhs, c.sol, P.outer, P.inner, flexible, adaptive, a.refine_tol, P.tol_abs, P.tol_rel);
       if (cold) break;
       // a proposed set that makes the KKT matrix singular (dependent
       // constraints): start cold instead
       int bad = 0;
+#pragma unroll 1
       for (int i = tid; i < N; i += nt)
         if (!isfinite(c.sol[i])) bad++;
       bad = block_sum_int(bad, redi);
-      if (bad > 0 || (s_status & (ST_ZERO_PIVOT | ST_NONFINITE))) {
+      if (bad > 0 || (c.status & (ST_ZERO_PIVOT | ST_NONFINITE))) {
+#pragma unroll 1
         for (int k = tid; k < mineq; k += nt) c.act[k] = 0;
         __syncthreads();
-        if (tid == 0) s_status = 0;
+        if (tid == 0) c.status = 0;
         cold = true;
         full = true;
         __syncthreads();
         continue;
       }
       // drop proposed constraints with negative multipliers, then solve again
-      if (tid == 0) {
-        int nd = 0;
-        for (int k = 0; k < mineq; ++k)
-          if (c.act[k] && c.sol[c.base + k] < 0.0) {
-            edit_constraint(c, k, false);
-            nd++;
-          }
-        s_int[2] = nd;
-      }
-      __syncthreads();
-      const int ndrop = s_int[2];
+      int ndrop = 0;
+#pragma unroll 1
+      for (int k = tid; k < mineq; k += nt)
+        if (c.act[k] && c.sol[c.base + k] < 0.0) {
+          edit_constraint(c, k, false);
+          ndrop++;
+        }
+      ndrop = block_sum_int(ndrop, redi);
       warm_dropped += ndrop;
       if (ndrop == 0) break;
       full = false;
       if (round >= 2) {  // no consistent set after three rounds: cold start
+#pragma unroll 1
         for (int k = tid; k < mineq; k += nt) c.act[k] = 0;
-        if (tid == 0) {
-          for (int t = 0; t < *c.nmark; ++t) c.mark[c.mlist[t]] = 0;
-          *c.nmark = 0;
-        }
+#pragma unroll 1
+        for (int s = tid; s < c.ns; s += nt) c.mark[s] = 0;
+        if (tid == 0) c.nmark = 0;
         cold = true;
         full = true;
         __syncthreads();
       }
     }
+#pragma unroll 1
     for (int i = tid; i < n; i += nt) xv[i] = c.sol[i];
+#pragma unroll 1
     for (int i = tid; i < meq; i += nt) yv[i] = c.sol[n + i];
+#pragma unroll 1
     for (int k = tid; k < mineq; k += nt) zv[k] = c.act[k] ? c.sol[c.base + k] : 0.0;
     __syncthreads();
     if (tid == 0) {
+#pragma unroll 1
       for (int k = 0; k < mineq; ++k)
         if (c.act[k]) c.alist[nact++] = k;
       s_int[0] = nact;
     }
     __syncthreads();
     nact = s_int[0];
-    if (c.cyc && tid == 0) c.cyc[PH_INIT] += (unsigned long long)(clock64() - tp0);
+    if (c.prof && tid == 0) c.cyc[PH_INIT] += (unsigned long long)(clock64() - tp0);
 
     // ---- the dual active-set iteration (reference numeric_QP)
     int num_iter = 0, converged = 0, nxt_active = -1, nxt_drop = -1, to_add = 1;
     int typ = 0;  // 0 solve, 1 update (partial refactorization first)
     const double DMAX = DBL_MAX;
+#pragma unroll 1
     for (int pol = 0;; ++pol) {
+#pragma unroll 1
     for (;;) {
       if (num_iter > P.max_iter_nas) {
         converged = 0;
@@ -1706,8 +2364,10 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
         int viol = 0;
         double best = P.eps_abs;
         int bi = -1;
+#pragma unroll 1
         for (int k = tid; k < mineq; k += nt) {
           double t = 0.0;
+#pragma unroll 1
           for (int e = c.bt_ptr[k]; e < c.bt_ptr[k + 1]; ++e) t += c.kv[c.bt_q[e]] * xv[c.bt_var[e]];
           t -= c.dq[k];
           if (t > P.eps_abs) viol++;
@@ -1728,8 +2388,10 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
         }
         nxt_active = bi;
         // update_rhs (src/nasoq.cpp:880-889): the constraint's row as the rhs
+#pragma unroll 1
         for (int i = tid; i < N; i += nt) c.rhs[i] = 0.0;
         __syncthreads();
+#pragma unroll 1
         for (int e = c.bt_ptr[nxt_active] + tid; e < c.bt_ptr[nxt_active + 1]; e += nt)
           c.rhs[c.bt_var[e]] = c.kv[c.bt_q[e]];
         __syncthreads();
@@ -1738,23 +2400,21 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       // solve_kkt (src/nasoq.cpp:918-957)
       if (typ == 1) {
         BQ_T0(c);
-        sort_mlist(c);
-        factor_marked(c);
-        build_vlist(c);
+        refactor(c);
         typ = 0;
         BQ_T1(c, PH_FACTOR);
       }
       {
         BQ_T0(c);
-        precond(c, c.rhs, c.sol);
         solves++;
-        steps += refine(c, c.rhs, c.sol, P.outer, P.inner, flexible, adaptive, a.refine_tol, P.tol_abs, P.tol_rel, gs);
+        steps += solve_refined(c, c.rhs, c.sol, P.outer, P.inner, flexible, adaptive, a.refine_tol, P.tol_abs, P.tol_rel);
         BQ_T1(c, PH_REFINE);
       }
       const long long tu0 = clock64();
       // step lengths (src/nasoq.cpp:852-878)
       double dual_step = DMAX;
       int drop = -1;
+#pragma unroll 1
       for (int t = tid; t < nact; t += nt) {
         const int k = c.alist[t];
         const double lm = c.sol[c.base + k];
@@ -1770,6 +2430,7 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       if (drop < 0) dual_step = DMAX;
       if (tid == 0) {
         double bdotx = 0.0, ddotb = 0.0;
+#pragma unroll 1
         for (int e = c.bt_ptr[nxt_active]; e < c.bt_ptr[nxt_active + 1]; ++e) {
           bdotx += c.kv[c.bt_q[e]] * xv[c.bt_var[e]];
           ddotb += c.kv[c.bt_q[e]] * c.sol[c.bt_var[e]];
@@ -1789,8 +2450,11 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       const bool dual_only = prime_step == DMAX && step == dual_step;
       // update_primal / update_dual (src/nasoq.cpp:612-632)
       if (!dual_only)
+#pragma unroll 1
         for (int i = tid; i < n; i += nt) xv[i] = xv[i] - step * c.sol[i];
+#pragma unroll 1
       for (int i = tid; i < meq; i += nt) yv[i] -= step * c.sol[n + i];
+#pragma unroll 1
       for (int t = tid; t < nact; t += nt) {
         const int k = c.alist[t];
         zv[k] -= step * c.sol[c.base + k];
@@ -1810,9 +2474,11 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
         } else if (del >= 0) {
           edit_constraint(c, del, false);
           int pos = -1;
+#pragma unroll 1
           for (int t = 0; t < nact; ++t)
             if (c.alist[t] == del) pos = t;
           if (pos >= 0) {
+#pragma unroll 1
             for (int t = pos; t + 1 < nact; ++t) c.alist[t] = c.alist[t + 1];
             nact--;
           }
@@ -1829,7 +2495,7 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
         typ = 1;
       }
       num_iter++;
-      if (c.cyc && tid == 0) {
+      if (c.prof && tid == 0) {
         c.cyc[PH_UPDATE] += (unsigned long long)(clock64() - tu0);
         c.cyc[PH_ITER] += 1;
       }
@@ -1851,12 +2517,11 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
     // long trajectory its active set is settled, and its KKT norms decide the
     // status
     const double polish_tol = fmin(a.refine_tol, 1e-12);
-    if (*c.nmark > 0) {
-      sort_mlist(c);
-      factor_marked(c);
-      build_vlist(c);
+    if (c.nmark > 0) {
+      refactor(c);
     }
     typ = 0;
+#pragma unroll 1
     for (int i = tid; i < N; i += nt) {
       double v = 0.0;
       if (i < n) v = -c.q[i];
@@ -1865,18 +2530,20 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       c.rhs[i] = v;
     }
     __syncthreads();
-    precond(c, c.rhs, c.sol);
     solves++;
-    steps += refine(c, c.rhs, c.sol, P.outer, P.inner, flexible, adaptive, polish_tol, P.tol_abs, P.tol_rel, gs);
+    steps += solve_refined(c, c.rhs, c.sol, P.outer, P.inner, flexible, adaptive, polish_tol, P.tol_abs, P.tol_rel);
     // a negative multiplier: that constraint does not belong to the active
     // set of this point; drop it and solve again (at most three times)
+#pragma unroll 1
     for (int rep = 0; rep < 3; ++rep) {
       if (tid == 0) {
         int nd = 0;
+#pragma unroll 1
         for (int t = 0; t < nact;) {
           const int k = c.alist[t];
           if (c.sol[c.base + k] < 0.0) {
             edit_constraint(c, k, false);
+#pragma unroll 1
             for (int u = t; u + 1 < nact; ++u) c.alist[u] = c.alist[u + 1];
             nact--;
             nd++;
@@ -1890,28 +2557,32 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       __syncthreads();
       nact = s_int[0];
       if (s_int[2] == 0) break;
-      sort_mlist(c);
-      factor_marked(c);
-      build_vlist(c);
+      refactor(c);
+#pragma unroll 1
       for (int i = c.base + tid; i < N; i += nt)
         if (!c.act[i - c.base]) c.rhs[i] = 0.0;
       __syncthreads();
-      precond(c, c.rhs, c.sol);
       solves++;
-      steps += refine(c, c.rhs, c.sol, P.outer, P.inner, flexible, adaptive, polish_tol, P.tol_abs, P.tol_rel, gs);
+      steps += solve_refined(c, c.rhs, c.sol, P.outer, P.inner, flexible, adaptive, polish_tol, P.tol_abs, P.tol_rel);
     }
+#pragma unroll 1
     for (int k = tid; k < mineq; k += nt)
       if (!c.act[k]) zv[k] = 0.0;
+#pragma unroll 1
     for (int i = tid; i < n; i += nt) xv[i] = c.sol[i];
+#pragma unroll 1
     for (int i = tid; i < meq; i += nt) yv[i] = c.sol[n + i];
+#pragma unroll 1
     for (int t = tid; t < nact; t += nt) {
       const int k = c.alist[t];
       zv[k] = c.sol[c.base + k];
     }
     __syncthreads();
     int viol = 0;
+#pragma unroll 1
     for (int k = tid; k < mineq; k += nt) {
       double t = 0.0;
+#pragma unroll 1
       for (int e = c.bt_ptr[k]; e < c.bt_ptr[k + 1]; ++e) t += c.kv[c.bt_q[e]] * xv[c.bt_var[e]];
       if (t - c.dq[k] > P.eps_abs) viol++;
     }
@@ -1923,6 +2594,7 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
 
     // ---- results: objective and KKT norms (src/nasoq.cpp:712-728, 1013-1106)
     // Hx, Ax, Cx and H x + A^T y + C^T z from the original values
+#pragma unroll 1
     for (int i = tid; i < N; i += nt) {
       double v = 0.0;
       if (i < n) v = xv[i];
@@ -1934,8 +2606,10 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
     }
     __syncthreads();
     double quad = 0.0, lin = 0.0, lag = 0.0;
+#pragma unroll 1
     for (int i = tid; i < n; i += nt) {
       double hx = 0.0, full = 0.0;
+#pragma unroll 1
       for (int qq = c.Rp[i]; qq < c.Rp[i + 1]; ++qq) {
         const int j = c.Rj[qq];
         const double v = c.kv[c.Rq[qq]];
@@ -1947,8 +2621,10 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       lag = fmax(lag, fabs(full + c.q[i]));
     }
     double cons = 0.0, dual_obj = 0.0, nonneg = 0.0, comp = 0.0;
+#pragma unroll 1
     for (int k = tid; k < mineq; k += nt) {
       double t = 0.0;
+#pragma unroll 1
       for (int e = c.bt_ptr[k]; e < c.bt_ptr[k + 1]; ++e) t += c.kv[c.bt_q[e]] * xv[c.bt_var[e]];
       t -= c.dq[k];
       cons = fmax(cons, t < 0.0 ? 0.0 : t);
@@ -1956,14 +2632,17 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       nonneg = fmax(nonneg, zv[k] > 0.0 ? 0.0 : fabs(zv[k]));
       comp = fmax(comp, fabs(zv[k] * t));
     }
+#pragma unroll 1
     for (int r = tid; r < meq; r += nt) {
       double t = 0.0;
+#pragma unroll 1
       for (int e = c.eq_ptr[r]; e < c.eq_ptr[r + 1]; ++e) t += c.kv[c.eq_q[e]] * xv[c.eq_var[e]];
       cons = fmax(cons, fabs(t - c.bq[r]));
     }
     // a non-finite solution (non-finite data, or a breakdown the loop could
     // not recover from) is never reported as converged
     int nonfin = 0;
+#pragma unroll 1
     for (int i = tid; i < N; i += nt)
       if (!isfinite(c.tmp[i]) || !isfinite(c.w[i])) nonfin = 1;
     nonfin = block_sum_int(nonfin, redi);
@@ -1971,6 +2650,7 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
     lin = block_sum(lin, red);
     dual_obj = block_sum(dual_obj, red);
     double mx[4] = {lag, cons, nonneg, comp};
+#pragma unroll 1
     for (int m = 0; m < 4; ++m) {
       double v = mx[m];
 #pragma unroll
@@ -1980,6 +2660,7 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       __syncthreads();
       if (tid == 0) {
         double w = 0.0;
+#pragma unroll 1
         for (int t = 0; t < num_warps(); ++t) w = fmax(w, red[t]);
         s_dbl[m] = w;
       }
@@ -1987,12 +2668,13 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       mx[m] = s_dbl[m];
       __syncthreads();
     }
+#pragma unroll 1
     for (int t = tid; t < mineq; t += nt) as_out[t] = t < nact ? c.alist[t] : -1;
     if (tid == 0) {
       BResult &R = a.res[pi];
       R.num_iter = num_iter;
       R.active_size = nact;
-      R.flags = s_status | (nonfin ? ST_NONFINITE : 0);
+      R.flags = c.status | (nonfin ? ST_NONFINITE : 0);
       R.refine_steps = steps;
       R.solves = solves;
       R.warm_dropped = warm_dropped;
@@ -2010,11 +2692,11 @@ __global__ void __launch_bounds__(BT_MAX_THREADS) k_nasoq_batch(BArgs a) {
       else if (mx[1] <= P.eps_abs) st = 2;
       else st = 3;
       R.status = st;
-      if (c.cyc) c.cyc[PH_TOTAL] += (unsigned long long)(clock64() - tp0);
+      if (c.prof) c.cyc[PH_TOTAL] += (unsigned long long)(clock64() - tp0);
     }
     __syncthreads();
   }
-  if (a.prof && tid < PH_N) atomicAdd(a.prof + tid, s_cyc[tid]);
+  if (a.prof && tid < PH_N) atomicAdd(a.prof + tid, c.cyc[tid]);
 }
 
 // batch_fp64.cu compiles this file again with NQG_BATCH_FP64_UNIT defined for
@@ -2044,6 +2726,7 @@ __global__ void k_ws_scores(int nprob, BProb *probs, const BPat *pats, const int
   const float *sc = scores + (size_t)i * ld;
   int cnt = 0;
   const int mi = min(pt.mineq, ld);
+#pragma unroll 1
   for (int c0 = 0; c0 < mi; c0 += 32) {
     const int kk = c0 + lane;
     unsigned cand = __ballot_sync(0xffffffffu, kk < mi && sc[kk] > thr);
@@ -2052,11 +2735,13 @@ __global__ void k_ws_scores(int nprob, BProb *probs, const BPat *pats, const int
       cand &= cand - 1;
       const int ka = bt_ptr[k], kn = bt_ptr[k + 1] - ka;
       bool parallel = false;
+#pragma unroll 1
       for (int t = lane; t < cnt; t += 32) {
         const int j = as[t], ja = bt_ptr[j], jn = bt_ptr[j + 1] - ja;
         if (jn != kn || kn == 0) continue;
         bool same = true;
         const double r = kv[bt_q[ka]] / kv[bt_q[ja]];
+#pragma unroll 1
         for (int e = 0; e < kn && same; ++e)
           same = bt_var[ka + e] == bt_var[ja + e] &&
                  fabs(kv[bt_q[ka + e]] - r * kv[bt_q[ja + e]]) <= 1e-12 * fabs(kv[bt_q[ka + e]]);
@@ -2081,10 +2766,13 @@ __global__ void k_scatter_vectors(int nprob, const BProb *probs, const BPat *pat
   const BPat &pt = pats[P.pat];
   const int64_t oq = voff[3 * i], ob = voff[3 * i + 1], od = voff[3 * i + 2];
   if (oq >= 0)
+#pragma unroll 1
     for (int t = threadIdx.x; t < pt.n; t += blockDim.x) dpool[P.o_q + t] = stage[oq + t];
   if (ob >= 0)
+#pragma unroll 1
     for (int t = threadIdx.x; t < pt.meq; t += blockDim.x) dpool[P.o_b + t] = stage[ob + t];
   if (od >= 0)
+#pragma unroll 1
     for (int t = threadIdx.x; t < pt.mineq; t += blockDim.x) dpool[P.o_d + t] = stage[od + t];
 }
 
@@ -2113,16 +2801,9 @@ int batch_ws_clear(int nprob, BProb *probs, cudaStream_t st) {
 
 size_t batch_smem_bytes(const BArgs &a, size_t tsize) {
   auto up = [](size_t b) { return (b + 15) / 16 * 16; };
-  size_t wf = 0;
-  if (a.warp_factor) {
-    const size_t wcap = (size_t)std::min(a.w_max, 32), rcap = (size_t)std::min(a.nr_max, 32);
-    wf = up(WF_WARPS * wcap * rcap * tsize) + 2 * up(WF_WARPS * wcap * tsize) + up(WF_WARPS * wcap * sizeof(int)) +
-         up((size_t)WF_WARPS * 64 * tsize);
-  }
-  return up((size_t)a.N_max * sizeof(int)) + up((size_t)a.N_max * tsize) + up((size_t)a.nr_max * a.w_max * tsize) +
-         up((size_t)a.w_max * 32 * tsize) + 2 * up((size_t)a.w_max * tsize) + up((size_t)a.w_max * sizeof(int)) +
-         up((size_t)a.w_max * a.w_max * tsize) + 4 * up((size_t)(a.nlev_max + 1) * sizeof(int)) + up((size_t)a.ns_max) +
-         up((size_t)a.mi_max) + wf + (size_t)a.stage_bytes;
+  return BATCH_CTX_BYTES + 2 * up((size_t)a.N_max * tsize) + up(batch_rowbuf(a) * tsize) + 2 * up((size_t)a.w_max * tsize) +
+         up((size_t)a.w_max * sizeof(int)) + (size_t)a.nlev_max * 48 + up((size_t)(2 * a.nlev_max + 2) * sizeof(int)) +
+         2 * up((size_t)a.ns_max) + up((size_t)a.mi_max) + batch_block_bytes(a, tsize) + (size_t)a.stage_bytes;
 }
 
 #endif  // NQG_BATCH_FP64_UNIT

@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -42,9 +43,9 @@ struct HostPattern {
   BPat P{};
   nqg::Symbolic S;
   // integer arrays of this pattern, in BPat offset order (filled by build_pattern)
-  std::vector<int> super, sparent, col2sup, lpi, lpx, ls0, perm0, lvl_ptr, lvl_sn, lev, pair_ptr, pair_mid, pair_d,
+  std::vector<int> super, sparent, col2sup, lpi, lpx, ls0, perm0, lev, pair_ptr, pair_mid, pair_d,
       pair_lb, pair_ub, Rp, Rj, Rq, ent, bt_ptr, bt_var, bt_q, bt_rpos, sn_con, con_sn, eq_ptr, eq_var, eq_q,
-      snrec, prec, con_ptr, con_tgt, sn_big;
+      snrec, prec, con_ptr, con_tgt, so_sn, so_seg, so_rec, so_e, so_f, so_b, so_g, so_gj, so_gs, gidx, lvl;
   std::vector<int> diag_q;  // per column: value index of its diagonal
 };
 
@@ -104,7 +105,7 @@ void super_kkt(const HostQP &Q, nqg::Csc &K, std::vector<double> *vals) {
   }
 }
 
-std::string build_pattern(const HostQP &Q, HostPattern &H, const int nrelax[3], const double zrelax[3]) {
+std::string build_pattern(const HostQP &Q, HostPattern &H, const int nrelax[3], const double zrelax[3], int threads) {
   const int n = Q.n, meq = Q.meq, mineq = Q.mineq, N = n + meq + mineq, base = n + meq;
   nqg::Csc K;
   super_kkt(Q, K, nullptr);
@@ -158,14 +159,6 @@ std::string build_pattern(const HostQP &Q, HostPattern &H, const int nrelax[3], 
     maxl = std::max(maxl, lev[s]);
   }
   P.nlev = ns ? maxl + 1 : 0;
-  H.lvl_ptr.assign(P.nlev + 1, 0);
-  for (int s = 0; s < ns; ++s) H.lvl_ptr[lev[s] + 1]++;
-  for (int l = 0; l < P.nlev; ++l) H.lvl_ptr[l + 1] += H.lvl_ptr[l];
-  H.lvl_sn.assign(ns, 0);
-  {
-    std::vector<int> pos(H.lvl_ptr.begin(), H.lvl_ptr.end() - (P.nlev ? 1 : 0));
-    for (int s = 0; s < ns; ++s) H.lvl_sn[pos[lev[s]]++] = s;
-  }
   H.lev = lev;
   // descendant pairs from the elimination-tree reach (reference ereach_sn)
   nqg::Csc up;
@@ -257,32 +250,93 @@ std::string build_pattern(const HostQP &Q, HostPattern &H, const int nrelax[3], 
       if (H.bt_rpos[e] < 0) return "constraint entry missing from the symmetric pattern";
     }
   P.nnzR = H.Rp[N];
+  if (N >= 65536 || P.max_w >= 32768) return "pattern too large for the batched solver";  // packed records
+  // ---- values, row lists and work lists of the factorization and the solves
+  const auto s_ld = [](int w) { return (w + 3) & ~3; };
+  const auto width = [&](int s) { return S.super[s + 1] - S.super[s]; };
+  const auto nrows = [&](int s) { return (int)(S.lpi[s + 1] - S.lpi[s]); };
+  // single columns that never hide, of at most 32 rows: 32 at a time
+  const auto packed = [&](int s) { return width(s) == 1 && H.sn_con[s] < 0 && nrows(s) <= nqg::BATCH_SN_LONG; };
+  // single columns of a level, spread out: neighbours in the tree push into the
+  // same rows, and lanes of one warp that do so wait for one another
+  const auto spread = [](const std::vector<int> &v) {
+    std::vector<int> o;
+    const int m = (int)v.size(), rows = (m + 31) / 32;
+    for (int a = 0; a < rows; ++a)  // every rows-th one: 32 lanes reach across the whole group
+      for (int t = a; t < m; t += rows) o.push_back(v[t]);
+    return o;
+  };
+  std::vector<std::vector<int>> packs((size_t)P.nlev), shorts((size_t)P.nlev), longs((size_t)P.nlev), wide((size_t)P.nlev);
+  for (int s = 0; s < ns; ++s)
+    (width(s) > 1 ? wide : packed(s) ? packs : nrows(s) <= nqg::BATCH_SN_LONG ? shorts : longs)[lev[s]].push_back(s);
+  std::vector<int> voff(ns, 0), roff(ns, 0);
+  int64_t lsz = 0, rsz = 0, sb = 0;
+  for (int l = 0; l < P.nlev; ++l) {
+    packs[l] = spread(packs[l]);
+    shorts[l] = spread(shorts[l]);
+    for (size_t g = 0; g < packs[l].size(); g += 32) {
+      int most = 0;
+      for (size_t t = g; t < std::min(g + 32, packs[l].size()); ++t) {
+        const int s = packs[l][t];
+        voff[s] = (int)(lsz + (t - g));
+        roff[s] = (int)(rsz + (t - g));
+        most = std::max(most, nrows(s));
+      }
+      lsz += 32 * (int64_t)most;
+      rsz += 32 * (int64_t)most;
+    }
+    for (const auto *v : {&shorts[l], &longs[l]})
+      for (int s : *v) {
+        voff[s] = (int)lsz;
+        roff[s] = (int)rsz;
+        lsz += nrows(s);
+        rsz += nrows(s);
+      }
+    for (int s : wide[l]) {
+      voff[s] = (int)sb;
+      roff[s] = (int)rsz;
+      rsz += nrows(s);
+      sb += (int64_t)(2 * nrows(s) - width(s)) * s_ld(width(s));
+    }
+    if (sb > (1ll << 30) || lsz > (1ll << 30)) return "pattern too large for the batched solver";
+  }
+  P.lsize = (int)lsz;
+  P.rsize = (int)rsz;
+  P.sbsize = (int)sb;
+  H.ls0.assign((size_t)rsz, 0);
+  for (int s = 0; s < ns; ++s)
+    for (int r = 0; r < nrows(s); ++r) H.ls0[roff[s] + (size_t)r * (packed(s) ? 32 : 1)] = S.ls[S.lpi[s] + r];
   // packed records: one load brings a supernode's or a pair's numbers
   H.snrec.assign((size_t)8 * ns, 0);
   for (int s = 0; s < ns; ++s) {
     int *r = H.snrec.data() + 8 * (size_t)s;
     r[0] = S.super[s];
-    r[1] = S.super[s + 1] - S.super[s];
-    r[2] = (int)(S.lpi[s + 1] - S.lpi[s]);
-    r[3] = (int)S.lpx[s];
-    r[4] = (int)S.lpi[s];
+    r[1] = width(s);
+    r[2] = nrows(s) | (packed(s) ? 1 << 16 : 0);
+    r[3] = voff[s];
+    r[4] = roff[s];
     r[5] = H.pair_ptr[s];
     r[6] = H.pair_mid[s];
     r[7] = H.pair_ptr[s + 1];
   }
   const int npairs = (int)H.pair_d.size();
-  H.prec.assign((size_t)4 * npairs, 0);
+  H.prec.assign((size_t)8 * npairs, 0);
   std::vector<std::vector<int>> ctg(mineq);
   P.cmask_ok = 1;
   for (int s = 0; s < ns; ++s) {
     if (H.pair_ptr[s + 1] - H.pair_mid[s] > 64) P.cmask_ok = 0;
     for (int pq = H.pair_ptr[s]; pq < H.pair_ptr[s + 1]; ++pq) {
       const int d = H.pair_d[pq];
-      int *r = H.prec.data() + 4 * (size_t)pq;
-      r[0] = d;
-      r[1] = H.pair_lb[pq];
-      r[2] = H.pair_ub[pq];
-      r[3] = (int)S.lpi[d];
+      int *r = H.prec.data() + 8 * (size_t)pq;
+      const int lb = H.pair_lb[pq], wd = width(d), st = packed(d) ? 32 : 1, ld = wd > 1 ? s_ld(wd) : st;
+      r[0] = S.super[d];
+      r[1] = (packed(d) ? 0 : wd << 16) | nrows(d);
+      r[2] = H.pair_ub[pq] - lb + 1;
+      r[3] = roff[d] + lb * st;
+      r[4] = voff[d] + lb * ld;
+      r[5] = wd > 1 ? voff[d] + (nrows(d) + lb - wd) * ld : 0;
+      r[6] = d;
+      r[7] = lb;
       if (pq >= H.pair_mid[s]) {
         const int k = H.sn_con[d];
         ctg[k].push_back(s);
@@ -290,12 +344,79 @@ std::string build_pattern(const HostQP &Q, HostPattern &H, const int nrelax[3], 
       }
     }
   }
-  // supernodes the solves give a warp: wide or tall blocks (one flag byte each, packed in ints)
-  H.sn_big.assign((ns + 3) / 4 + 1, 0);
-  for (int s = 0; s < ns; ++s) {
-    const int w = S.super[s + 1] - S.super[s], nr = (int)(S.lpi[s + 1] - S.lpi[s]);
-    if (w > 4 || (int64_t)nr * w > 64) reinterpret_cast<unsigned char *>(H.sn_big.data())[s] = 1;
+  // what the solves read, level by level
+  const auto record = [&](int s, std::vector<int> &to) {
+    to.insert(to.end(), {S.super[s], nrows(s), voff[s], roff[s]});
+  };
+  // lanes that share an item: as many as keep the CTA's threads at work, with
+  // at least `least` terms for each
+  const auto lanes = [&](int items, int terms, int least) {
+    int lg = 0;
+    while (lg < 5 && (items << (lg + 1)) <= threads && terms >= least << (lg + 1)) ++lg;
+    return lg;
+  };
+  // Entries of a level's packed single columns by target variable, 32 targets
+  // side by side (those with the most entries first): from BATCH_GATHER_MIN
+  // columns on, where pushes would meet on the same targets.
+  H.gidx.assign((size_t)rsz, -1);
+  const auto gather = [&](const std::vector<int> &cols) {
+    std::map<int, std::vector<std::pair<int, int>>> by;  // variable -> (column, row-list position)
+    for (int s : cols)
+      for (int r = 1; r < nrows(s); ++r)
+        by[S.perm[S.ls[S.lpi[s] + r]]].push_back({S.super[s], roff[s] + 32 * r});
+    std::vector<int> vars;
+    for (auto &t : by) vars.push_back(t.first);
+    std::stable_sort(vars.begin(), vars.end(), [&](int x, int y) { return by[x].size() > by[y].size(); });
+    for (size_t g = 0; g < vars.size(); g += 32) {
+      const int first = (int)H.so_gs.size(), most = ((int)by[vars[g]].size() + 3) & ~3;
+      H.so_g.insert(H.so_g.end(), {first, most});
+      H.so_gs.resize((size_t)first + 32 * (size_t)most, by[vars[g]][0].first);  // a valid column for the zeros
+      for (int i = 0; i < 32; ++i) {
+        const bool in = g + i < vars.size();
+        H.so_gj.push_back(in ? vars[g + i] : -1);
+        if (!in) continue;
+        const auto &list = by[vars[g + i]];
+        for (size_t k = 0; k < list.size(); ++k) {
+          H.so_gs[first + 32 * k + i] = list[k].first;
+          H.gidx[list[k].second] = first + 32 * (int)k + i;
+        }
+      }
+    }
+  };
+  for (int l = 0; l < P.nlev; ++l) {
+    for (const auto *v : {&shorts[l], &longs[l]}) {
+      H.so_seg.push_back((int)H.so_sn.size());
+      for (int s : *v) {
+        H.so_sn.push_back(s);
+        record(s, H.so_rec);
+      }
+    }
+    const int e0 = (int)H.so_e.size() / 4, f1 = (int)H.so_f.size() / 4, b0 = (int)H.so_b.size() / 4;
+    for (int s : packs[l]) record(s, H.so_e);
+    int wmax = 0, mmax = 0;
+    for (int s : wide[l]) {
+      const int c0 = S.super[s], w = width(s), m = nrows(s) - w, ld = s_ld(w);
+      wmax = std::max(wmax, w);
+      mmax = std::max(mmax, m);
+      for (int i = 0; i < w; ++i) H.so_f.insert(H.so_f.end(), {voff[s] + i * ld, c0, i + 1, roff[s] + i});
+      for (int j = 0; j < w; ++j)
+        H.so_b.insert(H.so_b.end(), {voff[s] + w * ld + j, (int)((unsigned)c0 << 16 | (unsigned)w),
+                                     (int)((unsigned)j << 16 | (unsigned)m), roff[s] + w});
+    }
+    const int f2 = (int)H.so_f.size() / 4;
+    for (int s : wide[l])
+      for (int r = width(s); r < nrows(s); ++r)
+        H.so_f.insert(H.so_f.end(), {voff[s] + r * s_ld(width(s)), S.super[s], width(s), roff[s] + r});
+    const int n1 = f2 - f1, n2 = (int)H.so_f.size() / 4 - f2, en = (int)H.so_e.size() / 4 - e0;
+    H.lvl.insert(H.lvl.end(), {f1, n1 << 5 | lanes(n1, wmax, 4), f2, n2 << 5 | lanes(n2, wmax, 4), b0,
+                               n1 << 5 | lanes(n1, std::max(wmax, mmax), 2), e0, en});
+    const int g0 = (int)H.so_g.size() / 2;
+    if (en >= nqg::BATCH_GATHER_MIN) gather(packs[l]);
+    H.lvl.insert(H.lvl.end(), {g0, (int)H.so_g.size() / 2 - g0, 0, 0});
   }
+  H.so_seg.push_back((int)H.so_sn.size());
+  P.n1 = (int)H.so_sn.size();
+  P.gsize = (int)H.so_gs.size();
   H.con_ptr.assign(mineq + 1, 0);
   for (int k = 0; k < mineq; ++k) {
     H.con_ptr[k + 1] = H.con_ptr[k] + (int)ctg[k].size() / 2;
@@ -542,6 +663,7 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
   // ---- patterns
   const int nrelax[3] = {4, 16, 48};
   const double zrelax[3] = {0.8, 0.1, 0.05};
+  const int threads = b->set.threads > 0 ? b->set.threads : 128;
   std::unordered_map<uint64_t, std::vector<int>> by_key;
   for (int i = 0; i < np; ++i) {
     HostQP &Q = b->qp[i];
@@ -552,7 +674,7 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
     if (found < 0) {
       HostPattern H;
       H.rep = i;
-      std::string err = build_pattern(Q, H, nrelax, zrelax);
+      std::string err = build_pattern(Q, H, nrelax, zrelax, threads);
       if (!err.empty()) return fail(b, NQG_ERR_SYMBOLIC, err);
       found = (int)b->pats.size();
       b->pats.push_back(std::move(H));
@@ -563,7 +685,7 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
   // ---- integer pool
   std::vector<int> ipool;
   std::vector<BPat> hp;
-  int N_max = 0, nr_max = 1, w_max = 1, xs_max = 0, ss_max = 0, ns_max = 1, mi_max = 1, nlev_max = 1, nR_max = 1;
+  int N_max = 0, nr_max = 1, w_max = 1, xs_max = 0, ss_max = 0, sb_max = 0, g_max = 0, b_max = 1, ns_max = 1, mi_max = 1, nlev_max = 1, nR_max = 1;
   for (HostPattern &H : b->pats) {
     BPat &P = H.P;
     auto put = [&ipool](const std::vector<int> &v) {
@@ -579,8 +701,6 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
     P.o_lpx = put(H.lpx);
     P.o_ls0 = put(H.ls0);
     P.o_perm0 = put(H.perm0);
-    P.o_lvl_ptr = put(H.lvl_ptr);
-    P.o_lvl_sn = put(H.lvl_sn);
     P.o_lev = put(H.lev);
     P.o_pair_ptr = put(H.pair_ptr);
     P.o_pair_mid = put(H.pair_mid);
@@ -607,13 +727,23 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
     P.o_prec = put(H.prec);
     P.o_con_ptr = put(H.con_ptr);
     P.o_con_tgt = put(H.con_tgt);
-    P.o_sn_big = put(H.sn_big);
+    P.o_so_sn = put(H.so_sn);
+    P.o_so_seg = put(H.so_seg);
+    for (auto [o, v] : {std::make_pair(&P.o_so_rec, &H.so_rec), {&P.o_so_e, &H.so_e}, {&P.o_so_f, &H.so_f},
+                        {&P.o_so_b, &H.so_b}, {&P.o_lvl, &H.lvl}, {&P.o_so_g, &H.so_g}, {&P.o_so_gj, &H.so_gj}, {&P.o_so_gs, &H.so_gs},
+                        {&P.o_gidx, &H.gidx}}) {
+      while (ipool.size() % 4) ipool.push_back(0);
+      *o = put(*v);
+    }
     hp.push_back(P);
     N_max = std::max(N_max, P.N);
     nr_max = std::max(nr_max, P.max_nr);
     w_max = std::max(w_max, P.max_w);
-    xs_max = std::max(xs_max, P.xsize);
-    ss_max = std::max(ss_max, P.ssize);
+    xs_max = std::max(xs_max, P.lsize);
+    sb_max = std::max(sb_max, P.sbsize);
+    g_max = std::max(g_max, P.gsize);
+    for (size_t q = 0; q < H.snrec.size(); q += 8) b_max = std::max(b_max, H.snrec[q + 1] * (H.snrec[q + 2] & 0xffff));
+    ss_max = std::max(ss_max, P.rsize);
     ns_max = std::max(ns_max, P.ns);
     mi_max = std::max(mi_max, P.mineq);
     nlev_max = std::max(nlev_max, P.nlev);
@@ -716,17 +846,19 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
     return o;
   };
   sl.o_L = seg((int64_t)xs_max * ts);
-  sl.o_D = seg((int64_t)2 * N_max * ts);
+  sl.o_S = seg((int64_t)sb_max * ts);
+  sl.o_G = seg((int64_t)g_max * ts);
+  sl.o_D = seg((int64_t)3 * N_max * ts);  // D, D^-1
   sl.o_ls = seg((int64_t)ss_max * 4);
   sl.o_perm = seg((int64_t)N_max * 4);
   sl.o_iperm = seg((int64_t)N_max * 4);
   sl.o_lperm = seg((int64_t)N_max * 4);
-  sl.o_mark = seg(ns_max);
   sl.o_piv = seg(ns_max);
   sl.o_alist = seg((int64_t)mi_max * 4);
-  sl.o_vlist = seg((int64_t)ns_max * 4);
+  sl.o_vrec = seg((int64_t)ns_max * 16);
+  sl.o_arow = seg((int64_t)mi_max * 4);
   sl.o_mlist = seg((int64_t)ns_max * 4);
-  sl.o_Fv = seg((int64_t)nR_max * 8);
+  sl.o_Fv = seg((int64_t)nR_max * ts);
   sl.o_Rv = seg((int64_t)nR_max * 8);
   sl.o_cmask = seg((int64_t)ns_max * 8);
   sl.o_rhs = seg((int64_t)N_max * 8);
@@ -748,12 +880,13 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
   BQ_CUDA(cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, dev));
   int smem_optin = 0;
   BQ_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  b->threads = b->set.threads > 0 ? b->set.threads : 128;
+  b->threads = threads;
   if (b->threads % 32 || b->threads > 256) return fail(b, NQG_ERR_ARG, "threads must be a multiple of 32, at most 256");
   nqg::BArgs base_args{};
   base_args.N_max = N_max;
   base_args.w_max = w_max;
   base_args.nr_max = nr_max;
+  base_args.b_max = b_max;
   base_args.ns_max = ns_max;
   base_args.mi_max = mi_max;
   base_args.nlev_max = nlev_max;
@@ -789,7 +922,7 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
   std::vector<int64_t> need(np);
   for (int i = 0; i < np; ++i) {
     const BPat &P = b->pats[b->qp[i].pat].P;
-    need[i] = ((int64_t)P.xsize * (int64_t)ts + 15) / 16 * 16 + (int64_t)P.ssize * 4;
+    need[i] = ((int64_t)P.lsize * (int64_t)ts + 15) / 16 * 16 + (int64_t)P.sbsize * (int64_t)ts + (int64_t)P.rsize * 4;
   }
   std::vector<int64_t> budgets;
   if (b->set.stage) {
