@@ -316,262 +316,12 @@ __device__ __forceinline__ int sn_stride(const int4 &r0) { return r0.z >> 16 ? 3
   v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
 }
 
-constexpr int LD_BATCH = 8;  // loads in flight per lane
 
-// Warp-wide argmax of |value| with the smallest index winning ties (the
-// LAPACK idamax convention) over the lanes that have one (idx >= 0, rising
-// with the lane); every lane returns the winner.  The bits of a non-negative
-// floating-point number order like an integer: two integer reductions and a
-// vote instead of a tree of compares (an FP64 compare holds the FP64 pipe of
-// the SM quarter for 64 cycles).
-[[maybe_unused]] __device__ __forceinline__ void warp_argmax(float &v, int &idx) {
-  const unsigned FULL = 0xffffffffu;
-  const unsigned key = idx >= 0 ? __float_as_uint(v) + 1u : 0u;
-  const unsigned best = __reduce_max_sync(FULL, key);
-  const unsigned who = __ballot_sync(FULL, best && key == best);
-  const int src = who ? __ffs(who) - 1 : 0;
-  v = __shfl_sync(FULL, v, src);
-  idx = best ? __shfl_sync(FULL, idx, src) : -1;
-}
-[[maybe_unused]] __device__ __forceinline__ void warp_argmax(double &v, int &idx) {
-  const unsigned FULL = 0xffffffffu;
-  const bool has = idx >= 0;
-  const unsigned hi = has ? (unsigned)__double2hiint(v) + 1u : 0u;
-  const unsigned bh = __reduce_max_sync(FULL, hi);
-  const bool top = has && hi == bh;
-  const unsigned lo = top ? (unsigned)__double2loint(v) : 0u;
-  const unsigned bl = __reduce_max_sync(FULL, lo);
-  const unsigned who = __ballot_sync(FULL, top && lo == bl);
-  const int src = who ? __ffs(who) - 1 : 0;
-  v = __shfl_sync(FULL, v, src);
-  idx = bh ? __shfl_sync(FULL, idx, src) : -1;
-}
 
-// Lanes (rows of 32, two rows deep) to one candidate each: the larger, the
-// smaller index on ties.
-template <class T> __device__ __forceinline__ void take_larger(T &v, int &i, T v2, int i2) {
-  if (i2 >= 0 && (i < 0 || v2 > v)) {
-    v = v2;
-    i = i2;
-  }
-}
-
-// Bunch-Kaufman (alpha = (1+sqrt(17))/8, the LAPACK dsytf2('L') pivot rule
-// and the reference's reorder_after_sytrf form: explicit interchanges, L with
-// unit diagonal, D / E the diagonal and 2x2 sub-diagonals, perm[m] = original
-// local column at position m) on a lower-stored block of at most 64 columns.
-// Every warp of the group finds the pivot by itself from the shared block (no
-// broadcast to wait for), and the trailing columns are dealt to the warps, a
-// lane per row.  wi of nw: this warp's place in the group that calls together;
-// nw = 1 synchronizes the warp only.  Returns whether any interchange happened.
-// A 22-column FP64 block took about 100k cycles by one warp whose lanes walked
-// their rows' columns one after another (w^2 / 2 multiply-adds of 64 cycles).
+// bk_block on blocks in dynamic shared memory, by their offsets.
 template <class T>
-__device__ __noinline__ bool bk_block(Sh<T> a_, int lda, int w, Sh<T> D_, Sh<T> E_, Sh<int> perm_, int wi, int nw) {
-  T *a = a_, *D = D_, *E = E_;
-  int *perm = perm_, *status = &ctx<T>().status;
-  const unsigned FULL = 0xffffffffu;
-  const T alpha = (T)((1.0 + sqrt(17.0)) / 8.0);
-  const int lane = lane_id();
-  auto sync = [&]() {
-    if (nw > 1) __syncthreads();
-    else __syncwarp();
-  };
-  bool pivoted = false;
-  if (wi == 0)
-#pragma unroll 1
-    for (int m = lane; m < w; m += 32) perm[m] = m;
-  int k = 0;
-  while (k < w) {
-    const T akk = a[k + k * lda], absakk = tabs(akk);
-    // rows k+1+lane and k+33+lane of column k
-    const int i0 = k + 1 + lane, i1 = i0 + 32;
-    T c0 = i0 < w ? a[i0 + k * lda] : T(0), c1 = i1 < w ? a[i1 + k * lda] : T(0);
-    T cv = tabs(c0);
-    int ci = i0 < w ? i0 : -1;
-    warp_argmax(cv, ci);
-    if (w - k > 33) {
-      T v2 = tabs(c1);
-      int j2 = i1 < w ? i1 : -1;
-      warp_argmax(v2, j2);
-      take_larger(cv, ci, v2, j2);
-    }
-    const T colmax = ci >= 0 ? cv : T(0);
-    const int imax = ci;
-    int kp = k, kstep = 1, zero = 0;
-    if ((absakk >= colmax ? absakk : colmax) == T(0) || absakk != absakk) {
-      zero = 1;
-    } else if (!(absakk >= alpha * colmax)) {
-      T rv = T(-1);
-      int ri = -1;
-#pragma unroll 1
-      for (int b = k; b < w; b += 32) {
-        const int j = b + lane;
-        int jj = j < w && j != imax ? j : -1;
-        T v = jj < 0 ? T(0) : (j < imax ? tabs(a[imax + j * lda]) : tabs(a[j + imax * lda]));
-        warp_argmax(v, jj);
-        take_larger(rv, ri, v, jj);
-      }
-      const T rowmax = rv;
-      if (!(absakk >= alpha * colmax * (colmax / rowmax))) {
-        kp = imax;
-        if (!(tabs(a[imax + imax * lda]) >= alpha * rowmax)) kstep = 2;
-      }
-    }
-    const int kk = k + kstep - 1;
-    if (zero && wi == 0 && lane == 0) atomicOr(status, absakk == absakk ? ST_ZERO_PIVOT : ST_NONFINITE);
-    sync();
-    if (kp != kk) {  // symmetric interchange of kk and kp (kp > kk), by the first warp
-      pivoted = true;
-      if (wi == 0) {
-#pragma unroll 1
-        for (int i = kp + 1 + lane; i < w; i += 32) {
-          const T t = a[i + kk * lda];
-          a[i + kk * lda] = a[i + kp * lda];
-          a[i + kp * lda] = t;
-        }
-#pragma unroll 1
-        for (int j = kk + 1 + lane; j < kp; j += 32) {
-          const T t = a[j + kk * lda];
-          a[j + kk * lda] = a[kp + j * lda];
-          a[kp + j * lda] = t;
-        }
-        const int ncols_left = kstep == 2 ? k + 1 : k;
-#pragma unroll 1
-        for (int cc = lane; cc < ncols_left; cc += 32) {
-          const T t = a[kk + cc * lda];
-          a[kk + cc * lda] = a[kp + cc * lda];
-          a[kp + cc * lda] = t;
-        }
-        if (lane == 0) {
-          const T t = a[kk + kk * lda];
-          a[kk + kk * lda] = a[kp + kp * lda];
-          a[kp + kp * lda] = t;
-          const int pt = perm[kk];
-          perm[kk] = perm[kp];
-          perm[kp] = pt;
-        }
-      }
-      sync();
-    }
-    if (kstep == 1) {
-      const T d = kp != kk ? a[k + k * lda] : akk;
-      if (kp != kk) {
-        c0 = i0 < w ? a[i0 + k * lda] : T(0);
-        c1 = i1 < w ? a[i1 + k * lda] : T(0);
-      }
-      if (!zero) {
-        const T r1 = T(1) / d;
-        const T m0 = r1 * c0;  // multipliers, row i0 (and i1)
-        T m1 = T(0);
-        if (w - k > 33) m1 = r1 * c1;
-        // column j by warp (j - k - 1) mod nw: rows i >= j, four columns at a time
-#pragma unroll 1
-        for (int j = k + 1 + wi; j < w; j += 4 * nw) {
-          T v[4], mj[4];
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            const int jj = j + h * nw, q = jj - k - 1;
-            v[h] = i0 >= jj && i0 < w ? a[i0 + jj * lda] : T(0);
-            mj[h] = q < 32 ? __shfl_sync(FULL, m0, q & 31) : __shfl_sync(FULL, m1, q & 31);
-          }
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            const int jj = j + h * nw;
-            if (jj < w) v[h] -= mj[h] * c0;
-            if (i0 >= jj && i0 < w) a[i0 + jj * lda] = v[h];
-          }
-          if (w - k > 33)
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-              const int jj = j + h * nw;
-              if (i1 >= jj && i1 < w) a[i1 + jj * lda] -= mj[h] * c1;
-            }
-        }
-        sync();  // every warp has read column k
-        if (wi == 0) {
-          if (i0 < w) a[i0 + k * lda] = m0;
-          if (i1 < w) a[i1 + k * lda] = m1;
-        }
-      }
-      if (wi == 0 && lane == 0) {
-        D[k] = d;
-        E[k] = T(0);
-      }
-    } else {
-      // 2x2 pivot on rows/cols k, k+1
-      const T a11 = a[k + k * lda], a21 = a[k + 1 + k * lda], a22 = a[k + 1 + (k + 1) * lda];
-      const T i21 = T(1) / a21;
-      const T d11 = a22 * i21, d22 = a11 * i21;
-      const T d21 = (T(1) / (d11 * d22 - T(1))) * i21;
-      const int p0 = k + 2 + lane, p1 = p0 + 32;
-      T x0 = T(0), y0 = T(0), x1 = T(0), y1 = T(0);
-      if (p0 < w) {
-        x0 = a[p0 + k * lda];
-        y0 = a[p0 + (k + 1) * lda];
-      }
-      if (p1 < w) {
-        x1 = a[p1 + k * lda];
-        y1 = a[p1 + (k + 1) * lda];
-      }
-      const T u0 = d21 * (d11 * x0 - y0), v0 = d21 * (d22 * y0 - x0);
-      T u1 = T(0), v1 = T(0);
-      if (w - k > 34) {
-        u1 = d21 * (d11 * x1 - y1);
-        v1 = d21 * (d22 * y1 - x1);
-      }
-#pragma unroll 2
-      for (int j = k + 2 + wi; j < w; j += nw) {
-        const int q = j - k - 2;
-        const T uj = q < 32 ? __shfl_sync(FULL, u0, q & 31) : __shfl_sync(FULL, u1, q & 31);
-        const T vj = q < 32 ? __shfl_sync(FULL, v0, q & 31) : __shfl_sync(FULL, v1, q & 31);
-        if (p0 >= j && p0 < w) a[p0 + j * lda] -= x0 * uj + y0 * vj;
-        if (w - k > 34 && p1 >= j && p1 < w) a[p1 + j * lda] -= x1 * uj + y1 * vj;
-      }
-      sync();
-      if (wi == 0) {
-        if (p0 < w) {
-          a[p0 + k * lda] = u0;
-          a[p0 + (k + 1) * lda] = v0;
-        }
-        if (p1 < w) {
-          a[p1 + k * lda] = u1;
-          a[p1 + (k + 1) * lda] = v1;
-        }
-        if (lane == 0) {
-          D[k] = a11;
-          D[k + 1] = a22;
-          E[k] = a21;
-          E[k + 1] = T(0);
-          a[k + 1 + k * lda] = T(0);
-        }
-      }
-    }
-    sync();
-    k += kstep;
-  }
-  if (wi == 0)
-#pragma unroll 1
-    for (int m = lane; m < w; m += 32) a[m + m * lda] = T(1);
-  sync();
-  return pivoted;
-}
-
-// D^-1 of a block as diagonal and 2x2 off-diagonal: entry m of both (D, E: the
-// w diagonals and 2x2 sub-diagonals; 2x2 pivots by Cramer's rule, the
-// arithmetic of blocked_2by2_solver, Sym_BLAS.cpp:492-529).
-template <class T>
-__device__ __forceinline__ void d_inverse(const T *D, const T *E, int w, int m, T &inv, T &off) {
-  const bool first = m + 1 < w && E[m] != T(0), second = m > 0 && E[m - 1] != T(0);
-  off = T(0);
-  if (first || second) {
-    const int k = second ? m - 1 : m;
-    const T e = E[k], det = T(1) / (D[k] * D[k + 1] - e * e);
-    inv = det * D[second ? k : k + 1];
-    if (first) off = -e * det;
-  } else {
-    inv = T(1) / D[m];
-  }
+__device__ __noinline__ bool bk_block_at(Sh<T> a, int lda, int w, Sh<T> D, Sh<T> E, Sh<int> perm, int wi, int nw) {
+  return bk_block<T>((T *)a, lda, w, (T *)D, (T *)E, (int *)perm, &ctx<T>().status, wi, nw);
 }
 
 [[maybe_unused]] __device__ __forceinline__ bool finite_bits(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
@@ -924,7 +674,7 @@ template <class T> __device__ __noinline__ void factor_sn(Ctx<T> &, int s) {
     return;
   }
   bool pivoted = false;
-  if (w <= 64) pivoted = bk_block<T>(c.B, nr, w, c.Dsm, c.Esm, c.lp, warp_id(), num_warps());
+  if (w <= 64) pivoted = bk_block_at<T>(c.B, nr, w, c.Dsm, c.Esm, c.lp, warp_id(), num_warps());
   else bk_factor<T>(B, nr, w, c.Dsm, c.Esm, c.lp, &c.status, &pivoted);
   __syncthreads();
   lap(PH_SN_BK);
@@ -969,7 +719,7 @@ template <class T> __device__ __noinline__ void factor_sn_warp(Ctx<T> &, int s, 
     const int p = map8[4 * r + wi];
     return p < nr && rows[p] == r ? p : -1;
   });
-  const bool pivoted = bk_block<T>(sB, nr, w, sD, sE, slp, 0, 1);
+  const bool pivoted = bk_block_at<T>(sB, nr, w, sD, sE, slp, 0, 1);
   sn_finish<T, false>(c, s, c0, w, nr, r0, B, I, Dw, Ew, lpw, dv, pivoted, lane, 32, [](int) {});
 }
 

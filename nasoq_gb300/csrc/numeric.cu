@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 
@@ -30,7 +31,7 @@ namespace nqg {
 
 namespace {
 
-constexpr int BK_THREADS = 128;
+constexpr int BK_THREADS = 256;
 constexpr int UPD_THREADS = 256;
 constexpr int UPD_KC = 16;
 
@@ -121,10 +122,11 @@ __global__ void k_assemble(int n, const int *Kp, const int *Ki, const double *Kx
 }
 
 // ---------------------------------------------------------------------------
-// Schur update tiles.  C = (L_d D_d)[rows] * L_d[cols]^T, subtracted from the
+// Schur update tiles.  C = L_d[rows] * (L_d D_d)[cols]^T, subtracted from the
 // target with atomics.  D_d is block diagonal with 1x1 and 2x2 blocks:
 // (L D)(:,t) = d_t L(:,t) + e_t L(:,t+1) + e_{t-1} L(:,t-1) with e the 2x2
-// sub-diagonals (zero outside 2x2 blocks), which is blocked_2by2_mult.
+// sub-diagonals (zero outside 2x2 blocks), which is blocked_2by2_mult; it is
+// formed for the tile's columns, usually the fewer.
 template <class T>
 __global__ void __launch_bounds__(UPD_THREADS) k_update(const UpdTile *tiles, const int *tile_ids, int ntiles, int n,
                                                        const int *super, const int64_t *lpi, const int64_t *lpx,
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(const UpdTile *tiles, co
                                                        const int *rowmap, const int64_t *pmoff, const int *pair_lb) {
   __shared__ T As[UPD_KC][UPD_TM + 1];
   __shared__ T Bs[UPD_KC][UPD_TN + 1];
-  __shared__ T Raw[UPD_KC + 2][UPD_TM + 1];
+  __shared__ T Raw[UPD_KC + 2][UPD_TN + 1];
   __shared__ T dk[UPD_KC + 2], ek[UPD_KC + 2];
   __shared__ int prow[UPD_TM], pcol[UPD_TN];
   const int tid = threadIdx.x;
@@ -161,59 +163,68 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(const UpdTile *tiles, co
     }
     pcol[j] = pos;
   }
+  // rows tx + 16 a, columns ty + 16 b of the tile: what lies beyond the pair's
+  // rows, columns or depth costs nothing (an FP64 multiply-add holds its SM
+  // quarter's pipe for 64 cycles whatever the lanes hold: a pair of one column
+  // and seven rows took as long as a full 64 x 64 x 16 step, 46 us a level)
   const int tx = tid & 15, ty = tid >> 4;
+  const int na = tx < mrows ? (mrows - 1 - tx) / 16 + 1 : 0, nb = ty < ncols ? (ncols - 1 - ty) / 16 + 1 : 0;
   T acc[4][4];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int b = 0; b < 4; ++b) acc[a][b] = T(0);
+#pragma unroll 1
   for (int t0 = 0; t0 < wd; t0 += UPD_KC) {
+    const int kc = min(UPD_KC, wd - t0);
     __syncthreads();
-    // raw columns t0-1 .. t0+KC of the tile rows, plus D entries
-    for (int e = tid; e < (UPD_KC + 2) * UPD_TM; e += blockDim.x) {
-      int cc = e / UPD_TM, i = e % UPD_TM;
-      int t = t0 - 1 + cc;
-      T v = T(0);
-      if (t >= 0 && t < wd && i < mrows) v = Ld[(size_t)t * nrd + tl.ri + i];
-      Raw[cc][i] = v;
+    for (int e = tid; e < kc * UPD_TM; e += blockDim.x) {
+      const int cc = e / UPD_TM, i = e % UPD_TM;
+      if (i < mrows) As[cc][i] = Ld[(size_t)(t0 + cc) * nrd + tl.ri + i];
     }
-    for (int cc = tid; cc < UPD_KC + 2; cc += blockDim.x) {
-      int t = t0 - 1 + cc;
+    // columns t0-1 .. t0+kc of the tile columns' rows, plus D entries
+    for (int e = tid; e < (kc + 2) * UPD_TN; e += blockDim.x) {
+      const int cc = e / UPD_TN, j = e % UPD_TN, t = t0 - 1 + cc;
+      if (j < ncols) Raw[cc][j] = t >= 0 && t < wd ? Ld[(size_t)t * nrd + tl.cj + j] : T(0);
+    }
+    for (int cc = tid; cc < kc + 2; cc += blockDim.x) {
+      const int t = t0 - 1 + cc;
       dk[cc] = (t >= 0 && t < wd) ? Dg[c0 + t] : T(0);
       ek[cc] = (t >= 0 && t < wd) ? Dg[n + c0 + t] : T(0);
     }
-    for (int e = tid; e < UPD_KC * UPD_TN; e += blockDim.x) {
-      int cc = e / UPD_TN, j = e % UPD_TN;
-      int t = t0 + cc;
-      Bs[cc][j] = (t < wd && j < ncols) ? Ld[(size_t)t * nrd + tl.cj + j] : T(0);
-    }
     __syncthreads();
-    for (int e = tid; e < UPD_KC * UPD_TM; e += blockDim.x) {
-      int cc = e / UPD_TM, i = e % UPD_TM;
+    for (int e = tid; e < kc * UPD_TN; e += blockDim.x) {
+      const int cc = e / UPD_TN, j = e % UPD_TN;
+      if (j >= ncols) continue;
       // column t = t0+cc sits at Raw index cc+1
-      As[cc][i] = dk[cc + 1] * Raw[cc + 1][i] + ek[cc + 1] * Raw[cc + 2][i] + ek[cc] * Raw[cc][i];
+      T v = dk[cc + 1] * Raw[cc + 1][j];
+      if (ek[cc + 1] != T(0)) v += ek[cc + 1] * Raw[cc + 2][j];
+      if (ek[cc] != T(0)) v += ek[cc] * Raw[cc][j];
+      Bs[cc][j] = v;
     }
     __syncthreads();
-#pragma unroll
-    for (int cc = 0; cc < UPD_KC; ++cc) {
+    if (na == 0 || nb == 0) continue;
+#pragma unroll 4
+    for (int cc = 0; cc < kc; ++cc) {
       T av[4], bv[4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) av[a] = As[cc][ty * 4 + a];
+      for (int a = 0; a < 4; ++a) av[a] = a < na ? As[cc][tx + 16 * a] : T(0);
 #pragma unroll
-      for (int b = 0; b < 4; ++b) bv[b] = Bs[cc][tx * 4 + b];
+      for (int b = 0; b < 4; ++b) bv[b] = b < nb ? Bs[cc][ty + 16 * b] : T(0);
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] += av[a] * bv[b];
+        for (int b = 0; b < 4; ++b)
+          if (a < na && b < nb) acc[a][b] += av[a] * bv[b];
     }
   }
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
-    const int i = ty * 4 + a;
+    const int i = tx + 16 * a;
     if (i >= mrows || prow[i] < 0) continue;
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const int j = tx * 4 + b;
+      const int j = ty + 16 * b;
       if (j >= ncols || pcol[j] < 0) continue;
       if (tl.ri + i < tl.cj + j) continue;  // lower part only
       atomicAdd(&Lt[(size_t)pcol[j] * nrs + prow[i]], -acc[a][b]);
@@ -299,42 +310,63 @@ __global__ void __launch_bounds__(t5::THREADS) k_update_t5(const UpdTile *tiles,
 }
 
 // ---------------------------------------------------------------------------
-// Diagonal block BK + panel, one CTA per supernode.  SMALL: the block and a
-// row chunk of the panel are staged in shared memory.
+// Diagonal block BK, one CTA per supernode of at most BK_SMALL columns, and
+// the rows below where there are at most rows_here of them (more go to
+// k_panel_rows, one CTA per 32: a level's single supernode would keep one SM
+// busy with all of them).
 template <class T>
 __global__ void __launch_bounds__(BK_THREADS) k_bk_small(const int *targets, int n, const int *super,
                                                          const int64_t *lpi, const int64_t *lpx, T *L, T *Dg,
-                                                         int *locperm, uint8_t *pivoted, int *status) {
+                                                         int *locperm, uint8_t *pivoted, int rows_here, int *status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *a = reinterpret_cast<T *>(smem_raw);                 // BK_SMALL * BK_SMALL
-  T *rowbuf = a + BK_SMALL * BK_SMALL;                     // BK_SMALL * BK_THREADS
+  T *a = reinterpret_cast<T *>(smem_raw);  // BK_SMALL * BK_SMALL
+  T *X = a + BK_SMALL * BK_SMALL;          // rows below, by columns: BK_SMALL * BK_SMALL_ROWS
   __shared__ int perm[BK_SMALL];
-  const int s = targets[blockIdx.x];
+  __shared__ T Ds[BK_SMALL], Es[BK_SMALL], di[BK_SMALL], db[BK_SMALL];
+  const int s = targets[blockIdx.x], tid = threadIdx.x, nt = blockDim.x;
   const int c0 = super[s], w = super[s + 1] - c0;
-  const int nrow = (int)(lpi[s + 1] - lpi[s]);
+  const int nrow = (int)(lpi[s + 1] - lpi[s]), m = nrow - w;
   T *Ls = L + lpx[s];
-  for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
-    int c = e / w, r = e % w;
+  for (int e = tid; e < w * w; e += nt) {
+    const int c = e / w, r = e % w;
     a[r + c * w] = r >= c ? Ls[r + (size_t)c * nrow] : T(0);
   }
   __syncthreads();
-  bool piv = false;
-  bk_factor(a, w, w, Dg + c0, Dg + n + c0, perm, status, &piv);
-  for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
-    int c = e / w, r = e % w;
+  const bool piv = bk_block<T>(a, w, w, Ds, Es, perm, status, tid >> 5, nt >> 5);
+  __syncthreads();
+  for (int e = tid; e < w * w; e += nt) {
+    const int c = e / w, r = e % w;
     Ls[r + (size_t)c * nrow] = r >= c ? a[r + c * w] : T(0);
   }
-  for (int m = threadIdx.x; m < w; m += blockDim.x) locperm[c0 + m] = perm[m];
-  if (threadIdx.x == 0) pivoted[s] = piv ? 1 : 0;
-  __syncthreads();
-  panel_solve_rows(Ls, nrow, w, a, w, Dg + c0, Dg + n + c0, perm, rowbuf, BK_THREADS, piv);
-  // non-finite check on D
   bool bad = false;
-  for (int m = threadIdx.x; m < w; m += blockDim.x) {
-    T v = Dg[c0 + m];
-    if (!isfinite((double)v)) bad = true;
+  for (int k = tid; k < w; k += nt) {
+    Dg[c0 + k] = Ds[k];
+    Dg[n + c0 + k] = Es[k];
+    locperm[c0 + k] = perm[k];
+    d_inverse(Ds, Es, w, k, di[k], db[k]);
+    if (!isfinite((double)Ds[k])) bad = true;
   }
-  if (block_any(bad) && threadIdx.x == 0) flag_status(status, ST_NONFINITE);
+  if (tid == 0) pivoted[s] = piv ? 1 : 0;
+  if (m <= rows_here)
+    for (int r0 = 0; r0 < m; r0 += BK_SMALL_ROWS) {
+      const int mr = min(BK_SMALL_ROWS, m - r0);
+      T *Lr = Ls + w + r0;
+      __syncthreads();
+      for (int e = tid; e < mr * w; e += nt) {
+        const int r = e % mr, j = e / mr;
+        X[e] = Lr[r + (size_t)(piv ? perm[j] : j) * nrow];
+      }
+      __syncthreads();
+      rows_solve(X, mr, w, 1, mr, a, 1, w, tid, nt);
+      for (int e = tid; e < mr * w; e += nt) {
+        const int r = e % mr, j = e / mr;
+        T v = X[e] * di[j];
+        if (db[j] != T(0)) v += db[j] * X[e + mr];
+        if (j > 0 && db[j - 1] != T(0)) v += db[j - 1] * X[e - mr];
+        Lr[r + (size_t)j * nrow] = v;
+      }
+    }
+  if (block_any(bad) && tid == 0) flag_status(status, ST_NONFINITE);
 }
 
 // GENERIC: the diagonal block is factored in place in global memory; the
@@ -450,10 +482,10 @@ __global__ void __launch_bounds__(256) k_bk_global(const int *targets, int n, co
 // memory: each panel's triangle is solved one row per thread, and its
 // contribution is subtracted from the later columns.  Every entry receives
 // the terms x_t L(j, t) in increasing t, as in the per-row substitution.
-constexpr int PR_ROWS = 64, PR_KB = 32, PR_CG = 4;  // rows per item, panel width, columns per thread
+constexpr int PR_ROWS = 32, PR_KB = 32, PR_CG = 4;  // rows per item, panel width, columns per thread
 
 __host__ __device__ constexpr size_t panel_rows_smem(int wmax, int vsize) {
-  return ((size_t)PR_ROWS * (wmax + 1) + (size_t)wmax * (PR_KB + 1)) * vsize;
+  return ((size_t)PR_ROWS * (wmax | 1) + (size_t)wmax * (PR_KB + 1) + 2 * (size_t)wmax) * vsize;
 }
 
 template <class T>
@@ -469,10 +501,12 @@ __global__ void __launch_bounds__(256) k_panel_rows(const int2 *items, int n, co
   const bool piv = pivoted[s] != 0;
   const int r0 = w + rb * PR_ROWS, m = min(PR_ROWS, nrow - r0);
   if (m <= 0) return;
-  const int ldx = w + 1;
+  const int ldx = w | 1;                 // odd: a warp's rows fall into different banks
   T *X = reinterpret_cast<T *>(pr_raw);  // [PR_ROWS][ldx]
   T *Lp = X + (size_t)PR_ROWS * ldx;     // [w][PR_KB + 1]: columns jb .. jb+kb of L11, rows jb .. w
+  T *di = Lp + (size_t)w * (PR_KB + 1), *db = di + w;  // D^-1: diagonal, 2x2 off-diagonals
   const int tid = threadIdx.x;
+  for (int k = tid; k < w; k += blockDim.x) d_inverse(Dg + c0, Dg + n + c0, w, k, di[k], db[k]);
   for (int e = tid; e < m * w; e += blockDim.x) {
     const int r = e % m, j = e / m;
     X[r * ldx + j] = Ls[(r0 + r) + (size_t)(piv ? perm[j] : j) * nrow];
@@ -485,16 +519,8 @@ __global__ void __launch_bounds__(256) k_panel_rows(const int2 *items, int n, co
       Lp[i * (PR_KB + 1) + jj] = Ls[(jb + i) + (size_t)(jb + jj) * nrow];
     }
     __syncthreads();
-    // triangle of the panel: row r, columns jb .. jb+kb
-    if (tid < m) {
-      T *xr = X + tid * ldx;
-      for (int j = 0; j < kb; ++j) {
-        T x = xr[jb + j];
-        for (int t = 0; t < j; ++t) x -= xr[jb + t] * Lp[j * (PR_KB + 1) + t];
-        xr[jb + j] = x;
-      }
-    }
-    __syncthreads();
+    // triangle of the panel: rows over lanes, columns over warps
+    rows_solve(X + jb, m, kb, ldx, 1, Lp, PR_KB + 1, 1, tid, (int)blockDim.x);
     // later columns c >= jb+kb: x(r, c) -= sum_t x(r, jb+t) L(c, jb+t), t increasing
     const int c_lo = jb + kb, ncg = (w - c_lo + PR_CG - 1) / PR_CG;
     for (int e = tid; e < m * ncg; e += blockDim.x) {
@@ -515,29 +541,14 @@ __global__ void __launch_bounds__(256) k_panel_rows(const int2 *items, int n, co
     }
   }
   __syncthreads();
-  // D^-1 (1x1 and 2x2 blocks, Cramer's rule) and write back
-  const T *D = Dg + c0, *E = Dg + n + c0;
-  if (tid < m) {
-    T *xr = X + tid * ldx;
-    for (int j = 0; j < w; ++j) {
-      if (E[j] == T(0)) {
-        T inv = T(1) / D[j];
-        xr[j] *= inv;
-      } else {
-        T sd = E[j];
-        T det = D[j] * D[j + 1] - sd * sd;
-        T inv = T(1) / det;
-        T x1 = xr[j], x2 = xr[j + 1];
-        xr[j] = (x1 * D[j + 1] - x2 * sd) * inv;
-        xr[j + 1] = (x2 * D[j] - x1 * sd) * inv;
-        ++j;
-      }
-    }
-  }
-  __syncthreads();
+  // D^-1 and write back
   for (int e = tid; e < m * w; e += blockDim.x) {
     const int r = e % m, j = e / m;
-    Ls[(r0 + r) + (size_t)j * nrow] = X[r * ldx + j];
+    const T *xr = X + r * ldx;
+    T v = xr[j] * di[j];
+    if (db[j] != T(0)) v += db[j] * xr[j + 1];
+    if (j > 0 && db[j - 1] != T(0)) v += db[j - 1] * xr[j - 1];
+    Ls[(r0 + r) + (size_t)j * nrow] = v;
   }
 }
 
@@ -714,10 +725,11 @@ template <class T> static int factor_impl(Plan &P, const std::vector<int> *subse
     lv_glob_off.push_back(go);
     lv_glob_cnt.push_back((int)order.size() - go);
     lv_row_off.push_back((int)row_items.size() / 2);
-    for (int q = go; q < (int)order.size(); ++q) {
+    for (int q = so; q < (int)order.size(); ++q) {
       const int s = order[q];
       const int w = P.sym.super[s + 1] - P.sym.super[s];
       const int nb_rows = (int)(P.sym.lpi[s + 1] - P.sym.lpi[s]) - w;
+      if (q < go && nb_rows <= BK_SMALL_ROWS) continue;  // k_bk_small does them
       for (int rb = 0; rb * PR_ROWS < nb_rows; ++rb) {
         row_items.push_back(s);
         row_items.push_back(rb);
@@ -770,7 +782,7 @@ template <class T> static int factor_impl(Plan &P, const std::vector<int> *subse
   for (int q = 0; q < (int)lv_glob_off.size(); ++q)
     for (int k = lv_glob_off[q]; k < lv_glob_off[q] + lv_glob_cnt[q]; ++k)
       wmax_glob = std::max(wmax_glob, P.sym.super[order[k] + 1] - P.sym.super[order[k]]);
-  const size_t pr_smem = panel_rows_smem(std::max(wmax_glob, 1), (int)sizeof(T));
+  const size_t pr_smem = panel_rows_smem(std::max(wmax_glob, BK_SMALL), (int)sizeof(T));
   const bool rows_split = pr_smem <= 227 * 1024 && !P.panel_rows_serial;
   if (rows_split && !row_items.empty()) {
     if (row_items.size() > P.row_items_cap) {
@@ -832,7 +844,7 @@ template <class T> static int factor_impl(Plan &P, const std::vector<int> *subse
     P.prof_end(NQG_K_OTHER, e0, 0.0, 0.0);
     P.nlaunch++;
   }
-  const size_t smem_small = (size_t)(BK_SMALL * BK_SMALL + BK_SMALL * BK_THREADS) * sizeof(T);
+  const size_t smem_small = (size_t)(BK_SMALL * BK_SMALL + BK_SMALL * BK_SMALL_ROWS) * sizeof(T);
   static bool attr_set[2] = {false, false};
   int ai = sizeof(T) == 8 ? 0 : 1;
   if (!attr_set[ai]) {
@@ -892,8 +904,8 @@ template <class T> static int factor_impl(Plan &P, const std::vector<int> *subse
       cudaEvent_t e0 = P.prof_begin();
       if (lv_small_cnt[l] > 0) {
         k_bk_small<T><<<lv_small_cnt[l], BK_THREADS, smem_small, st>>>(P.d_targets + lv_small_off[l], n, P.d_super,
-                                                                        P.d_lpi, P.d_lpx, L, D, P.d_locperm,
-                                                                        P.d_pivoted, P.d_status);
+                                                                        P.d_lpi, P.d_lpx, L, D, P.d_locperm, P.d_pivoted,
+                                                                        rows_split ? BK_SMALL_ROWS : INT_MAX, P.d_status);
         P.nlaunch++;
       }
       if (lv_glob_cnt[l] > 0) {
@@ -910,12 +922,12 @@ template <class T> static int factor_impl(Plan &P, const std::vector<int> *subse
             P.d_targets + lv_glob_off[l], n, P.d_super, P.d_lpi, P.d_lpx, L, D, P.d_locperm, P.d_pivoted,
             P.d_perm_tmp, rows_split ? 0 : 1, P.d_status, staged);
         P.nlaunch++;
-        if (rows_split && lv_row_cnt[l] > 0) {
-          k_panel_rows<T><<<lv_row_cnt[l], 256, pr_smem, st>>>(
-              reinterpret_cast<const int2 *>(P.d_row_items) + lv_row_off[l], n, P.d_super, P.d_lpi, P.d_lpx, L, D,
-              P.d_locperm, P.d_pivoted);
-          P.nlaunch++;
-        }
+      }
+      if (rows_split && lv_row_cnt[l] > 0) {
+        k_panel_rows<T><<<lv_row_cnt[l], 256, pr_smem, st>>>(
+            reinterpret_cast<const int2 *>(P.d_row_items) + lv_row_off[l], n, P.d_super, P.d_lpi, P.d_lpx, L, D,
+            P.d_locperm, P.d_pivoted);
+        P.nlaunch++;
       }
       P.prof_end(NQG_K_BK, e0, fl, 0.0);
     }
