@@ -426,6 +426,9 @@ static int upload_plan(Plan &P) {
   P.solve_small_w = small_w;
   if ((rc = dev_alloc_copy(P, &P.d_targets_lv, lvflat.data(), lvflat.size()))) return rc;
   P.lv_targets_host = lvflat;
+  // small FP64 plans: one launch does a whole refined solve (the override asks
+  // for the level and block kernels)
+  if (!std::getenv("NASOQ_GB300_SOLVE_SMALL") && (rc = solve_small_setup(P, Rp))) return rc;
   P.vis_host.assign(ns, 1);
   NQG_CUDA(cudaMalloc(&P.d_pivoted, std::max(2 * ns, 2)));
   NQG_CUDA(cudaMemset(P.d_pivoted, 0, std::max(2 * ns, 2)));
@@ -501,7 +504,7 @@ static void free_plan(Plan &P) {
                   P.d_xo, P.d_bo, P.d_r, P.d_w, P.d_in, P.d_out, P.d_V, P.d_scal, P.d_wide_W, P.d_wide_ctl,
                   P.d_wide_pack, P.d_pers_map, P.d_pair_map, P.d_pair_moff, P.d_map_items, P.d_locinv, P.d_pair_roff, P.d_rr_dest, P.d_rr_moved, P.d_rr_items, P.d_rr_stage,
                   P.d_solve_flags, P.d_xw, P.d_tinv, P.d_blk_items, P.d_flagoff, P.d_xf, P.d_Z, P.d_tiles_tc,
-                  P.d_tile_list_tc, P.d_row_items};
+                  P.d_tile_list_tc, P.d_row_items, P.d_ss_rec, P.d_ss_seg, P.d_ss_rows, P.d_ss_colp, P.d_ss_dinv};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   P.prof_collect();

@@ -150,6 +150,11 @@ struct Plan {
   unsigned long long *d_xw = nullptr;  // FP32 block solves: (epoch << 32) | x bits per column
   float *d_tinv = nullptr;             // FP32 block solves: inverses of the diagonal 64 x 64 tiles
   bool tinv_valid = false;             // formed for the current factor
+  // one-launch solves of small FP64 plans (solve_small.cu)
+  bool ss_ok = false;
+  int ss_nlong = 0, ss_nlev = 0, ss_wmax = 0;  // rows of K that take a warp; levels of the merged blocks; widest
+  int *d_ss_rec = nullptr, *d_ss_seg = nullptr, *d_ss_rows = nullptr, *d_ss_colp = nullptr;
+  double *d_ss_dinv = nullptr;         // 2n: D^-1 of the current solve
   int solve_flags_cap = 0;
   unsigned solve_epoch = 0;
   int wide_nb = 64;
@@ -213,6 +218,9 @@ int dev_spmv_orig(Plan &P, const double *d_x, double *d_y);
 int dev_solve(Plan &P, const double *d_rhs, double *d_x);
 int dev_refine_only(Plan &P, const double *d_rhs, double *d_x);
 int dev_assemble_upload(Plan &P);
+// solve_small.cu
+int solve_small_setup(Plan &P, const std::vector<int> &Rp);
+int solve_small(Plan &P, const double *d_rhs, double *d_x, bool solve_first);
 
 #define NQG_CUDA(call)                                                                   \
   do {                                                                                   \

@@ -558,6 +558,7 @@ static int fgmres_refine(Plan &P, double *x, const double *b, int &itr_used, dou
 }
 
 int dev_solve(Plan &P, const double *d_rhs, double *d_x) {
+  if (P.ss_ok) return solve_small(P, d_rhs, d_x, true);
   const int n = P.n;
   int rc;
   // x_ord = rhs[perm]; b_ord = rhs[perm]
@@ -581,6 +582,7 @@ int dev_solve(Plan &P, const double *d_rhs, double *d_x) {
 // Refinement alone from x0 = rhs (reference iterative_ref_only,
 // src/QP/linear_solver_wrapper.cpp:1406-1430): no initial triangular solve.
 int dev_refine_only(Plan &P, const double *d_rhs, double *d_x) {
+  if (P.ss_ok) return solve_small(P, d_rhs, d_x, false);
   const int n = P.n;
   int rc;
   k_gather<<<grid_for(n), 256, 0, P.stream>>>(n, P.d_perm, d_rhs, P.d_bo);
