@@ -34,6 +34,8 @@ namespace {
 constexpr int BK_THREADS = 256;
 constexpr int UPD_THREADS = 256;
 constexpr int UPD_KC = 16;
+constexpr int UPD_NARROW = 16;  // columns of the tiles that update_narrow takes
+constexpr int UPD_KN = 32;      // their depth per step
 
 // ---------------------------------------------------------------------------
 // k_zero_targets / k_assemble: reset the values of the supernodes being
@@ -127,15 +129,78 @@ __global__ void k_assemble(int n, const int *Kp, const int *Ki, const double *Kx
 // (L D)(:,t) = d_t L(:,t) + e_t L(:,t+1) + e_{t-1} L(:,t-1) with e the 2x2
 // sub-diagonals (zero outside 2x2 blocks), which is blocked_2by2_mult; it is
 // formed for the tile's columns, usually the fewer.
+// Entry (t, j) of D L^T of a pair's columns: row r of the descendant, its columns
+// t - 1 .. t + 1 (2 x 2 pivots); every load is unconditional.
+template <class T>
+__device__ __forceinline__ T d_times(const T *Ld, int nrd, int wd, const T *D, const T *E, int t, int r) {
+  const int tm = max(t - 1, 0), tp = min(t + 1, wd - 1);
+  const T v = Ld[(size_t)t * nrd + r], vm = Ld[(size_t)tm * nrd + r], vp = Ld[(size_t)tp * nrd + r];
+  const T d = D[t], e = t + 1 < wd ? E[t] : T(0), em = t > 0 ? E[tm] : T(0);
+  T y = d * v;
+  if (e != T(0)) y += e * vp;
+  if (em != T(0)) y += em * vm;
+  return y;
+}
+
+// A tile of at most N columns (N a power of two up to UPD_NARROW): a thread
+// holds one row and a quarter of the depth, with the whole step's operands in
+// flight at once; the quarters meet in shared memory before the reductions at L2.
+template <int N, class T>
+__device__ __forceinline__ void update_narrow(unsigned char *raw, const UpdTile &tl, int nrd, int wd, const T *Ld,
+                                              const T *D, const T *E, int mrows, int ncols, int prow, const int *pcol,
+                                              T *Lt, int nrs) {
+  T *Bs = reinterpret_cast<T *>(raw), *red = Bs + UPD_KN * N;
+  const int tid = threadIdx.x, i = tid & (UPD_TM - 1), part = tid / UPD_TM;
+  constexpr int PARTS = UPD_THREADS / UPD_TM, PER = UPD_KN / PARTS, NB = (UPD_KN * N + UPD_THREADS - 1) / UPD_THREADS;
+  const T *La = Ld + tl.ri + min(i, mrows - 1);
+  T acc[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) acc[j] = T(0);
+#pragma unroll 1
+  for (int t0 = 0; t0 < wd; t0 += UPD_KN) {
+    const int kc = min(UPD_KN, wd - t0), per = (kc + PARTS - 1) / PARTS;
+    const int k0 = part * per, k1 = min(k0 + per, kc);
+    T l[PER], b[NB];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) l[q] = La[(size_t)(t0 + min(k0 + q, kc - 1)) * nrd];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const int e = tid + q * UPD_THREADS;
+      b[q] = d_times(Ld, nrd, wd, D, E, t0 + min(e / N, kc - 1), tl.cj + min(e % N, ncols - 1));
+    }
+    if (t0 > 0) __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NB; ++q)
+      if (tid + q * UPD_THREADS < UPD_KN * N) Bs[tid + q * UPD_THREADS] = b[q];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      if (k0 + q >= k1) break;  // the same for the whole warp
+#pragma unroll
+      for (int j = 0; j < N; ++j) acc[j] += l[q] * Bs[(k0 + q) * N + j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j) red[(part * N + j) * UPD_TM + i] = acc[j];
+  __syncthreads();
+#pragma unroll 1
+  for (int j = part; j < ncols; j += PARTS) {
+    T v = T(0);
+#pragma unroll
+    for (int q = 0; q < PARTS; ++q) v += red[(q * N + j) * UPD_TM + i];
+    // lower part only
+    if (i < mrows && prow >= 0 && pcol[j] >= 0 && tl.ri + i >= tl.cj + j) atomicAdd(&Lt[(size_t)pcol[j] * nrs + prow], -v);
+  }
+}
+
 template <class T>
 __global__ void __launch_bounds__(UPD_THREADS) k_update(const UpdTile *tiles, const int *tile_ids, int ntiles, int n,
                                                        const int *super, const int64_t *lpi, const int64_t *lpx,
                                                        const int *ls, T *L, const T *Dg, int *status,
                                                        const int *rowmap, const int64_t *pmoff, const int *pair_lb) {
-  __shared__ T As[UPD_KC][UPD_TM + 1];
-  __shared__ T Bs[UPD_KC][UPD_TN + 1];
-  __shared__ T Raw[UPD_KC + 2][UPD_TN + 1];
-  __shared__ T dk[UPD_KC + 2], ek[UPD_KC + 2];
+  constexpr int WIDE = UPD_KC * (UPD_TM + 1) + UPD_KC * (UPD_TN + 1);
+  constexpr int NARROW = UPD_KN * UPD_NARROW + UPD_NARROW * UPD_THREADS;
+  __shared__ __align__(16) unsigned char raw[(WIDE > NARROW ? WIDE : NARROW) * sizeof(T)];
   __shared__ int prow[UPD_TM], pcol[UPD_TN];
   const int tid = threadIdx.x;
   const UpdTile tl = tiles[tile_ids ? tile_ids[blockIdx.x] : blockIdx.x];
@@ -149,26 +214,41 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(const UpdTile *tiles, co
   const int cs0 = super[s], ws = super[s + 1] - cs0;
   const int nrs = (int)(lpi[s + 1] - lpi[s]);
   T *Lt = L + lpx[s];
-  // target positions of the tile's rows (from the level's pair map) and columns
+  // target positions of the tile's rows (from the pair map) and columns
   const int *pmap = rowmap + pmoff[tl.q] + (tl.ri - pair_lb[tl.q]);
-  for (int i = tid; i < UPD_TM; i += blockDim.x) prow[i] = i < mrows ? pmap[i] : -1;
-  for (int j = tid; j < UPD_TN; j += blockDim.x) {
+  const int my_row = pmap[min(tid & (UPD_TM - 1), mrows - 1)];
+  if (tid < UPD_TN) {
     int pos = -1;
-    if (j < ncols) {
-      pos = rows_d[tl.cj + j] - cs0;
+    if (tid < ncols) {
+      pos = rows_d[tl.cj + tid] - cs0;
       if (pos < 0 || pos >= ws) {
         flag_status(status, ST_BOUNDS);
         pos = -1;
       }
     }
-    pcol[j] = pos;
+    pcol[tid] = pos;
+    prow[tid] = tid < mrows ? my_row : -1;
   }
+  const T *D = Dg + c0, *E = Dg + n + c0;
+  if (ncols <= UPD_NARROW) {
+    auto run = [&](auto width) {
+      update_narrow<decltype(width)::value>(raw, tl, nrd, wd, Ld, D, E, mrows, ncols, my_row, pcol, Lt, nrs);
+    };
+    if (ncols == 1) run(std::integral_constant<int, 1>{});
+    else if (ncols == 2) run(std::integral_constant<int, 2>{});
+    else if (ncols <= 4) run(std::integral_constant<int, 4>{});
+    else if (ncols <= 8) run(std::integral_constant<int, 8>{});
+    else run(std::integral_constant<int, 16>{});
+    return;
+  }
+  T(*As)[UPD_TM + 1] = reinterpret_cast<T(*)[UPD_TM + 1]>(raw);
+  T(*Bs)[UPD_TN + 1] = reinterpret_cast<T(*)[UPD_TN + 1]>(raw + UPD_KC * (UPD_TM + 1) * sizeof(T));
   // rows tx + 16 a, columns ty + 16 b of the tile: what lies beyond the pair's
   // rows, columns or depth costs nothing (an FP64 multiply-add holds its SM
-  // quarter's pipe for 64 cycles whatever the lanes hold: a pair of one column
-  // and seven rows took as long as a full 64 x 64 x 16 step, 46 us a level)
+  // quarter's pipe for 64 cycles whatever the lanes hold)
   const int tx = tid & 15, ty = tid >> 4;
   const int na = tx < mrows ? (mrows - 1 - tx) / 16 + 1 : 0, nb = ty < ncols ? (ncols - 1 - ty) / 16 + 1 : 0;
+  const int i = tid & 63, k4 = tid >> 6;  // UPD_TM == UPD_TN == 64
   T acc[4][4];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
@@ -177,30 +257,18 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(const UpdTile *tiles, co
 #pragma unroll 1
   for (int t0 = 0; t0 < wd; t0 += UPD_KC) {
     const int kc = min(UPD_KC, wd - t0);
-    __syncthreads();
-    for (int e = tid; e < kc * UPD_TM; e += blockDim.x) {
-      const int cc = e / UPD_TM, i = e % UPD_TM;
-      if (i < mrows) As[cc][i] = Ld[(size_t)(t0 + cc) * nrd + tl.ri + i];
-    }
-    // columns t0-1 .. t0+kc of the tile columns' rows, plus D entries
-    for (int e = tid; e < (kc + 2) * UPD_TN; e += blockDim.x) {
-      const int cc = e / UPD_TN, j = e % UPD_TN, t = t0 - 1 + cc;
-      if (j < ncols) Raw[cc][j] = t >= 0 && t < wd ? Ld[(size_t)t * nrd + tl.cj + j] : T(0);
-    }
-    for (int cc = tid; cc < kc + 2; cc += blockDim.x) {
-      const int t = t0 - 1 + cc;
-      dk[cc] = (t >= 0 && t < wd) ? Dg[c0 + t] : T(0);
-      ek[cc] = (t >= 0 && t < wd) ? Dg[n + c0 + t] : T(0);
+    T va[UPD_KC / 4], vb[UPD_KC / 4];
+#pragma unroll
+    for (int q = 0; q < UPD_KC / 4; ++q) {
+      const int t = t0 + min(k4 + 4 * q, kc - 1);
+      va[q] = Ld[(size_t)t * nrd + tl.ri + min(i, mrows - 1)];
+      vb[q] = d_times(Ld, nrd, wd, D, E, t, tl.cj + min(i, ncols - 1));
     }
     __syncthreads();
-    for (int e = tid; e < kc * UPD_TN; e += blockDim.x) {
-      const int cc = e / UPD_TN, j = e % UPD_TN;
-      if (j >= ncols) continue;
-      // column t = t0+cc sits at Raw index cc+1
-      T v = dk[cc + 1] * Raw[cc + 1][j];
-      if (ek[cc + 1] != T(0)) v += ek[cc + 1] * Raw[cc + 2][j];
-      if (ek[cc] != T(0)) v += ek[cc] * Raw[cc][j];
-      Bs[cc][j] = v;
+#pragma unroll
+    for (int q = 0; q < UPD_KC / 4; ++q) {
+      As[k4 + 4 * q][i] = va[q];
+      Bs[k4 + 4 * q][i] = vb[q];
     }
     __syncthreads();
     if (na == 0 || nb == 0) continue;
@@ -220,14 +288,14 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(const UpdTile *tiles, co
   }
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
-    const int i = tx + 16 * a;
-    if (i >= mrows || prow[i] < 0) continue;
+    const int r = tx + 16 * a;
+    if (r >= mrows || prow[r] < 0) continue;
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int j = ty + 16 * b;
       if (j >= ncols || pcol[j] < 0) continue;
-      if (tl.ri + i < tl.cj + j) continue;  // lower part only
-      atomicAdd(&Lt[(size_t)pcol[j] * nrs + prow[i]], -acc[a][b]);
+      if (tl.ri + r < tl.cj + j) continue;  // lower part only
+      atomicAdd(&Lt[(size_t)pcol[j] * nrs + prow[r]], -acc[a][b]);
     }
   }
 }
@@ -706,8 +774,7 @@ template <class T> static int factor_impl(Plan &P, const std::vector<int> *subse
   std::vector<int> row_items, lv_row_off, lv_row_cnt;  // (supernode, row block) items of k_panel_rows
   std::vector<int> tile_ids, tile_ids_tc;
   std::vector<int64_t> lv_tile_off, lv_tile_cnt, lv_tc_off, lv_tc_cnt;
-  std::vector<int> map_items;  // (pair, first row) of the pair row maps, per level
-  std::vector<int64_t> lv_map_off, lv_map_cnt;
+  std::vector<int> map_items;  // (pair, first row) of the pair row maps
   const int nlev = (int)P.levels.size();
   for (int l = 0; l < nlev; ++l) {
     int so = (int)order.size();
@@ -748,7 +815,6 @@ template <class T> static int factor_impl(Plan &P, const std::vector<int> *subse
         for (int64_t t = P.tile_ptr_tc[s]; t < P.tile_ptr_tc[s + 1]; ++t) tile_ids_tc.push_back((int)t);
     lv_tc_off.push_back(tco);
     lv_tc_cnt.push_back((int64_t)tile_ids_tc.size() - tco);
-    const int64_t mo = (int64_t)map_items.size() / 2;
     for (int s : P.levels[l])
       if (mark[s])
         for (int q = P.pair_ptr[s]; q < P.pair_ptr[s + 1]; ++q) {
@@ -760,8 +826,6 @@ template <class T> static int factor_impl(Plan &P, const std::vector<int> *subse
             map_items.push_back(r0);
           }
         }
-    lv_map_off.push_back(mo);
-    lv_map_cnt.push_back((int64_t)map_items.size() / 2 - mo);
   }
   bool any = false;
   for (int s = 0; s < ns && !any; ++s) any = mark[s] != 0;
@@ -856,6 +920,16 @@ template <class T> static int factor_impl(Plan &P, const std::vector<int> *subse
     // sum_{k<w} (r-k)^2, the conventional factorization flop count of one supernode
     return w * r * r - r * w * (w - 1) + (w - 1) * w * (2 * w - 1) / 6.0;
   };
+  // the row lists change after the last level only (k_row_rename): one launch
+  // forms the maps of all pairs (per level: 6 us times 42 levels of a QP's system)
+  if (!map_items.empty()) {
+    cudaEvent_t e0 = P.prof_begin();
+    k_pair_rowmap<<<(unsigned)(map_items.size() / 2), 256, 0, st>>>(reinterpret_cast<const int2 *>(P.d_map_items),
+                                                                    P.d_pair_s, P.d_pair_d, P.d_pair_lb, P.d_pair_moff,
+                                                                    P.d_super, P.d_lpi, P.d_ls, P.d_pair_map, P.d_status);
+    P.prof_end(NQG_K_UPDATE, e0, 0.0, 0.0);
+    P.nlaunch++;
+  }
   for (int l = 0; l < nlev; ++l) {
     if (lv_tile_cnt[l] + lv_tc_cnt[l] > 0) {
       double fl = 0;
@@ -865,12 +939,6 @@ template <class T> static int factor_impl(Plan &P, const std::vector<int> *subse
             for (int q = P.pair_ptr[s]; q < P.pair_ptr[s + 1]; ++q)
               if (!P.pair_pers[q]) fl += P.pair_flops[q];
       cudaEvent_t e0 = P.prof_begin();
-      if (lv_map_cnt[l] > 0) {
-        k_pair_rowmap<<<(unsigned)lv_map_cnt[l], 256, 0, st>>>(
-            reinterpret_cast<const int2 *>(P.d_map_items) + lv_map_off[l], P.d_pair_s, P.d_pair_d, P.d_pair_lb,
-            P.d_pair_moff, P.d_super, P.d_lpi, P.d_ls, P.d_pair_map, P.d_status);
-        P.nlaunch++;
-      }
       if (lv_tile_cnt[l] > 0) {
         k_update<T><<<(unsigned)lv_tile_cnt[l], UPD_THREADS, 0, st>>>(P.d_tiles, P.d_tile_list + lv_tile_off[l],
                                                                       (int)lv_tile_cnt[l], n, P.d_super, P.d_lpi,
