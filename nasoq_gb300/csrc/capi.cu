@@ -504,7 +504,8 @@ static void free_plan(Plan &P) {
                   P.d_xo, P.d_bo, P.d_r, P.d_w, P.d_in, P.d_out, P.d_V, P.d_scal, P.d_wide_W, P.d_wide_ctl,
                   P.d_wide_pack, P.d_pers_map, P.d_pair_map, P.d_pair_moff, P.d_map_items, P.d_locinv, P.d_pair_roff, P.d_rr_dest, P.d_rr_moved, P.d_rr_items, P.d_rr_stage,
                   P.d_solve_flags, P.d_xw, P.d_tinv, P.d_blk_items, P.d_flagoff, P.d_xf, P.d_Z, P.d_tiles_tc,
-                  P.d_tile_list_tc, P.d_row_items, P.d_ss_rec, P.d_ss_seg, P.d_ss_rows, P.d_ss_colp, P.d_ss_dinv};
+                  P.d_tile_list_tc, P.d_row_items, P.d_ss_rec, P.d_ss_seg, P.d_ss_rows, P.d_ss_colp, P.d_ss_dinv, P.d_ss_inv0, P.d_ss_chunk,
+                  P.d_ss_inv};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   P.prof_collect();

@@ -154,6 +154,10 @@ struct Plan {
   bool ss_ok = false;
   int ss_nlong = 0, ss_nlev = 0, ss_wmax = 0;  // rows of K that take a warp; levels of the merged blocks; widest
   int *d_ss_rec = nullptr, *d_ss_seg = nullptr, *d_ss_rows = nullptr, *d_ss_colp = nullptr;
+  int ss_nchunk = 0;                   // 32-column chunks of the blocks that take a CTA
+  int *d_ss_inv0 = nullptr, *d_ss_chunk = nullptr;
+  double *d_ss_inv = nullptr;          // their inverted triangles, formed by each solve
+  size_t ss_smem = 0;
   double *d_ss_dinv = nullptr;         // 2n: D^-1 of the current solve
   int solve_flags_cap = 0;
   unsigned solve_epoch = 0;

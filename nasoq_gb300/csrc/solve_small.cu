@@ -12,12 +12,14 @@
 //
 // One cluster of eight CTAs does all of it; the vectors live in L2, a level of
 // the tree ends with a cluster barrier.  What bounds it is latency: per level
-// about 5000 cycles (block record, column table, factor entries, vector: four
-// dependent reads of 300-500 cycles, the additions to the rows below, the
-// barrier), and per 32 columns of a wide block about 9000 cycles of dependent
-// FP64 operations.  FP64 itself (one warp instruction per SM quarter and 64
-// cycles) is why one CTA was not enough: 1.79 ms for the solve of 4820 columns
-// in 10 levels on one SM, 0.99 ms on eight; with the level kernels 1.98 ms.
+// 5000 to 15000 cycles (dependent reads of 330 cycles at L2, 95 at L1; 380 cycles
+// for the barrier alone, 1000 to 2000 after stores and reductions), and per 32
+// columns of a wide block 2300 and, for what its columns take from the ones
+// before, 512 per chunk.  FP64 itself (one warp instruction per SM quarter and 64
+// cycles) is why one CTA was not enough.  The solve of 4820 columns in 10 levels:
+// 1.98 ms with the level kernels, 1.79 on one SM, 0.99 on eight with
+// substitutions, 0.83 with inverted 32 x 32 triangles; 916 columns in 83
+// levels: 6.1, 2.65, 1.29 and 1.03 ms.
 // Loads are issued eight at a time before they are used, and never under a
 // condition; entries below a block are added with reductions at L2.
 #include <cuda_runtime.h>
@@ -51,6 +53,10 @@ struct Args {
   int n, nlev, itr_max, mr, nlong, solve_first, wmax;
   double tol_abs, tol_rel;
   const int4 *rec;  // blocks in the order of the levels: c0, w, nr, first row
+  const int *inv0;  // first 32-column chunk of the blocks that take a CTA
+  const int4 *chunk;  // those chunks: the block's first column, chunk's first column in it, its columns
+  double *inv;      // their inverted unit triangles, by columns and by rows
+  int nchunk;
   const int *seg;   // thread / warp / CTA blocks of every level: 3 nlev + 1 starts
   const int *colp, *col2sup;
   const int *ls;
@@ -75,7 +81,7 @@ struct Block {
 
 struct Shared {
   double part[2][SS_WARPS], sum[2];
-  double chunk[SS_WARPS][32];
+  double left[SS_WARPS][32], tri[SS_WARPS][32];
   double c[SS_MR + 1], s[SS_MR + 1], g[SS_MR + 1], y[SS_MR + 1], h[SS_MR + 1][SS_MR];
   double rho, rho_tol, scale;
   int go, again, parity;
@@ -178,21 +184,6 @@ __device__ __forceinline__ double row_sum(const double *L, const int *c, int i, 
   }
   return y;
 }
-// Column entries [i0, i1) times x.
-__device__ __forceinline__ double col_sum(const double *L, int c, int i0, int i1, const double *x) {
-  double y = 0.0;
-#pragma unroll 1
-  for (int i = i0; i < i1; i += 8) {
-    double l[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) l[q] = entry(L, c, min(i + q, i1 - 1));
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (i + q < i1) y += l[q] * x[i + q];
-  }
-  return y;
-}
-
 // Sums of columns j .. j+7 (those below jend) against x over the rows below the
 // block, by one warp; lane 4q returns column j+q's.  Lanes take rows; the
 // reduction halves the columns with the lanes (9 additions for 8 columns: an
@@ -229,10 +220,24 @@ __device__ __forceinline__ double below_sums(const double *L, const int *c, cons
   return acc[0];
 }
 
+// Brings a block's first entries and rows to L1, by n threads: what follows
+// reads them in several rounds, of 330 cycles each at L2 and 95 here (a cluster
+// barrier empties L1, so nothing can be fetched ahead of the level).
+__device__ __forceinline__ void fetch(const double *L, const int *c, const Block &b, int t, int n) {
+  constexpr int LINES = 512;
+  const int c0 = c[0], c1 = c[b.w - 1];
+  if (c0 >= 0 && c1 >= 0) {
+    const int lines = min((c1 + b.nr - c0 + 15) / 16, LINES);
+    for (int q = t; q < lines; q += n) asm volatile("prefetch.global.L1 [%0];" ::"l"(L + c0 + min(16 * q, c1 + b.nr - 1 - c0)));
+  }
+  for (int q = 32 * t; q < b.nr; q += 32 * n) asm volatile("prefetch.global.L1 [%0];" ::"l"(b.rows + q));
+}
+
 // A block of up to 32 columns by one warp.
 __device__ __forceinline__ void fwd_warp(const double *L, const int *cp, const Block &b, double *xs) {
   const int lane = threadIdx.x & 31;
   const int *c = cp + b.c0;
+  fetch(L, c, b, lane, 32);
   double t = lane < b.w ? __ldcg(xs + b.c0 + lane) : 0.0;
   if (b.w > 1) {
     t = tri_fwd(L, c, 0, b.w, t);
@@ -249,6 +254,7 @@ __device__ __forceinline__ void fwd_warp(const double *L, const int *cp, const B
 __device__ __forceinline__ void bwd_warp(const double *L, const int *cp, const Block &b, double *xs) {
   const int lane = threadIdx.x & 31;
   const int *c = cp + b.c0;
+  fetch(L, c, b, lane, 32);
   double t = lane < b.w ? __ldcg(xs + b.c0 + lane) : 0.0;
   if (b.nr > b.w) {
 #pragma unroll 1
@@ -261,44 +267,114 @@ __device__ __forceinline__ void bwd_warp(const double *L, const int *cp, const B
   if (lane < b.w) xs[b.c0 + lane] = t;
 }
 
-// A block by the CTA, 32 columns of the triangle at a time.  While the first
-// warp solves a chunk of the triangle (a chain of 31 dependent steps), the
-// others add up what the chunks before it contribute to the next one; what the
-// chunk itself contributes is added by all warps afterwards.  xb: the block's
-// part of the vector, in shared memory.
-__device__ __noinline__ void fwd_cta(Shared &sh, const double *L, const int *cp, const Block b, double *xb, double *xs) {
+// The four entries 4 wi .. 4 wi + 3 of the sum of the warps' vectors v[][32], one
+// in each lane by lane % 4.
+__device__ __forceinline__ double own_four(const double (*v)[32], int wi) {
+  const int lane = threadIdx.x & 31;
+  double t = v[lane >> 2][4 * wi + (lane & 3)];
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) t += __shfl_xor_sync(FULL, t, o);
+  return t;
+}
+
+// Inverts the unit triangles of the 32-column chunks, one per CTA at a time: lane =
+// row, a warp does the columns wi, wi + 8, ... in the order of elimination.
+__device__ __noinline__ void invert_chunks(const Args &a, const int *cp) {
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+#pragma unroll 1
+  for (int q = cta_rank(); q < a.nchunk; q += SS_CTAS) {
+    const int4 u = a.chunk[q];
+    const int *c = cp + u.x + u.y;
+    const int kb = u.z, i = u.y + min(lane, kb - 1);
+    double l[32];
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+      const double v = entry(a.L, c[min(k, kb - 1)], i);
+      l[k] = k < lane && lane < kb ? v : 0.0;
+    }
+    double x[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) x[v] = lane == wi + 8 * v ? 1.0 : 0.0;
+#pragma unroll
+    for (int k = 0; k < 31; ++k)
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        if (k >= 8 * v) {
+          const double xk = __shfl_sync(FULL, x[v], k);
+          x[v] -= l[k] * xk;
+        }
+    double *out = a.inv + (size_t)q * 2048;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int col = wi + 8 * v;
+      out[col * 32 + lane] = x[v];
+      out[1024 + lane * 32 + col] = x[v];
+    }
+  }
+}
+
+// A block by the CTA, 32 columns (a chunk) at a time.  Of every chunk a warp has
+// four columns: it adds up what they contribute to the later chunks, and its
+// part of the product with the chunk's inverted triangle (a substitution is a
+// chain of 31 steps of about 110 cycles; by chunks 9000 cycles each, with the
+// inverse and the sums spread over the warps 2300).  xb: the block's part of the vector,
+// in shared memory; inv: the block's inverted triangles.
+__device__ __noinline__ void fwd_cta(Shared &sh, const double *L, const int *cp, const double *inv, const Block b,
+                                     double *xb, double *xs) {
   const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5;
   const int *c = cp + b.c0;
+  fetch(L, c, b, tid, SS_THREADS);
   for (int i = tid; i < b.w; i += SS_THREADS) xb[i] = __ldcg(xs + b.c0 + i);
-  double acc = 0.0;
+  double acc = 0.0, x = 0.0;
   __syncthreads();
 #pragma unroll 1
-  for (int jb = 0; jb < b.w; jb += 32) {
-    const int kb = min(32, b.w - jb);
-    if (jb > 0) {
-      constexpr int kw = 32 / SS_WARPS;
-      const int k0 = jb - 32 + kw * wi, i = jb + min(lane, kb - 1);
-      sh.chunk[wi][lane] = acc + row_sum(L, c, i, k0, k0 + kw, [&](int k) { return xb[k]; });
-      __syncthreads();
-    }
-    if (wi == 0) {
-      double t = lane < kb ? xb[jb + lane] : 0.0;
-      if (jb > 0)
+  for (int jb = 0; jb < b.w; jb += 32, inv += 2048) {
+    const int kb = min(32, b.w - jb), mine = 4 * wi + (lane & 3);
+    double m[4];
 #pragma unroll
-        for (int q = 0; q < SS_WARPS; ++q) t -= sh.chunk[q][lane];
-      t = tri_fwd(L, c, jb, kb, t);
-      if (lane < kb) {
-        xb[jb + lane] = t;
-        xs[b.c0 + jb + lane] = t;
+    for (int q = 0; q < 4; ++q) m[q] = inv[(4 * wi + q) * 32 + lane];
+    double t = mine < kb ? xb[jb + mine] : 0.0;
+    if (jb > 0) {
+      const int i = jb + min(lane, kb - 1);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc += entry(L, c[jb - 32 + 4 * wi + q], i) * __shfl_sync(FULL, x, q);
+      sh.left[wi][lane] = acc;
+      __syncthreads();
+      const double left = own_four(sh.left, wi);
+      if (mine < kb) t -= left;
+    }
+    double y = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) y += m[q] * __shfl_sync(FULL, t, q);
+    sh.tri[wi][lane] = y;
+    acc = 0.0;
+    if (jb + 32 < b.w) {  // the chunks before this one, for the next
+      const int i = min(jb + 32 + lane, b.w - 1);
+#pragma unroll 1
+      for (int k = 4 * wi; k < jb; k += 64) {
+        double l[8];
+        const int k2 = min(k + 32, jb - 32 + 4 * wi);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          l[q] = entry(L, c[k + q], i);
+          l[q + 4] = entry(L, c[k2 + q], i);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc += l[q] * xb[k + q];
+        if (k + 32 < jb)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) acc += l[q + 4] * xb[k2 + q];
       }
-      acc = 0.0;
-    } else if (jb > 0 && jb + 32 < b.w) {
-      const int i = min(jb + 32 + lane, b.w - 1), per = (jb + SS_WARPS - 2) / (SS_WARPS - 1);
-      const int k0 = min(per * (wi - 1), jb), k1 = min(k0 + per, jb);
-      acc = row_sum(L, c, i, k0, k1, [&](int k) { return xb[k]; });
     }
     __syncthreads();
+    x = own_four(sh.tri, wi);
+    if (lane < 4 && mine < kb) {
+      xb[jb + mine] = x;
+      xs[b.c0 + jb + mine] = x;
+    }
+    __syncwarp();
   }
+  __syncthreads();
   // rows below: chunks of 32 rows, and of the columns where there are fewer
   const int rc = (b.nr - b.w + 31) / 32;
   const int split = rc == 0 ? 1 : max(1, min(SS_WARPS / rc, b.w / 8)), per = (b.w + split - 1) / split;
@@ -311,61 +387,106 @@ __device__ __noinline__ void fwd_cta(Shared &sh, const double *L, const int *cp,
   }
   __syncthreads();  // xb is free again
 }
-__device__ __noinline__ void bwd_cta(Shared &sh, const double *L, const int *cp, const Block b, double *xb, double *xs) {
+__device__ __noinline__ void bwd_cta(Shared &sh, const double *L, const int *cp, const double *inv, const Block b,
+                                     double *xb, double *xs) {
   const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5;
   const int *c = cp + b.c0;
+  fetch(L, c, b, tid, SS_THREADS);
   for (int i = tid; i < b.w; i += SS_THREADS) xb[i] = __ldcg(xs + b.c0 + i);
   __syncthreads();
-  if (b.nr > b.w) {
+  // What the rows below contribute to chunk j's columns (a lane each): a warp
+  // has an eighth of the rows.
+  const int per = (b.nr - b.w + SS_WARPS - 1) / SS_WARPS;
+  const int ra = min(b.w + per * wi, b.nr), rb = min(ra + per, b.nr);
+  auto below = [&](int j) {
+    const int cl = c[min(j + lane, b.w - 1)];
+    double y = 0.0;
 #pragma unroll 1
-    for (int j = 8 * wi; j < b.w; j += 8 * SS_WARPS) {
-      const double y = below_sums(L, c, b, j, b.w, xs);
-      const int k = j + (lane >> 2);
-      if ((lane & 3) == 0 && k < b.w) xb[k] -= y;
-    }
-    __syncthreads();
-  }
-  double acc = 0.0;
-  const int last = (b.w - 1) / 32 * 32;
+    for (int r0 = ra; r0 < rb; r0 += 32) {
+      const int n = min(32, rb - r0);
+      const double xr = __ldcg(xs + b.rows[r0 + min(lane, n - 1)]);
 #pragma unroll 1
-  for (int jb = last; jb >= 0; jb -= 32) {
-    const int kb = min(32, b.w - jb);
-    const int cl = c[jb + min(lane, kb - 1)];
-    if (jb < last) {
-      constexpr int kw = 32 / SS_WARPS;
-      const int i0 = min(jb + 32 + kw * wi, b.w), i1 = min(i0 + kw, b.w);
-      sh.chunk[wi][lane] = acc + col_sum(L, cl, i0, i1, xb);
-      __syncthreads();
-    }
-    if (wi == 0) {
-      double t = lane < kb ? xb[jb + lane] : 0.0;
-      if (jb < last)
+      for (int k = 0; k < n; k += 8) {
+        double l[8];
 #pragma unroll
-        for (int q = 0; q < SS_WARPS; ++q) t -= sh.chunk[q][lane];
-      t = tri_bwd(L, c, jb, kb, t);
-      if (lane < kb) {
-        xb[jb + lane] = t;
-        xs[b.c0 + jb + lane] = t;
+        for (int q = 0; q < 8; ++q) l[q] = entry(L, cl, r0 + min(k + q, n - 1));
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (k + q < n) y += l[q] * __shfl_sync(FULL, xr, k + q);
       }
-      acc = 0.0;
-    } else if (jb > 0 && jb < last) {
-      const int rows = b.w - jb - 32, per = (rows + SS_WARPS - 2) / (SS_WARPS - 1);
-      const int i0 = jb + 32 + min(per * (wi - 1), rows), i1 = min(i0 + per, b.w);
-      acc = col_sum(L, c[jb - 32 + lane], i0, i1, xb);
+    }
+    return y;
+  };
+  const int last = (b.w - 1) / 32 * 32;
+  double acc = below(last), x = 0.0;
+  inv += (size_t)(last / 32) * 2048 + 1024;
+#pragma unroll 1
+  for (int jb = last; jb >= 0; jb -= 32, inv -= 2048) {
+    const int kb = min(32, b.w - jb), mine = 4 * wi + (lane & 3);
+    double m[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) m[q] = inv[(4 * wi + q) * 32 + lane];
+    double t = mine < kb ? xb[jb + mine] : 0.0;
+    if (jb < last) {
+      const int cl = c[jb + lane];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = jb + 32 + 4 * wi + q;
+        const double l = entry(L, cl, min(i, b.w - 1)), v = __shfl_sync(FULL, x, q);
+        if (i < b.w) acc += l * v;
+      }
+    }
+    if (jb < last || b.nr > b.w) {
+      sh.left[wi][lane] = acc;
+      __syncthreads();
+      const double left = own_four(sh.left, wi);
+      if (mine < kb) t -= left;
+    }
+    double y = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) y += m[q] * __shfl_sync(FULL, t, q);
+    sh.tri[wi][lane] = y;
+    acc = 0.0;
+    if (jb > 0) {  // the rows below and the chunks after this one, for the next
+      if (b.nr > b.w) acc = below(jb - 32);
+      const int cl = c[jb - 32 + lane];
+#pragma unroll 1
+      for (int i = jb + 32 + 4 * wi; i < b.w; i += 64) {
+        double l[8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          l[q] = entry(L, cl, min(i + q, b.w - 1));
+          l[q + 4] = entry(L, cl, min(i + 32 + q, b.w - 1));
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (i + q < b.w) acc += l[q] * xb[i + q];
+        if (i + 32 < b.w)
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (i + 32 + q < b.w) acc += l[q + 4] * xb[i + 32 + q];
+      }
     }
     __syncthreads();
+    x = own_four(sh.tri, wi);
+    if (lane < 4 && mine < kb) {
+      xb[jb + mine] = x;
+      xs[b.c0 + jb + mine] = x;
+    }
+    __syncwarp();
   }
+  __syncthreads();  // xb is free again
 }
 
 // xs <- (L D L^T)^-1 xs.  A level's blocks are independent of each other:
 // short single columns take a thread each, small blocks a warp, the others a CTA.
-__device__ __noinline__ void ldlt(const Args &a, Shared &sh, const int *cp, double *xb) {
+__device__ __noinline__ void ldlt(const Args &a, Shared &sh, const int *cp, const int *seg, double *xb) {
   const int tid = threadIdx.x, rank = cta_rank();
   const int thread = (SS_THREADS - 1 - tid) * SS_CTAS + rank, warp = (tid >> 5) * SS_CTAS + rank;
   double *xs = a.xs;
 #pragma unroll 1
   for (int l = 0; l < a.nlev; ++l) {
-    const int *sg = a.seg + 3 * l;
+    const int *sg = seg + 3 * l;
     const int s0 = sg[0], s1 = sg[1], s2 = sg[2], s3 = sg[3];
 #pragma unroll 1
     for (int q = s0 + thread; q < s1; q += SS_ALL) {
@@ -379,7 +500,8 @@ __device__ __noinline__ void ldlt(const Args &a, Shared &sh, const int *cp, doub
 #pragma unroll 1
     for (int q = s1 + warp; q < s2; q += SS_CTAS * SS_WARPS) fwd_warp(a.L, cp, block_at(a, q), xs);
 #pragma unroll 1
-    for (int q = s2 + rank; q < s3; q += SS_CTAS) fwd_cta(sh, a.L, cp, block_at(a, q), xb, xs);
+    for (int q = s2 + rank; q < s3; q += SS_CTAS)
+      fwd_cta(sh, a.L, cp, a.inv + (size_t)a.inv0[q] * 2048, block_at(a, q), xb, xs);
     cluster_sync();
   }
   for (int i = rank * SS_THREADS + tid; i < a.n; i += SS_ALL) {
@@ -397,7 +519,7 @@ __device__ __noinline__ void ldlt(const Args &a, Shared &sh, const int *cp, doub
   cluster_sync();
 #pragma unroll 1
   for (int l = a.nlev - 1; l >= 0; --l) {
-    const int *sg = a.seg + 3 * l;
+    const int *sg = seg + 3 * l;
     const int s0 = sg[0], s1 = sg[1], s2 = sg[2], s3 = sg[3];
 #pragma unroll 1
     for (int q = s0 + thread; q < s1; q += SS_ALL) {
@@ -412,7 +534,8 @@ __device__ __noinline__ void ldlt(const Args &a, Shared &sh, const int *cp, doub
 #pragma unroll 1
     for (int q = s1 + warp; q < s2; q += SS_CTAS * SS_WARPS) bwd_warp(a.L, cp, block_at(a, q), xs);
 #pragma unroll 1
-    for (int q = s2 + rank; q < s3; q += SS_CTAS) bwd_cta(sh, a.L, cp, block_at(a, q), xb, xs);
+    for (int q = s2 + rank; q < s3; q += SS_CTAS)
+      bwd_cta(sh, a.L, cp, a.inv + (size_t)a.inv0[q] * 2048, block_at(a, q), xb, xs);
     cluster_sync();
   }
 }
@@ -501,7 +624,8 @@ __global__ void __cluster_dims__(SS_CTAS, 1, 1) __launch_bounds__(SS_THREADS) k_
   extern __shared__ double xb[];
   __shared__ Shared sh;
   const int tid = threadIdx.x, n = a.n, me = cta_rank() * SS_THREADS + tid;
-  int *cp = reinterpret_cast<int *>(xb + a.wmax);
+  int *cp = reinterpret_cast<int *>(xb + a.wmax), *seg = cp + n;
+  for (int i = tid; i < 3 * a.nlev + 1; i += SS_THREADS) seg[i] = a.seg[i];
   double *xs = a.xs;
   for (int i = tid; i < n; i += SS_THREADS) {
     const int c = a.colp[i];
@@ -536,9 +660,11 @@ __global__ void __cluster_dims__(SS_CTAS, 1, 1) __launch_bounds__(SS_THREADS) k_
     sh.rho = 0.0;
     sh.parity = 0;
   }
+  __syncthreads();
+  invert_chunks(a, cp);
   cluster_sync();
   if (a.solve_first) {
-    ldlt(a, sh, cp, xb);
+    ldlt(a, sh, cp, seg, xb);
     for (int i = me; i < n; i += SS_ALL) a.x[i] = __ldcg(xs + a.iperm[i]);
     cluster_sync();
   }
@@ -548,7 +674,7 @@ __global__ void __cluster_dims__(SS_CTAS, 1, 1) __launch_bounds__(SS_THREADS) k_
   for (int itr = 0; itr < (a.mr > 0 ? a.itr_max : 0); ++itr) {
     spmv(a, a.x, [&](int i, double v) { xs[a.iperm[i]] = a.b[i] - v; });
     cluster_sync();
-    ldlt(a, sh, cp, xb);
+    ldlt(a, sh, cp, seg, xb);
     ++applied;
     double s0 = 0.0;
     for (int i = me; i < n; i += SS_ALL) s0 += __ldcg(xs + i) * __ldcg(xs + i);
@@ -574,7 +700,7 @@ __global__ void __cluster_dims__(SS_CTAS, 1, 1) __launch_bounds__(SS_THREADS) k_
       double *vk = a.V + (size_t)k * n, *v1 = vk + n;
       spmv(a, vk, [&](int i, double v) { xs[a.iperm[i]] = v; });
       cluster_sync();
-      ldlt(a, sh, cp, xb);
+      ldlt(a, sh, cp, seg, xb);
       ++applied;
       s0 = 0.0;
       double s1 = 0.0;
@@ -710,15 +836,15 @@ int solve_small_setup(Plan &P, const std::vector<int> &Rp) {
   }
   // The level kernels and the block kernels stay the better ones where one
   // wide block is most of the work (they spread it over the chip): dense
-  // systems take 0.96 ms here and 1.33 ms there at 512 columns, 1.77 and 1.63 at
-  // 768; a 20^3 Laplacian (widest block 615) 2.72 and 3.37; a 160^2 one (237)
-  // 1.85 and 2.86; a QP's 2064 columns in 115 levels 8.8 and 18.2 ms per
+  // systems take 0.85 ms here and 1.33 ms there at 512 columns, 1.65 and 1.63 at
+  // 768; a 20^3 Laplacian (widest block 615) 2.47 and 3.37; a 160^2 one (237)
+  // 2.31 and 2.86; a QP's 2064 columns in 115 levels 8.8 and 18.2 ms per
   // active-set iteration, 6522 columns in 368 levels 54.6 and 105.0.
   int launches = 0;
   for (size_t l = 0; l < P.levels.size(); ++l)
     launches += (P.level_off[l + 1] > P.level_off[l]) + (P.blk_fwd_off[l + 1] > P.blk_fwd_off[l]);
   if (P.ss_wmax > std::max(SS_WIDE, 4 * launches)) return NQG_OK;
-  std::vector<int> rec, seg(1, 0), rows;
+  std::vector<int> rec, seg(1, 0), rows, inv0, chunk;
   for (auto &list : lists) {
     // the largest first: they are dealt out in turn
     std::stable_sort(list.begin(), list.end(),
@@ -726,18 +852,30 @@ int solve_small_setup(Plan &P, const std::vector<int> &Rp) {
     for (int b : list) {
       const int r[4] = {S.super[first[b]], width(b), height(b), (int)S.lpi[first[b]]};
       rec.insert(rec.end(), r, r + 4);
+      inv0.push_back((int)chunk.size() / 4);
+      if ((&list - lists.data()) % 3 == 2)
+        for (int j = 0; j < r[1]; j += 32) chunk.insert(chunk.end(), {r[0], j, std::min(32, r[1] - j), 0});
     }
     seg.push_back((int)rec.size() / 4);
   }
   P.ss_nlev = nlev;
   for (int i = 0; i < P.n; ++i)
     if (Rp[i + 1] - Rp[i] > SS_ROW) rows.push_back(i);
+  P.ss_nchunk = (int)chunk.size() / 4;
+  P.ss_smem = (size_t)P.ss_wmax * sizeof(double) + ((size_t)P.n + seg.size()) * sizeof(int);
+  if (P.ss_smem > SS_SMEM_MAX) return NQG_OK;
   P.ss_nlong = (int)rows.size();
   rows.push_back(0);
+  chunk.resize(chunk.size() + 4);
   NQG_CUDA(cudaMalloc(&P.d_ss_rec, rec.size() * sizeof(int)));
   NQG_CUDA(cudaMalloc(&P.d_ss_seg, seg.size() * sizeof(int)));
   NQG_CUDA(cudaMalloc(&P.d_ss_colp, colp.size() * sizeof(int)));
   NQG_CUDA(cudaMemcpy(P.d_ss_colp, colp.data(), colp.size() * sizeof(int), cudaMemcpyHostToDevice));
+  NQG_CUDA(cudaMalloc(&P.d_ss_inv0, inv0.size() * sizeof(int)));
+  NQG_CUDA(cudaMemcpy(P.d_ss_inv0, inv0.data(), inv0.size() * sizeof(int), cudaMemcpyHostToDevice));
+  NQG_CUDA(cudaMalloc(&P.d_ss_chunk, chunk.size() * sizeof(int)));
+  NQG_CUDA(cudaMemcpy(P.d_ss_chunk, chunk.data(), chunk.size() * sizeof(int), cudaMemcpyHostToDevice));
+  NQG_CUDA(cudaMalloc(&P.d_ss_inv, std::max<size_t>(P.ss_nchunk, 1) * 2048 * sizeof(double)));
   NQG_CUDA(cudaMalloc(&P.d_ss_rows, rows.size() * sizeof(int)));
   NQG_CUDA(cudaMalloc(&P.d_ss_dinv, 2 * (size_t)P.n * sizeof(double)));
   NQG_CUDA(cudaMemcpy(P.d_ss_rec, rec.data(), rec.size() * sizeof(int), cudaMemcpyHostToDevice));
@@ -778,14 +916,17 @@ int solve_small(Plan &P, const double *d_rhs, double *d_x, bool solve_first) {
   a.x = P.d_xo;
   a.V = P.d_V;
   a.dinv = P.d_ss_dinv;
+  a.inv0 = P.d_ss_inv0;
+  a.chunk = reinterpret_cast<const int4 *>(P.d_ss_chunk);
+  a.nchunk = P.ss_nchunk;
+  a.inv = P.d_ss_inv;
   a.wmax = P.ss_wmax;
   a.xs = P.d_r;
   a.part = P.d_scal + 64;
   a.info = P.d_scal;
-  const size_t smem = (size_t)P.ss_wmax * sizeof(double) + (size_t)P.n * sizeof(int);
   NQG_CUDA(cudaFuncSetAttribute(k_solve_small, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_SMEM_MAX));
   cudaEvent_t e0 = P.prof_begin();
-  k_solve_small<<<SS_CTAS, SS_THREADS, smem, P.stream>>>(a);
+  k_solve_small<<<SS_CTAS, SS_THREADS, P.ss_smem, P.stream>>>(a);
   P.prof_end(NQG_K_SOLVE, e0, 0.0, 0.0);
   P.nlaunch++;
   NQG_CUDA(cudaGetLastError());
