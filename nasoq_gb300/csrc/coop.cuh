@@ -19,13 +19,10 @@ struct WideCtl {
   int halt;        // a speculative fast panel stopped early: later queued kernels skip
   int pad;
   int kb_log[16];  // columns done by each fast panel of a speculative batch
-  double cval[2][1024];
-  int cidx[2][1024];
-  double rval[2][1024];
-  int ridx[2][1024];
   // panel exchanges: per CTA and parity, (candidate << 8) | epoch; cleared
   // before every panel launch
   unsigned long long pslot[2][1024];
+  unsigned long long pair[2][2048];  // FP64 candidates: two words per CTA, cleared with pslot
   // fast panels: up to four candidate words per CTA and exchange
   unsigned long long mslot[2][4][1024];
   // polls before a cross-CTA wait gives up (0: SPIN_LIMIT); kept across the

@@ -66,81 +66,63 @@ __device__ __forceinline__ void pk_store_unit(unsigned char *hi, unsigned char *
   *reinterpret_cast<uint4 *>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-constexpr int WP_THREADS = 256;
+// Threads (rows) per CTA of the general panel kernel.  FP64: a multiply-add
+// holds its SM quarter's pipe for 64 cycles, so one warp per quarter and more
+// SMs; at eight warps a column of 32 updates took 4100 cycles, not 2050.
+template <class T> constexpr int WP_THREADS = sizeof(T) == 8 ? 128 : 256;
 constexpr int WP_NB = 64;  // widest panel; the row cache holds WP_NB + 2 columns
 
 template <class T> __device__ __forceinline__ T tabs_w(T v) { return v < T(0) ? -v : v; }
 
-// Block-local argmax (value, smallest index on ties) of the thread
-// candidates; result valid in thread 0.
-template <class T> __device__ void cta_argmax(T &v, int &i) {
-  __shared__ T sv[32];
+// Magnitudes as integers: the bits of a non-negative floating-point number
+// order like one (an FP64 compare holds the FP64 pipe for 64 cycles; a search
+// by compares took some 3000 of a column's 12000 cycles).
+template <class T> using Key = std::conditional_t<sizeof(T) == 8, unsigned long long, unsigned>;
+__device__ __forceinline__ unsigned mag(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned long long mag(double v) {
+  return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+template <class T> __device__ __forceinline__ bool mag_nan(Key<T> k) {
+  return k > (sizeof(T) == 8 ? (Key<T>)0x7ff0000000000000ull : (Key<T>)0x7f800000u);
+}
+__device__ __forceinline__ float mag_value(unsigned k) { return __uint_as_float(k); }
+__device__ __forceinline__ double mag_value(unsigned long long k) { return __longlong_as_double((long long)k); }
+
+// Largest key of the warp's candidates (i >= 0), the smallest index on ties.
+__device__ __forceinline__ void warp_best(unsigned &k, int &i) {
+  const unsigned FULL = 0xffffffffu;
+  const unsigned b = __reduce_max_sync(FULL, i >= 0 ? k + 1u : 0u);
+  const unsigned win = __reduce_min_sync(FULL, b && i >= 0 && k + 1u == b ? (unsigned)i : ~0u);
+  k = b ? b - 1u : 0u;
+  i = b ? (int)win : -1;
+}
+__device__ __forceinline__ void warp_best(unsigned long long &k, int &i) {
+  const unsigned FULL = 0xffffffffu;
+  const unsigned hi = i >= 0 ? (unsigned)(k >> 32) + 1u : 0u;
+  const unsigned bh = __reduce_max_sync(FULL, hi);
+  const bool top = bh && hi == bh;
+  const unsigned bl = __reduce_max_sync(FULL, top ? (unsigned)k : 0u);
+  const unsigned win = __reduce_min_sync(FULL, top && (unsigned)k == bl ? (unsigned)i : ~0u);
+  k = bh ? (unsigned long long)(bh - 1u) << 32 | bl : 0ull;
+  i = bh ? (int)win : -1;
+}
+
+// The same over the CTA's warps; valid in the first warp.
+template <class K> __device__ void cta_best(K &k, int &i) {
+  __shared__ K sk[32];
   __shared__ int si[32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    T ov = __shfl_down_sync(0xffffffffu, v, o);
-    int oi = __shfl_down_sync(0xffffffffu, i, o);
-    if (oi >= 0 && (i < 0 || ov > v || (ov == v && oi < i))) {
-      v = ov;
-      i = oi;
-    }
-  }
+  warp_best(k, i);
   if (lane == 0) {
-    sv[wid] = v;
+    sk[wid] = k;
     si[wid] = i;
   }
   __syncthreads();
   if (wid == 0) {
-    v = lane < nw ? sv[lane] : T(-1);
+    k = lane < nw ? sk[lane] : K(0);
     i = lane < nw ? si[lane] : -1;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      T ov = __shfl_down_sync(0xffffffffu, v, o);
-      int oi = __shfl_down_sync(0xffffffffu, i, o);
-      if (oi >= 0 && (i < 0 || ov > v || (ov == v && oi < i))) {
-        v = ov;
-        i = oi;
-      }
-    }
+    warp_best(k, i);
   }
-  __syncthreads();
-}
-
-// Reduce the G partial (value, index) pairs of one phase; every CTA does this
-// redundantly so that all take the same pivoting decision.
-template <class T> __device__ void reduce_partials(const double *pv, const int *pi, int G, T &v, int &idx) {
-  __shared__ double rv;
-  __shared__ int ri;
-  if (threadIdx.x < 32) {
-    double bv = -1.0;
-    int bi = -1;
-    for (int g = threadIdx.x; g < G; g += 32) {
-      double x = __ldcg(pv + g);
-      int xi = __ldcg(pi + g);
-      if (xi >= 0 && (bi < 0 || x > bv || (x == bv && xi < bi))) {
-        bv = x;
-        bi = xi;
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      double ov = __shfl_down_sync(0xffffffffu, bv, o);
-      int oi = __shfl_down_sync(0xffffffffu, bi, o);
-      if (oi >= 0 && (bi < 0 || ov > bv || (ov == bv && oi < bi))) {
-        bv = ov;
-        bi = oi;
-      }
-    }
-    if (threadIdx.x == 0) {
-      rv = bv;
-      ri = bi;
-    }
-  }
-  __syncthreads();
-  v = (T)rv;
-  idx = ri;
-  __syncthreads();
 }
 
 // Panel exchange: every CTA publishes one 64-bit word per synchronisation,
@@ -152,17 +134,27 @@ template <class T> __device__ void reduce_partials(const double *pv, const int *
 // __threadfence (later reads see the other CTAs' writes); data written by
 // other CTAs is read with ld.cg.  Two parities let a fast CTA publish the
 // next exchange while a slow one still reads this one.  The wait is bounded.
-__device__ bool grid_exchange(WideCtl *ctl, unsigned &epoch, unsigned long long cand, int *status,
-                              unsigned long long &best) {
+// PAIR (FP64): a candidate is a 63-bit magnitude and a row, in two words that
+// each carry the epoch: (magnitude >> 8) << 8 | epoch and the low 8 bits of it,
+// 48 bits of row + 1 (0: none), epoch.  `best` and `row` are valid in every thread.
+template <bool PAIR>
+__device__ bool grid_exchange(WideCtl *ctl, unsigned &epoch, unsigned long long cand, int cand_row, int *status,
+                              unsigned long long &best, int &row) {
   __shared__ unsigned long long s_best;
-  __shared__ int s_ok;
+  __shared__ int s_ok, s_row;
   ++epoch;
   const unsigned e = epoch & 0xFFu;  // at most 255 exchanges per panel launch: never 0
   const int par = epoch & 1;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    *(volatile unsigned long long *)&ctl->pslot[par][blockIdx.x] = (cand << 8) | e;
+    if constexpr (PAIR) {
+      volatile unsigned long long *slot = &ctl->pair[par][2 * blockIdx.x];
+      slot[0] = (cand & ~0xFFull) | e;
+      slot[1] = cand << 56 | (unsigned long long)(cand_row + 1) << 8 | e;
+    } else {
+      *(volatile unsigned long long *)&ctl->pslot[par][blockIdx.x] = (cand << 8) | e;
+    }
   }
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
@@ -170,13 +162,30 @@ __device__ bool grid_exchange(WideCtl *ctl, unsigned &epoch, unsigned long long 
     const long long lim_ = wait_limit(ctl);
     int ok = 1;
     unsigned long long m = 0;
+    int mi = -1;
     while (true) {
       bool all = true;
       m = 0;
+      mi = -1;
       for (int g = lane; g < (int)gridDim.x; g += 32) {
-        const unsigned long long v = *(volatile unsigned long long *)&ctl->pslot[par][g];
-        if ((unsigned)(v & 0xFFu) != e) all = false;
-        else m = max(m, v >> 8);
+        if constexpr (PAIR) {
+          const volatile unsigned long long *slot = &ctl->pair[par][2 * g];
+          const unsigned long long u = slot[0], v = slot[1];
+          if ((unsigned)(u & 0xFFu) != e || (unsigned)(v & 0xFFu) != e) {
+            all = false;
+          } else {
+            const unsigned long long k = (u & ~0xFFull) | v >> 56;
+            const int r = (int)(v >> 8 & 0xFFFFFFFFFFull) - 1;
+            if (r >= 0 && (mi < 0 || k > m || (k == m && r < mi))) {
+              m = k;
+              mi = r;
+            }
+          }
+        } else {
+          const unsigned long long v = *(volatile unsigned long long *)&ctl->pslot[par][g];
+          if ((unsigned)(v & 0xFFu) != e) all = false;
+          else m = max(m, v >> 8);
+        }
       }
       if (__all_sync(0xffffffffu, all)) break;
       int ab = lane == 0 ? *(volatile int *)&ctl->abort : 0;
@@ -194,49 +203,44 @@ __device__ bool grid_exchange(WideCtl *ctl, unsigned &epoch, unsigned long long 
         break;
       }
     }
+    if constexpr (PAIR) {
+      warp_best(m, mi);
+    } else {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+      for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    }
     __threadfence();
     if (lane == 0) {
       s_best = m;
+      s_row = mi;
       s_ok = ok;
     }
   }
   __syncthreads();
   best = s_best;
+  row = s_row;
   return s_ok != 0;
 }
 
 // Column-step argmax over the whole grid (valid on return in every thread,
-// the same in every CTA).  FP32: the candidate rides in the exchange word as
-// (|value| bits << 24) | (0xFFFFFF - row), 0 for none, so the maximum keeps
-// the largest value and, among equal values, the smallest row (rows < 2^24).
-// FP64: per-CTA partials beside the exchange, reduced redundantly by all.
+// the same in every CTA); colmax 0 and imax -1 without a candidate.  FP32: the
+// candidate rides in the exchange word as (|value| bits << 24) | (0xFFFFFF -
+// row), 0 for none, so the maximum keeps the largest value and, among equal
+// values, the smallest row (rows < 2^24).
 template <class T>
-__device__ bool grid_argmax(T cv, int ci, WideCtl *ctl, int phase, unsigned &epoch, int *status, T &v, int &idx) {
-  cta_argmax(cv, ci);
+__device__ bool grid_argmax(Key<T> ck, int ci, WideCtl *ctl, unsigned &epoch, int *status, T &v, int &idx) {
+  cta_best(ck, ci);
   unsigned long long best = 0;
   if constexpr (sizeof(T) == 4) {
     unsigned long long cand = 0;
-    if (ci >= 0) cand = ((unsigned long long)__float_as_uint((float)cv) << 24) | (0xFFFFFFull - (unsigned)ci);
-    if (!grid_exchange(ctl, epoch, cand, status, best)) return false;
-    if (best == 0ull) {
-      v = T(0);
-      idx = -1;
-    } else {
-      v = (T)__uint_as_float((unsigned)(best >> 24));
-      idx = 0xFFFFFF - (int)(best & 0xFFFFFFull);
-    }
+    if (ci >= 0) cand = ((unsigned long long)ck << 24) | (0xFFFFFFull - (unsigned)ci);
+    int none;
+    if (!grid_exchange<false>(ctl, epoch, cand, -1, status, best, none)) return false;
+    idx = best == 0ull ? -1 : 0xFFFFFF - (int)(best & 0xFFFFFFull);
+    v = best == 0ull ? T(0) : mag_value((unsigned)(best >> 24));
   } else {
-    const int par = (epoch + 1) & 1;  // parity of the coming exchange
-    double *pv = phase ? ctl->rval[par] : ctl->cval[par];
-    int *pi = phase ? ctl->ridx[par] : ctl->cidx[par];
-    if (threadIdx.x == 0) {
-      pv[blockIdx.x] = (double)cv;
-      pi[blockIdx.x] = ci;
-    }
-    if (!grid_exchange(ctl, epoch, 0ull, status, best)) return false;
-    reduce_partials(pv, pi, gridDim.x, v, idx);
+    if (!grid_exchange<true>(ctl, epoch, ck, ci, status, best, idx)) return false;
+    v = idx < 0 ? T(0) : mag_value(best);
   }
   return true;
 }
@@ -889,10 +893,11 @@ __global__ void __launch_bounds__(FB_THREADS) k_wide_panel_blk(float *S, int nro
 // the row W(c+1, 0..j) of the next update; a pivot search or an interchange
 // (rare once the pivot order has settled) reloads what it changed.
 template <class T>
-__global__ void __launch_bounds__(WP_THREADS) k_wide_panel(T *S, int nrow, int w, int k0, int nb, T *Wb, int ldw,
+__global__ void __launch_bounds__(WP_THREADS<T>) k_wide_panel(T *S, int nrow, int w, int k0, int nb, T *Wb, int ldw,
                                                            T *Dd, T *De, int *perm, WideCtl *ctl, int *status) {
+  constexpr int WP = WP_THREADS<T>;
   extern __shared__ __align__(16) unsigned char wp_raw[];
-  T *lc = reinterpret_cast<T *>(wp_raw);  // [WP_NB + 2][WP_THREADS]
+  T *lc = reinterpret_cast<T *>(wp_raw);  // [WP_NB + 2][WP]
   __shared__ T wbuf[2][WP_NB + 2];        // W(c, 0..j-1) of the current column, and of the next
   __shared__ T wrB[WP_NB + 2];            // W(imax, 0..j-1) of a pivot-row update
   const T alpha = (T)((1.0 + sqrt(17.0)) / 8.0);
@@ -908,13 +913,14 @@ __global__ void __launch_bounds__(WP_THREADS) k_wide_panel(T *S, int nrow, int w
     const int c = k0 + j;
     const T *wrow = wbuf[cur];
     // ---- A: updated column c into W(:, j), rows [c, nrow)
-    T cv = T(-1), w_own = T(0);
+    Key<T> cv = 0;
+    T w_own = T(0);
     int ci = -1;
     for (int r = first_row(c); r < nrow; r += TT) {
       T acc;
       if (r == gt) {
         acc = s_own;
-        for (int t = 0; t < j; ++t) acc -= lc[t * WP_THREADS + tid] * wrow[t];
+        for (int t = 0; t < j; ++t) acc -= lc[t * WP + tid] * wrow[t];
         w_own = acc;
       } else {
         acc = __ldcg(S + r + (size_t)c * nrow);
@@ -922,8 +928,8 @@ __global__ void __launch_bounds__(WP_THREADS) k_wide_panel(T *S, int nrow, int w
       }
       Wb[(size_t)j * ldw + r] = acc;
       if (r > c && r < w) {
-        const T a = tabs_w(acc);
-        if (a == a && (ci < 0 || a > cv)) {
+        const Key<T> a = mag(acc);
+        if (!mag_nan<T>(a) && (ci < 0 || a > cv)) {
           cv = a;
           ci = r;
         }
@@ -931,38 +937,39 @@ __global__ void __launch_bounds__(WP_THREADS) k_wide_panel(T *S, int nrow, int w
     }
     T colmax;
     int imax;
-    if (!grid_argmax(cv, ci, ctl, 0, epoch, status, colmax, imax)) return;
-    if (imax < 0) colmax = T(0);
+    if (!grid_argmax<T>(cv, ci, ctl, epoch, status, colmax, imax)) return;
     // one round of loads: pivot, and the next column's inputs on the fast path
     const T wcc = __ldcg(Wb + (size_t)j * ldw + c);
     T *wnext = wbuf[cur ^ 1];
     if (tid <= j && c + 1 < nrow) wnext[tid] = __ldcg(Wb + (size_t)tid * ldw + c + 1);
     const T s_next = (gt >= c + 1 && gt < nrow && c + 1 < w) ? __ldcg(S + gt + (size_t)(c + 1) * nrow) : T(0);
-    const T absakk = tabs_w(wcc);
+    const Key<T> akk = mag(wcc);
+    const T absakk = mag_value(akk);
+    const bool akk_nan = mag_nan<T>(akk);
     int kp = c, kstep = 1;
     bool zero = false, slow = false;
     T w_own1 = T(0);
-    if ((absakk >= colmax ? absakk : colmax) == T(0) || absakk != absakk) {
+    if (akk_nan || (akk == 0 && mag(colmax) == 0)) {
       zero = true;
     } else if (absakk < alpha * colmax) {
       slow = true;
       // ---- B: updated column imax into W(:, j+1) and its off-diagonal max
       for (int t = tid; t < j; t += blockDim.x) wrB[t] = __ldcg(Wb + (size_t)t * ldw + imax);
       __syncthreads();
-      T rv = T(-1);
+      Key<T> rv = 0;
       int ri = -1;
       for (int r = first_row(c); r < nrow; r += TT) {
         T acc = r < imax ? __ldcg(S + imax + (size_t)r * nrow) : __ldcg(S + r + (size_t)imax * nrow);
         if (r == gt) {
-          for (int t = 0; t < j; ++t) acc -= lc[t * WP_THREADS + tid] * wrB[t];
+          for (int t = 0; t < j; ++t) acc -= lc[t * WP + tid] * wrB[t];
           w_own1 = acc;
         } else {
           for (int t = 0; t < j; ++t) acc -= __ldcg(S + r + (size_t)(k0 + t) * nrow) * wrB[t];
         }
         Wb[(size_t)(j + 1) * ldw + r] = acc;
         if (r < w && r != imax) {
-          const T a = tabs_w(acc);
-          if (a == a && (ri < 0 || a > rv)) {
+          const Key<T> a = mag(acc);
+          if (!mag_nan<T>(a) && (ri < 0 || a > rv)) {
             rv = a;
             ri = r;
           }
@@ -970,7 +977,7 @@ __global__ void __launch_bounds__(WP_THREADS) k_wide_panel(T *S, int nrow, int w
       }
       T rowmax;
       int rdummy;
-      if (!grid_argmax(rv, ri, ctl, 1, epoch, status, rowmax, rdummy)) return;
+      if (!grid_argmax<T>(rv, ri, ctl, epoch, status, rowmax, rdummy)) return;
       const T diag_imax = tabs_w(__ldcg(Wb + (size_t)(j + 1) * ldw + imax));
       if (absakk >= alpha * colmax * (colmax / rowmax)) {
         kp = c;
@@ -1005,6 +1012,13 @@ __global__ void __launch_bounds__(WP_THREADS) k_wide_panel(T *S, int nrow, int w
         S[kk + (size_t)col * nrow] = __ldcg(S + kp + (size_t)col * nrow);
         S[kp + (size_t)col * nrow] = t;
       }
+      // rows kk, kp of W, a column per thread (one thread walking them waited 350
+      // cycles for each)
+      for (int t2 = gt; t2 < (copycol ? j : j + 2); t2 += TT) {
+        T x = __ldcg(Wb + (size_t)t2 * ldw + kk);
+        Wb[(size_t)t2 * ldw + kk] = __ldcg(Wb + (size_t)t2 * ldw + kp);
+        Wb[(size_t)t2 * ldw + kp] = x;
+      }
       if (gt == 0) {
         T t = __ldcg(S + kk + (size_t)kk * nrow);
         S[kk + (size_t)kk * nrow] = __ldcg(S + kp + (size_t)kp * nrow);
@@ -1016,24 +1030,14 @@ __global__ void __launch_bounds__(WP_THREADS) k_wide_panel(T *S, int nrow, int w
           T a1 = __ldcg(Wb + (size_t)(j + 1) * ldw + kp), a2 = __ldcg(Wb + (size_t)(j + 1) * ldw + kk);
           Wb[(size_t)j * ldw + kk] = a1;
           Wb[(size_t)j * ldw + kp] = a2;
-          for (int t2 = 0; t2 < j; ++t2) {
-            T x = __ldcg(Wb + (size_t)t2 * ldw + kk);
-            Wb[(size_t)t2 * ldw + kk] = __ldcg(Wb + (size_t)t2 * ldw + kp);
-            Wb[(size_t)t2 * ldw + kp] = x;
-          }
-        } else {
-          for (int t2 = 0; t2 <= j + 1; ++t2) {
-            T x = __ldcg(Wb + (size_t)t2 * ldw + kk);
-            Wb[(size_t)t2 * ldw + kk] = __ldcg(Wb + (size_t)t2 * ldw + kp);
-            Wb[(size_t)t2 * ldw + kp] = x;
-          }
         }
         ctl->pivoted = 1;
       }
       unsigned long long dummy;
-      if (!grid_exchange(ctl, epoch, 0ull, status, dummy)) return;
+      int none;
+      if (!grid_exchange<false>(ctl, epoch, 0ull, -1, status, dummy, none)) return;
       if (gt == kk || gt == kp)
-        for (int t = 0; t < j; ++t) lc[t * WP_THREADS + tid] = __ldcg(S + gt + (size_t)(k0 + t) * nrow);
+        for (int t = 0; t < j; ++t) lc[t * WP + tid] = __ldcg(S + gt + (size_t)(k0 + t) * nrow);
     }
     if (slow && gt < nrow) {
       // W entries of the thread's own row after the pivot search / interchange
@@ -1049,10 +1053,10 @@ __global__ void __launch_bounds__(WP_THREADS) k_wide_panel(T *S, int nrow, int w
         // zero pivot column: kept unscaled (LAPACK dlasyf copies W(k:n,k))
         const T l = zero ? wv : wv * r1;
         S[r + (size_t)c * nrow] = l;
-        if (r == gt) lc[j * WP_THREADS + tid] = l;
+        if (r == gt) lc[j * WP + tid] = l;
       }
       if (gt == 0) {
-        if (zero && absakk == absakk) atomicOr(status, ST_ZERO_PIVOT);
+        if (zero && !akk_nan) atomicOr(status, ST_ZERO_PIVOT);
         S[c + (size_t)c * nrow] = T(1);
         Dd[c] = d;
         De[c] = T(0);
@@ -1071,8 +1075,8 @@ __global__ void __launch_bounds__(WP_THREADS) k_wide_panel(T *S, int nrow, int w
         S[r + (size_t)c * nrow] = l0;
         S[r + (size_t)(c + 1) * nrow] = l1;
         if (r == gt) {
-          lc[j * WP_THREADS + tid] = l0;
-          lc[(j + 1) * WP_THREADS + tid] = l1;
+          lc[j * WP + tid] = l0;
+          lc[(j + 1) * WP + tid] = l1;
         }
       }
       if (gt == 0) {
@@ -1706,12 +1710,12 @@ static int run_wide(T *S, int nrow, int w, T *Dd, T *De, int *perm, T *Wb, WideC
   k_wide_init_perm<T><<<(w + 255) / 256, 256, 0, st>>>(perm, w);
   if (P) P->nlaunch++;
   if (cudaMemsetAsync(ctl, 0, offsetof(WideCtl, spin_limit), st) != cudaSuccess) return NQG_ERR_CUDA;
-  const size_t smem = (size_t)(WP_NB + 2) * WP_THREADS * sizeof(T);
+  const size_t smem = (size_t)(WP_NB + 2) * WP_THREADS<T> * sizeof(T);
   // per call: the attribute belongs to the current device
   if (cudaFuncSetAttribute(k_wide_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return NQG_ERR_CUDA;
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wide_panel<T>, WP_THREADS, smem) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wide_panel<T>, WP_THREADS<T>, smem) != cudaSuccess)
     return NQG_ERR_CUDA;
   const int maxG = std::max(1, std::min(occ * num_sms, 1024));
   // FP32 trailing updates: the persistent tcgen05 kernel on packed split
@@ -2074,13 +2078,13 @@ static int run_wide(T *S, int nrow, int w, T *Dd, T *De, int *perm, T *Wb, WideC
     if (fast) {
       if ((rc = launch_fast(k0, kb_want, Wp, -1, delayed ? cs.pend_C : 0, packed))) return rc;
     } else {
-      if (cudaMemsetAsync(&ctl->pslot[0][0], 0, sizeof(ctl->pslot), st) != cudaSuccess) return NQG_ERR_CUDA;
+      if (cudaMemsetAsync(&ctl->pslot[0][0], 0, sizeof(ctl->pslot) + sizeof(ctl->pair), st) != cudaSuccess) return NQG_ERR_CUDA;
       cudaEvent_t e0 = P ? P->prof_begin() : nullptr;
       // one row per thread where the grid allows it
       const int rows_left = nrow - k0;
-      const int G = std::max(1, std::min(maxG, (rows_left + WP_THREADS - 1) / WP_THREADS));
+      const int G = std::max(1, std::min(maxG, (rows_left + WP_THREADS<T> - 1) / WP_THREADS<T>));
       void *args[] = {&S, &nrow, &w, &k0, &kbw, &Wp, &ldw, &Dd, &De, &perm, &ctl, &status};
-      if (cudaLaunchCooperativeKernel((void *)k_wide_panel<T>, dim3(G), dim3(WP_THREADS), args, smem, st) !=
+      if (cudaLaunchCooperativeKernel((void *)k_wide_panel<T>, dim3(G), dim3(WP_THREADS<T>), args, smem, st) !=
           cudaSuccess)
         return NQG_ERR_CUDA;
       if (P) {
