@@ -25,6 +25,7 @@ struct WideCtl {
   unsigned long long pair[2][2048];  // FP64 candidates: two words per CTA, cleared with pslot
   // fast panels: up to four candidate words per CTA and exchange
   unsigned long long mslot[2][4][1024];
+  unsigned long long colkey[64];  // FP64 block-first panel: column maxima as integers
   // polls before a cross-CTA wait gives up (0: SPIN_LIMIT); kept across the
   // per-supernode resets, which clear the fields above only
   long long spin_limit;

@@ -884,6 +884,190 @@ __global__ void __launch_bounds__(FB_THREADS) k_wide_panel_blk(float *S, int nro
   }
 }
 
+// FP64 block-first panel: the same scheme as k_wide_panel_blk with the FP64 pipe
+// as the scarce resource (a warp instruction takes an SM quarter's pipe for 64
+// cycles).  Every CTA factors the diagonal block, P64_RB columns at a time, and
+// carries 32 rows along on warps that the block's chain leaves idle: while one
+// warp factors the P64_RB x P64_RB diagonal, four others apply the step before to
+// the CTA's rows.  W goes to Wb and the column maxima to colkey, nothing to S:
+// k_panel64_finish keeps the columns before the first that needs a pivot search.
+// Entries take the same multiply-adds in the same order as in k_wide_panel.
+// The 26 panels of a 1135-column front: 78 us each, 355 us column by column (an
+// exchange of about 2500 cycles and 32 dependent multiply-adds per column).
+constexpr int P64_THREADS = 256, P64_ROWS = 32, P64_RB = 8, P64_LD = WP_NB;
+constexpr size_t P64_SMEM =
+    ((size_t)WP_NB * P64_LD + (size_t)WP_NB * P64_ROWS + (size_t)P64_RB * P64_LD + (size_t)P64_RB * P64_ROWS) * sizeof(double);
+
+// Columns b .. b + nc of one row against the finished diagonal block there:
+// v becomes W, the result L.
+__device__ __forceinline__ void row_step64(const double *Rc, const double *rinv, int b, int nc, double (&v)[P64_RB],
+                                           double (&lv)[P64_RB]) {
+#pragma unroll
+  for (int c = 0; c < P64_RB; ++c) {
+    if (c >= nc) break;
+#pragma unroll
+    for (int t = 0; t < c; ++t) v[c] -= lv[t] * Rc[(b + t) * P64_LD + b + c];
+    lv[c] = v[c] * rinv[b + c];
+  }
+}
+
+__global__ void __launch_bounds__(P64_THREADS) k_panel64(const double *S, int nrow, int w, int k0, int nb, double *Wb,
+                                                         int ldw, unsigned long long *colkey) {
+  extern __shared__ __align__(16) unsigned char p64_raw[];
+  __shared__ double rinv[WP_NB];
+  double *Rc = reinterpret_cast<double *>(p64_raw);  // [WP_NB][P64_LD]: the block by columns, W values once final
+  double *ws = Rc + WP_NB * P64_LD;                  // [WP_NB][P64_ROWS]: the CTA's rows
+  double *Lb = ws + WP_NB * P64_ROWS;                // [P64_RB][P64_LD]: L of the block's rows in this step
+  double *Lw = Lb + P64_RB * P64_LD;                 // [P64_RB][P64_ROWS]: L of the CTA's rows in this step
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int nbR = min(nb, w - k0);
+  const int r_own = k0 + nbR + blockIdx.x * P64_ROWS + lane;
+#pragma unroll 8
+  for (int e = tid; e < WP_NB * P64_LD; e += P64_THREADS) {
+    const int t = e / P64_LD, i = e % P64_LD;
+    const bool in = t < nbR && i < nbR && i >= t;
+    const double v = S[(k0 + (in ? i : 0)) + (size_t)(k0 + (in ? t : 0)) * nrow];
+    Rc[e] = in ? v : 0.0;
+  }
+#pragma unroll 8
+  for (int j = wid; j < WP_NB; j += P64_THREADS / 32) {
+    const bool in = j < nbR && r_own < nrow;
+    const double v = S[(in ? r_own : k0) + (size_t)(k0 + (in ? j : 0)) * nrow];
+    ws[j * P64_ROWS + lane] = in ? v : 0.0;
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int b = 0; b < nbR; b += P64_RB) {
+    const int nc = min(P64_RB, nbR - b), mb = nbR - b - P64_RB;
+    if (wid == 0) {
+      double v[P64_RB];
+#pragma unroll
+      for (int c = 0; c < P64_RB; ++c) v[c] = lane < nc && c <= lane ? Rc[(b + c) * P64_LD + b + lane] : 0.0;
+      // entries right of the diagonal and beyond the block are never stored
+#pragma unroll
+      for (int t = 0; t < P64_RB; ++t) {
+        const double r1 = 1.0 / __shfl_sync(0xffffffffu, v[t], t);
+        const double l = v[t] * r1;
+#pragma unroll
+        for (int c = t + 1; c < P64_RB; ++c) v[c] -= l * __shfl_sync(0xffffffffu, v[t], c);
+        if (lane == 0 && t < nc) rinv[b + t] = r1;
+      }
+#pragma unroll
+      for (int c = 0; c < P64_RB; ++c)
+        if (lane < nc && c <= lane) Rc[(b + c) * P64_LD + b + lane] = v[c];
+    } else if (wid >= 4 && b > 0) {
+      double l[P64_RB];
+#pragma unroll
+      for (int t = 0; t < P64_RB; ++t) l[t] = Lw[t * P64_ROWS + lane];
+#pragma unroll 1
+      for (int c = b + wid - 4; c < nbR; c += 4) {
+        double v = ws[c * P64_ROWS + lane];
+#pragma unroll
+        for (int t = 0; t < P64_RB; ++t) v -= l[t] * Rc[(b - P64_RB + t) * P64_LD + c];
+        ws[c * P64_ROWS + lane] = v;
+      }
+    }
+    __syncthreads();
+    if (wid < 2) {
+      if (tid < mb) {
+        const int i = b + P64_RB + tid;
+        double v[P64_RB], lv[P64_RB];
+#pragma unroll
+        for (int c = 0; c < P64_RB; ++c) v[c] = Rc[(b + c) * P64_LD + i];
+        row_step64(Rc, rinv, b, P64_RB, v, lv);
+#pragma unroll
+        for (int c = 0; c < P64_RB; ++c) {
+          Rc[(b + c) * P64_LD + i] = v[c];
+          Lb[c * P64_LD + i] = lv[c];
+        }
+      }
+    } else if (wid == 2) {
+      double v[P64_RB], lv[P64_RB];
+#pragma unroll
+      for (int c = 0; c < P64_RB; ++c) v[c] = ws[(b + min(c, nc - 1)) * P64_ROWS + lane];
+      row_step64(Rc, rinv, b, nc, v, lv);
+#pragma unroll
+      for (int c = 0; c < P64_RB; ++c)
+        if (c < nc) {
+          ws[(b + c) * P64_ROWS + lane] = v[c];
+          Lw[c * P64_ROWS + lane] = lv[c];
+        }
+    }
+    __syncthreads();
+    if (mb <= 0) break;
+    // the rest of the block, lower part: columns a and mb - 1 - a together have
+    // mb + 1 entries
+#pragma unroll 1
+    for (int e = tid; e < (mb + 1) / 2 * (mb + 1); e += P64_THREADS) {
+      const int a = e / (mb + 1), c = e % (mb + 1);
+      const bool first = c < mb - a;
+      if (!first && 2 * a == mb - 1) continue;
+      const int jo = first ? a : mb - 1 - a, io = first ? a + c : jo + c - (mb - a);
+      const int i = b + P64_RB + io, jj = b + P64_RB + jo;
+      double x = Rc[jj * P64_LD + i];
+#pragma unroll
+      for (int t = 0; t < P64_RB; ++t) x -= Lb[t * P64_LD + i] * Rc[(b + t) * P64_LD + jj];
+      Rc[jj * P64_LD + i] = x;
+    }
+    __syncthreads();
+  }
+  // column maxima inside the diagonal block of the supernode, and W
+#pragma unroll 1
+  for (int j = wid; j < nbR; j += P64_THREADS / 32) {
+    const double v = ws[j * P64_ROWS + lane];
+    unsigned long long m = r_own < min(nrow, w) ? mag(v) : 0ull;
+    if (mag_nan<double>(m)) m = 0ull;
+    if (r_own < nrow) Wb[(size_t)j * ldw + r_own] = v;
+    if (blockIdx.x == 0)
+      for (int i = j + lane; i < nbR; i += 32) {
+        const double x = Rc[j * P64_LD + i];
+        Wb[(size_t)j * ldw + k0 + i] = x;
+        const unsigned long long k = mag(x);
+        if (i > j && !mag_nan<double>(k)) m = max(m, k);
+      }
+    int any = 0;
+    warp_best(m, any);
+    if (lane == 0 && m) atomicMax(colkey + j, m);
+  }
+}
+
+// L, D of the columns of a block-first panel up to the first whose diagonal fails
+// the Bunch-Kaufman test; kb and stop for the host.
+__global__ void __launch_bounds__(P64_THREADS) k_panel64_finish(double *S, int nrow, int w, int k0, int nb,
+                                                                const double *Wb, int ldw, double *Dd, double *De,
+                                                                WideCtl *ctl) {
+  __shared__ double rinv[WP_NB];
+  __shared__ unsigned pass[2];
+  const int tid = threadIdx.x, nbR = min(nb, w - k0);
+  if (tid < WP_NB) {
+    const int j = min(tid, nbR - 1);
+    const double d = Wb[(size_t)j * ldw + k0 + j];
+    const double alpha = (1.0 + sqrt(17.0)) / 8.0;
+    const bool ok = tid < nbR && mag(d) != 0 && mag_value(mag(d)) >= alpha * mag_value(ctl->colkey[j]);
+    rinv[tid] = 1.0 / d;
+    const unsigned b = __ballot_sync(0xffffffffu, ok);
+    if ((tid & 31) == 0) pass[tid >> 5] = b;
+  }
+  __syncthreads();
+  const unsigned long long failed = ~((unsigned long long)pass[1] << 32 | pass[0]);
+  const int kept = failed ? __ffsll((long long)failed) - 1 : WP_NB;
+  const int r = k0 + blockIdx.x * P64_THREADS + tid;
+  if (r < nrow) {
+    const int below = min(kept, r - k0);  // columns left of the row's diagonal entry
+#pragma unroll 8
+    for (int j = 0; j < below; ++j) S[r + (size_t)(k0 + j) * nrow] = Wb[(size_t)j * ldw + r] * rinv[j];
+    if (r - k0 < kept) {
+      S[r + (size_t)r * nrow] = 1.0;
+      Dd[r] = Wb[(size_t)(r - k0) * ldw + r];
+      De[r] = 0.0;
+    }
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    ctl->kb = kept;
+    ctl->stop = kept < nbR ? 1 : 0;
+  }
+}
+
 // One panel: columns c = k0 .. (at most k0+nb, one more for a final 2x2).
 // Thread gt owns rows gt, gt + TT, ...; the panel entries L(gt, k0 + t) of
 // its first row are cached in shared memory (lc[t][threadIdx.x]) as they are
@@ -1757,6 +1941,10 @@ static int run_wide(T *S, int nrow, int w, T *Dd, T *De, int *perm, T *Wb, WideC
   const char *pe = std::getenv("NASOQ_GB300_PANEL");
   const bool fast_enabled = sizeof(T) == 4 && !(pe && std::string(pe) == "general");
   const bool blk_enabled = fast_enabled && !(pe && std::string(pe) == "group");
+  // FP64: block-first panels (k_panel64) wherever no column needs a search
+  const bool fast64 = sizeof(T) == 8 && !(pe && std::string(pe) == "general");
+  if (fast64 && cudaFuncSetAttribute(k_panel64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P64_SMEM) != cudaSuccess)
+    return NQG_ERR_CUDA;
   const size_t fsmem = fast_panel_smem(nb);
   int maxG_fast = 0, maxG_blk = 0;
   if (fast_enabled) {
@@ -1787,9 +1975,9 @@ static int run_wide(T *S, int nrow, int w, T *Dd, T *De, int *perm, T *Wb, WideC
   // path: 8 columns, NASOQ_GB300_PIVOT_NB overrides, 2 .. nb): the pivots of
   // the KKT systems come singly or in 2 x 2 blocks, so the fast kernel takes
   // over again right after them
-  int pivot_nb = fast_enabled ? std::min(nb, 8) : nb;
+  int pivot_nb = fast_enabled || fast64 ? std::min(nb, 8) : nb;
   if (const char *e = std::getenv("NASOQ_GB300_PIVOT_NB"))
-    if (fast_enabled) pivot_nb = std::min(nb, std::max(2, std::atoi(e)));
+    if (fast_enabled || fast64) pivot_nb = std::min(nb, std::max(2, std::atoi(e)));
   // where pivots are dense (a fast panel stops again within nb / 4 columns)
   // the general panels double in width, up to nb, so that fewer of them --
   // each flushes the pending updates -- are needed; back to pivot_nb after a
@@ -1798,6 +1986,11 @@ static int run_wide(T *S, int nrow, int w, T *Dd, T *De, int *perm, T *Wb, WideC
   auto after_fast = [&](bool stopped, int kept) {
     gen_w = !stopped || kept >= nb / 4 ? pivot_nb : std::min(nb, 2 * gen_w);
   };
+  // FP64: a panel that stops early costs about a fifth of a general one; where
+  // they keep stopping, 1, 3, then 7 general panels follow each (2545 columns,
+  // 2 x 2 pivots throughout: 34.2 ms, all panels general 33.3; 1100 columns
+  // without a search 3.0 and 8.1)
+  int misses = 0, skip = 0;
   bool use_general = false;  // the next panel starts at a column that needs a pivot search
   // Delayed trailing updates (FP32 tcgen05 path): up to `depth` consecutive
   // panels are pending, their W columns side by side in Wb, and one update of
@@ -1944,9 +2137,9 @@ static int run_wide(T *S, int nrow, int w, T *Dd, T *De, int *perm, T *Wb, WideC
         int tm = (nrow - k1 + BM - 1) / BM, tn = (w - k1 + BN - 1) / BN;
         k_wide_trailing<T, BM, BN, 8, 8><<<tm * tn, 256, 0, st>>>(S, nrow, w, k0, kb, Wb, nrow, tn);
       } else {
-        constexpr int BM = 64, BN = 64;
+        constexpr int BM = 32, BN = 32;
         int tm = (nrow - k1 + BM - 1) / BM, tn = (w - k1 + BN - 1) / BN;
-        k_wide_trailing<T, BM, BN, 4, 4><<<tm * tn, 256, 0, st>>>(S, nrow, w, k0, kb, Wb, nrow, tn);
+        k_wide_trailing<T, BM, BN, 2, 2><<<tm * tn, 256, 0, st>>>(S, nrow, w, k0, kb, Wb, nrow, tn);
       }
       if (cudaGetLastError() != cudaSuccess) return NQG_ERR_CUDA;
       if (P) {
@@ -2049,7 +2242,7 @@ static int run_wide(T *S, int nrow, int w, T *Dd, T *De, int *perm, T *Wb, WideC
     // that needs a pivot search) is at most gen_w columns wide, so that the
     // fast kernel takes over again soon after the pivots
     const int kb_want = std::min(use_general ? gen_w : nb, w - cs.k0);
-    const bool fast = fast_enabled && !use_general && nrow - cs.k0 - kb_want <= maxG_fast * FP_THREADS;
+    const bool fast = !use_general && (fast64 || (fast_enabled && nrow - cs.k0 - kb_want <= maxG_fast * FP_THREADS));
     if (fast && spec_ok) {
       int rc = pre(cs, false, kb_want);
       if (rc) return rc;
@@ -2075,7 +2268,22 @@ static int run_wide(T *S, int nrow, int w, T *Dd, T *De, int *perm, T *Wb, WideC
     T *Wp = Wb + (size_t)woff * nrow;
     int kb = 0, abort = 0, stop = 0, ldw = nrow, kbw = kb_want, k0 = cs.k0;
     bool packed = false;
-    if (fast) {
+    if (fast && fast64) {
+      if constexpr (sizeof(T) == 8) {
+        if (cudaMemsetAsync(&ctl->colkey[0], 0, sizeof(ctl->colkey), st) != cudaSuccess) return NQG_ERR_CUDA;
+        cudaEvent_t e0 = P ? P->prof_begin() : nullptr;
+        const int below = nrow - k0 - kb_want;
+        k_panel64<<<std::max(1, (below + P64_ROWS - 1) / P64_ROWS), P64_THREADS, P64_SMEM, st>>>(
+            S, nrow, w, k0, kb_want, Wp, ldw, &ctl->colkey[0]);
+        k_panel64_finish<<<(nrow - k0 + P64_THREADS - 1) / P64_THREADS, P64_THREADS, 0, st>>>(S, nrow, w, k0, kb_want,
+                                                                                           Wp, ldw, Dd, De, ctl);
+        if (cudaGetLastError() != cudaSuccess) return NQG_ERR_CUDA;
+        if (P) {
+          P->nlaunch += 2;
+          P->prof_end(NQG_K_WIDE_PANEL, e0, panel_flops(k0, kb_want), 0.0);
+        }
+      }
+    } else if (fast) {
       if ((rc = launch_fast(k0, kb_want, Wp, -1, delayed ? cs.pend_C : 0, packed))) return rc;
     } else {
       if (cudaMemsetAsync(&ctl->pslot[0][0], 0, sizeof(ctl->pslot) + sizeof(ctl->pair), st) != cudaSuccess) return NQG_ERR_CUDA;
@@ -2101,12 +2309,16 @@ static int run_wide(T *S, int nrow, int w, T *Dd, T *De, int *perm, T *Wb, WideC
     if (fast) {
       use_general = stop != 0;
       after_fast(use_general, kb);
+      if (fast64) {
+        misses = use_general && kb < nb / 4 ? std::min(misses + 1, 3) : 0;
+        skip = (1 << misses) - 1;
+      }
       if (kb <= 0) {
         if (!use_general) return NQG_ERR_TIMEOUT;
         continue;  // the first column already needs the general kernel
       }
     } else {
-      use_general = false;
+      use_general = fast64 && --skip > 0;
       if (kb <= 0) return NQG_ERR_TIMEOUT;
     }
     if ((rc = post(cs, kb, woff, packed && kb == kb_want))) return rc;
