@@ -423,6 +423,8 @@ static int upload_plan(Plan &P) {
   // flag) its inverse and the two last-link products, 64 x 65 floats each
   if (P.set.precision == NQG_FP32 && P.set.solve_precision == NQG_FP32)
     NQG_CUDA(cudaMalloc(&P.d_tinv, (size_t)std::max(nflags, 1) * 3 * 64 * 65 * sizeof(float)));
+  else if (P.set.precision == NQG_FP64)  // the two inverted triangles and L21 of a tile
+    NQG_CUDA(cudaMalloc(&P.d_tinv, (size_t)std::max(nflags, 1) * 64 * 65 * sizeof(double)));
   P.solve_small_w = small_w;
   if ((rc = dev_alloc_copy(P, &P.d_targets_lv, lvflat.data(), lvflat.size()))) return rc;
   P.lv_targets_host = lvflat;

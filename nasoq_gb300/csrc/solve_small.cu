@@ -42,7 +42,8 @@ constexpr int SS_LONG = 16;           // rows of a single column above which it 
 constexpr int SS_WARP_BLOCK = 128;    // rows x columns of the largest block a warp takes ...
 constexpr int SS_WARP_CROWD = 1024;   // ... and in a level with more large blocks than SS_CROWD
 constexpr int SS_CROWD = 2 * SS_CTAS;
-constexpr int SS_WIDE = 640;          // widest block (merged), unless there are many levels
+constexpr int SS_WIDE = 448;          // widest block (merged) ...
+constexpr int64_t SS_PER_LEVEL = 1 << 14;  // ... its square per level kernel, where there are many
 constexpr int SS_ROW = 16;            // entries of K's longest rows that take a thread
 constexpr int SS_N_MAX = 32000;       // columns: the column table has to fit in shared memory
 constexpr int64_t SS_ENTRIES_MAX = 1 << 24;  // factor entries: offsets are 32-bit
@@ -835,15 +836,16 @@ int solve_small_setup(Plan &P, const std::vector<int> &Rp) {
     if (c == 2) P.ss_wmax = std::max(P.ss_wmax, width(b));
   }
   // The level kernels and the block kernels stay the better ones where one
-  // wide block is most of the work (they spread it over the chip): dense
-  // systems take 0.85 ms here and 1.33 ms there at 512 columns, 1.65 and 1.63 at
-  // 768; a 20^3 Laplacian (widest block 615) 2.47 and 3.37; a 160^2 one (237)
-  // 2.31 and 2.86; a QP's 2064 columns in 115 levels 8.8 and 18.2 ms per
-  // active-set iteration, 6522 columns in 368 levels 54.6 and 105.0.
+  // wide block is most of the work (they spread it over the chip; here its cost
+  // grows with the square of the width, there with the levels).  A refined
+  // solve, here and there: dense 256 columns 0.31 and 0.62 ms, 384 0.55 and 0.70,
+  // 512 0.84 and 0.71; 16^3 Laplacian (widest block 277) 0.84 and 1.11, 20^3 (615)
+  // 2.44 and 2.32, 160^2 (237) 2.28 and 2.38.  An active-set iteration of a QP with
+  // 2064 columns in 115 levels 6.6 and 15.6 ms, 6522 in 368 levels 41 and 91.
   int launches = 0;
   for (size_t l = 0; l < P.levels.size(); ++l)
     launches += (P.level_off[l + 1] > P.level_off[l]) + (P.blk_fwd_off[l + 1] > P.blk_fwd_off[l]);
-  if (P.ss_wmax > std::max(SS_WIDE, 4 * launches)) return NQG_OK;
+  if ((int64_t)P.ss_wmax * P.ss_wmax > std::max<int64_t>(SS_WIDE * SS_WIDE, SS_PER_LEVEL * launches)) return NQG_OK;
   std::vector<int> rec, seg(1, 0), rows, inv0, chunk;
   for (auto &list : lists) {
     // the largest first: they are dealt out in turn

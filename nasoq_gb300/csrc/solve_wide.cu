@@ -149,12 +149,98 @@ __global__ void __launch_bounds__(TB) k_tile_inverse(const int2 *items, const in
   }
 }
 
+// FP64 factors: the two 32 x 32 triangles of every diagonal tile inverted, L21
+// as it is, entry (k, c) at [c * (TB + 1) + k].  Substitution took 64 steps of
+// about 200 cycles per tile forward and, its column reads on one bank, twice
+// that backward: 10 and 18 us a tile along the chain of a wide block; the three
+// products of tile_solve take about 3000 cycles.  Warp h inverts half h, lane =
+// column, FP64 pipe bound (496 multiply-adds of 64 cycles).
+__global__ void __launch_bounds__(TB) k_tile_inverse64(const int2 *items, const int *super, const int64_t *lpi,
+                                                       const int64_t *lpx, const double *L, const int *flagoff,
+                                                       double *tinv) {
+  __shared__ double T11[TI];
+  const int s = items[blockIdx.x].x, q = items[blockIdx.x].y;
+  const int c0 = super[s], w = super[s + 1] - c0;
+  const int nrow = (int)(lpi[s + 1] - lpi[s]);
+  const int j = (w + TB - 1) / TB - 1 - q;
+  const int b0 = j * TB, m = min(TB, w - b0);
+  const double *S = L + lpx[s] + b0 + (size_t)b0 * nrow;
+#pragma unroll 8
+  for (int e = threadIdx.x; e < TB * TB; e += TB) {
+    const int cc = e / TB, r = e % TB;
+    const bool in = r < m && cc < r;
+    const double v = S[in ? r + (size_t)cc * nrow : 0];
+    T11[r + cc * (TB + 1)] = in ? v : 0.0;
+  }
+  __syncthreads();
+  const int h = (threadIdx.x & 32), c = threadIdx.x & 31;
+  double x[32];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) x[k] = k == c ? 1.0 : 0.0;
+  const double *A = T11 + h * (TB + 1) + h;
+  // entries above row c stay 0: the recurrence needs no predicate
+#pragma unroll
+  for (int i = 1; i < 32; ++i) {
+    double acc = 0.0;
+#pragma unroll
+    for (int k = 0; k < i; ++k) acc = fma(A[i + k * (TB + 1)], x[k], acc);
+    x[i] -= acc;
+  }
+  double *out = tinv + (size_t)(flagoff[s] + j) * TI + (size_t)(h + c) * (TB + 1);
+#pragma unroll
+  for (int k = 0; k < 32; ++k) {
+    out[h + k] = x[k];
+    out[32 - h + k] = h ? 0.0 : T11[32 + k + c * (TB + 1)];
+  }
+  out[TB] = 0.0;
+}
+
+// yb (64 entries, zeros beyond the block) := T^-1 yb, or T^-T yb, by the CTA:
+// every warp has four columns (rows) of each product.
+__device__ __forceinline__ void tile_solve(const double *Td, double *yb, double (*red)[SW_THREADS / 32][32], bool trans) {
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, own = 4 * wi + (lane & 3);
+  auto product = [&](const double *M, double v, int buf) {
+    double y = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = 4 * wi + q;
+      y += (trans ? M[lane * (TB + 1) + k] : M[k * (TB + 1) + lane]) * __shfl_sync(0xffffffffu, v, q);
+    }
+    red[buf][wi][lane] = y;
+    __syncthreads();
+    double t = red[buf][lane >> 2][own];
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+  };
+  const double *T22 = Td + 32 * (TB + 1) + 32, *L21 = Td + 32;
+  double x1, x2;
+  if (!trans) {
+    x1 = product(Td, yb[own], 0);
+    x2 = product(T22, yb[32 + own] - product(L21, x1, 1), 0);
+  } else {
+    x2 = product(T22, yb[32 + own], 0);
+    x1 = product(Td, yb[own] - product(L21, x2, 1), 0);
+  }
+  if (lane < 4) {
+    yb[own] = x1;
+    yb[32 + own] = x2;
+  }
+}
+
 // Matrix `part` (0: T, 1: Mf, 2: Mb) of diagonal tile (s, j) into shared
 // memory (FP32 sweeps).
 __device__ __forceinline__ void stage_inverse(const float *tinv, const int *flagoff, int s, int j, float *Ti,
                                               int part = 0) {
   const float4 *src = reinterpret_cast<const float4 *>(tinv + ((size_t)(flagoff[s] + j) * 3 + part) * TI);
   for (int e = threadIdx.x; e < TI / 4; e += blockDim.x) reinterpret_cast<float4 *>(Ti)[e] = __ldcg(src + e);
+}
+
+template <class V>
+__device__ __forceinline__ void stage_inverse64(const float *tinv, const int *flagoff, int s, int j, V *Td) {
+  const double *src = reinterpret_cast<const double *>(tinv) + (size_t)(flagoff[s] + j) * TI;
+#pragma unroll 4
+  for (int e = threadIdx.x; e < TI; e += blockDim.x) Td[e] = V(__ldcg(src + e));
 }
 
 // Entries (r, c0 .. c0 + CPT - 1) of matrix `part` of diagonal tile (s, j),
@@ -298,8 +384,10 @@ __global__ void __launch_bounds__(SW_THREADS) k_fwd_blk(const int2 *items, int n
                                                         unsigned epoch, const uint8_t *visible, WideCtl *ctl,
                                                         int *status, unsigned long long *xw, const float *tinv) {
   constexpr bool WORDS = sizeof(V) == 4;  // x of the diagonal blocks through words
+  constexpr bool INV64 = sizeof(T) == 8;  // FP64 factor: tiles with inverted triangles
   __shared__ __align__(16) V Td[TB * (TB + 1)];  // diagonal tile (FP32: its inverse)
   __shared__ V red[SW_THREADS];
+  __shared__ double red64[INV64 ? 2 : 1][SW_THREADS / 32][32];
   __shared__ V yb[TB];
   __shared__ int s_front;
   const int t = threadIdx.x, r = t & (TB - 1), cg = t / TB;
@@ -327,6 +415,8 @@ __global__ void __launch_bounds__(SW_THREADS) k_fwd_blk(const int2 *items, int n
     if constexpr (WORDS) {
       if (diag) stage_inverse(tinv, flagoff, s, q, Td);
       if (diag && q > 0) load_link(tinv, flagoff, s, q, 1, r, cg * CPT, mlink);
+    } else if constexpr (INV64) {
+      if (diag) stage_inverse64(tinv, flagoff, s, q, Td);
     } else {
       if (diag) stage_tile(S, nrow, r0, m, Td);
     }
@@ -385,7 +475,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_fwd_blk(const int2 *items, int n
     if (t < TB) yb[t] = red[t] + red[t + TB] + red[t + 2 * TB] + red[t + 3 * TB];
     __syncthreads();
     if (diag) {
-      if (t < m) yb[t] = bq - yb[t];
+      if (t < TB) yb[t] = t < m ? bq - yb[t] : V(0);
       __syncthreads();
       if constexpr (WORDS) {
         // c_q = T_q y_q (thread t < TB keeps entry t)
@@ -416,7 +506,8 @@ __global__ void __launch_bounds__(SW_THREADS) k_fwd_blk(const int2 *items, int n
           put_word(xw + c0 + r0 + t, epoch, float(xq));
         }
       } else {
-        if (t < 32) warp_trsv_lower(Td, m, yb);
+        if constexpr (INV64) tile_solve(Td, yb, red64, false);
+        else if (t < 32) warp_trsv_lower(Td, m, yb);
         __syncthreads();
         if (t < m) xs[r0 + t] = yb[t];
         __syncthreads();
@@ -439,8 +530,10 @@ __global__ void __launch_bounds__(SW_THREADS) k_bwd_blk(const int2 *items, int n
                                                         unsigned epoch, const uint8_t *visible, WideCtl *ctl,
                                                         int *status, unsigned long long *xw, const float *tinv) {
   constexpr bool WORDS = sizeof(V) == 4;  // x of the diagonal blocks through words
+  constexpr bool INV64 = sizeof(T) == 8;  // FP64 factor: tiles with inverted triangles
   __shared__ __align__(16) V Td[TB * (TB + 1)];  // diagonal tile (FP32: its inverse)
   __shared__ V red[2][TB];
+  __shared__ double red64[INV64 ? 2 : 1][SW_THREADS / 32][32];
   __shared__ V redS[sizeof(V) == 4 ? TB * (TB + 1) : 1];  // FP32: column sums through a transpose
   __shared__ V yb[TB];
   __shared__ int s_front;
@@ -467,6 +560,8 @@ __global__ void __launch_bounds__(SW_THREADS) k_bwd_blk(const int2 *items, int n
     if constexpr (WORDS) {
       stage_inverse(tinv, flagoff, s, j, Td);
       if (j + 1 < nbd) load_link(tinv, flagoff, s, j, 2, r, cg * CPT, mlink);
+    } else if constexpr (INV64) {
+      stage_inverse64(tinv, flagoff, s, j, Td);
     } else {
       stage_tile(S, nrow, b0, nc, Td);
     }
@@ -567,16 +662,22 @@ __global__ void __launch_bounds__(SW_THREADS) k_bwd_blk(const int2 *items, int n
         yb[t] = __ldcg(xs + b0 + t) - ((a0 + a1) + (a2 + a3));
       }
     } else {
-      // warps 2cg and 2cg+1 hold rows 0-31, 32-63
+      // warps 2cg and 2cg+1 hold rows 0-31, 32-63; the columns are halved with
+      // the lanes (16 additions, not 80), lane 2c ends with column c
+      static_assert(CPT == 16, "four halvings");
 #pragma unroll
-      for (int cc = 0; cc < CPT; ++cc) {
-        V a = part[cc];
+      for (int h = CPT / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) red[(t >> 5) & 1][cg * CPT + cc] = a;
+        for (int c = 0; c < h; ++c) {
+          const V mine = up ? part[c + h] : part[c], other = up ? part[c] : part[c + h];
+          part[c] = mine + __shfl_xor_sync(0xffffffffu, other, o);
+        }
       }
+      part[0] += __shfl_xor_sync(0xffffffffu, part[0], 1);
+      if ((lane & 1) == 0) red[(t >> 5) & 1][cg * CPT + (lane >> 1)] = part[0];
       __syncthreads();
-      if (t < nc) yb[t] = __ldcg(xs + b0 + t) - (red[0][t] + red[1][t]);
+      if (t < TB) yb[t] = t < nc ? __ldcg(xs + b0 + t) - (red[0][t] + red[1][t]) : V(0);
     }
     __syncthreads();
     if constexpr (WORDS) {
@@ -608,7 +709,8 @@ __global__ void __launch_bounds__(SW_THREADS) k_bwd_blk(const int2 *items, int n
         put_word(xw + c0 + b0 + t, epoch, float(xj));
       }
     } else {
-      if (t < 32) warp_trsv_lower_t(Td, nc, yb);
+      if constexpr (INV64) tile_solve(Td, yb, red64, true);
+      else if (t < 32) warp_trsv_lower_t(Td, nc, yb);
       __syncthreads();
       if (t < nc) xs[b0 + t] = yb[t];
       __syncthreads();
@@ -666,6 +768,21 @@ template <class T, class V> static int launch_blk(Plan &P, bool fwd, int l, cons
                                                         P.blk_bwd_off.front(),
                                                     super, lpi, lpx, reinterpret_cast<const float *>(L), flagoff,
                                                     P.d_tinv);
+        NQG_CUDA(cudaGetLastError());
+        P.nlaunch++;
+        P.prof_end(NQG_K_SOLVE, ei, 0.0, 0.0);
+      }
+      P.tinv_valid = true;
+    }
+  } else if constexpr (sizeof(T) == 8) {
+    if (!tinv) return NQG_ERR_ARG;
+    if (!P.tinv_valid) {
+      const int nb_all = P.blk_bwd_off.back() - P.blk_bwd_off.front();
+      if (nb_all > 0) {
+        cudaEvent_t ei = P.prof_begin();
+        k_tile_inverse64<<<nb_all, TB, 0, P.stream>>>(
+            reinterpret_cast<const int2 *>(P.d_blk_items) + P.blk_bwd_off.front(), super, lpi, lpx,
+            reinterpret_cast<const double *>(L), flagoff, reinterpret_cast<double *>(P.d_tinv));
         NQG_CUDA(cudaGetLastError());
         P.nlaunch++;
         P.prof_end(NQG_K_SOLVE, ei, 0.0, 0.0);

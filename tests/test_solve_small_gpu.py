@@ -26,7 +26,7 @@ def _bordered(nblk, w, border, rng):
     return np.tril(a) + np.tril(a, -1).T
 
 
-CASES = {f"dense{n}": (lambda r, n=n: _dense(n, r)) for n in (1, 2, 31, 32, 33, 64, 65, 161)}
+CASES = {f"dense{n}": (lambda r, n=n: _dense(n, r)) for n in (1, 2, 31, 32, 33, 64, 65, 95, 97, 128, 161)}
 CASES |= {f"singles_border{m}": (lambda r, m=m: _bordered(300, 1, m, r)) for m in (1, 14, 15, 16, 17, 40)}
 CASES |= {
     "blocks17x24": lambda r: _bordered(17, 24, 30, r),
@@ -47,14 +47,14 @@ def test_matches_level_kernels(name, monkeypatch):
     low.sort_indices()
     rhs = rng.standard_normal(n)
     xs = []
-    for general in (False, True):
+    for general in (None, "64,256", "0,0"):  # 0,0: every supernode on the block kernels' 64-column tiles
         if general:
-            monkeypatch.setenv("NASOQ_GB300_SOLVE_SMALL", "64,256")
+            monkeypatch.setenv("NASOQ_GB300_SOLVE_SMALL", general)
         plan = nq.Plan(n, low.indptr, low.indices, low.data)
         plan.factor()
         before = plan.launch_count()
         xs.append(plan.solve(rhs))
-        assert (plan.launch_count() - before == 1) != general
+        assert (plan.launch_count() - before == 1) != bool(general)
     # a refined solve is backward stable: |b - Ax| <= n eps (|A||x| + |b|), row by row at most n products
     eps = np.finfo(float).eps
     for x in xs:
