@@ -33,7 +33,9 @@ def family_batch(fam: P.ParametricQP, count: int, **settings) -> nq.QPBatch:
 def set_theta(batch: nq.QPBatch, fam: P.ParametricQP, thetas: np.ndarray):
     """q = P theta, d = d0 + S theta for every problem of the batch."""
     q = thetas @ fam.P.T
-    d = fam.d0[None, :] + thetas @ fam.S.T
+    d = thetas @ fam.S.T
+    # in place: a second array of this size costs as much as the product
+    d = np.add(d, fam.d0, out=d if d.dtype == np.result_type(d, fam.d0) else None)
     batch.set_vectors(q_all=q.ravel(), d_all=d.ravel())
 
 
