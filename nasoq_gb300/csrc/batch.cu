@@ -498,7 +498,7 @@ __device__ __forceinline__ void sn_finish(Ctx<T> &c, int s, int c0, int w, int n
   const int m = nr - w;
   // a lane keeps its row: R of them, the other index over nt / R
   int R = 32;
-  while (R < nt && R < nr) R *= 2;
+  while (nt % (2 * R) == 0 && R < nr) R *= 2;  // nt need not be a power of two
   const int rr = tid & (R - 1), cq = tid / R, cs = nt / R;
   if (pivoted) {  // columns of the rows below into pivot order (cycles, in place)
 #pragma unroll 1

@@ -425,7 +425,7 @@ __device__ __forceinline__ void rows_solve(T *X, int m, int w, int lr, int lj, c
                                            int nt) {
   // a lane keeps its row: R of them, the other index over nt / R
   int R = 32;
-  while (R < nt && R < m) R *= 2;
+  while (nt % (2 * R) == 0 && R < m) R *= 2;  // nt need not be a power of two
   const int rr = tid & (R - 1), cq = tid / R, cs = nt / R;
 #pragma unroll 1
   for (int j = 0; j + 1 < w; ++j) {
