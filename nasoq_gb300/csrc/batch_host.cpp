@@ -39,6 +39,7 @@ struct HostQP {
 };
 
 struct HostPattern {
+  int threads = 128;  // CTA size its lists are laid out for
   int rep = -1;  // a problem of this pattern
   BPat P{};
   nqg::Symbolic S;
@@ -105,7 +106,19 @@ void super_kkt(const HostQP &Q, nqg::Csc &K, std::vector<double> *vals) {
   }
 }
 
-std::string build_pattern(const HostQP &Q, HostPattern &H, const int nrelax[3], const double zrelax[3], int threads) {
+// CTA size of a batch whose settings leave it open.  A batch of at most two
+// problems per SM leaves the chip's warps idle: larger systems then take more
+// threads (registers allow two CTAs of 256 on an SM, four of 128).  Kernel times
+// at 128 / 192 / 256 threads, FP64 unless said, by entries of the factor: 831 (152
+// random QPs) 5.0 / 5.1 / 5.3 ms; 2771 (152 MPC, horizon 10) 2.37 / 2.31 / 2.44; 5775
+// (horizon 20) 4.29 / 4.15 / 4.35; 7568 (horizon 30, FP32) 6.46 / 5.96 / 5.77; 8941 (96
+// random) 70.3 / 60.7 / 57.7; 14971 (152 MPC, horizon 50) 14.4 / 12.5 / 12.3.  Beyond two
+// problems per SM four CTAs of 128 are faster: 1024 of horizon 50 31.5 / 39.9 / 40.5.
+int threads_for(int64_t entries, bool few) { return !few || entries < 2500 ? 128 : entries < 6000 ? 192 : 256; }
+
+// threads: of a CTA (0: by size)
+std::string build_pattern(const HostQP &Q, HostPattern &H, const int nrelax[3], const double zrelax[3], int threads,
+                          bool few) {
   const int n = Q.n, meq = Q.meq, mineq = Q.mineq, N = n + meq + mineq, base = n + meq;
   nqg::Csc K;
   super_kkt(Q, K, nullptr);
@@ -115,6 +128,8 @@ std::string build_pattern(const HostQP &Q, HostPattern &H, const int nrelax[3], 
   std::string err = nqg::analyze(K, extra.data(), nrelax, zrelax, S);
   if (!err.empty()) return err;
   const int ns = S.nsuper;
+  if (threads <= 0) threads = threads_for(S.xsize, few);
+  H.threads = threads;
   if (S.xsize > (1ll << 30) || (int64_t)S.ls.size() > (1ll << 30)) return "pattern too large for the batched solver";
   BPat &P = H.P;
   P.n = n;
@@ -664,7 +679,11 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
   // ---- patterns
   const int nrelax[3] = {4, 16, 48};
   const double zrelax[3] = {0.8, 0.1, 0.05};
-  const int threads = b->set.threads > 0 ? b->set.threads : 128;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    b->num_sms = 0;  // reported below, after the problems' own errors
+  b->threads = 0;
   std::unordered_map<uint64_t, std::vector<int>> by_key;
   for (int i = 0; i < np; ++i) {
     HostQP &Q = b->qp[i];
@@ -675,8 +694,9 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
     if (found < 0) {
       HostPattern H;
       H.rep = i;
-      std::string err = build_pattern(Q, H, nrelax, zrelax, threads);
+      std::string err = build_pattern(Q, H, nrelax, zrelax, b->set.threads, np <= 2 * b->num_sms);
       if (!err.empty()) return fail(b, NQG_ERR_SYMBOLIC, err);
+      b->threads = std::max(b->threads, H.threads);
       found = (int)b->pats.size();
       b->pats.push_back(std::move(H));
       by_key[key].push_back(found);
@@ -884,12 +904,10 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
   // run side by side on forked streams.  Problems that fit no tier (or all
   // of them, with staging off) keep them in their slot (L2 / HBM).
   BQ_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
-  int dev = 0;
   BQ_CUDA(cudaGetDevice(&dev));
   BQ_CUDA(cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, dev));
   int smem_optin = 0;
   BQ_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  b->threads = threads;
   if (b->threads % 32 || b->threads > 256) return fail(b, NQG_ERR_ARG, "threads must be a multiple of 32, at most 256");
   nqg::BArgs base_args{};
   base_args.N_max = N_max;
