@@ -569,7 +569,11 @@ __global__ void __launch_bounds__(FP_THREADS) k_wide_panel_fast(float *S, int nr
   }
 }
 
-// Block-first fast panel (no pivot search).  The nbR x nbR diagonal block R
+// Block-first fast panel (no pivot search).  Latency bounds it: of 62000 cycles
+// with 26 CTAs, R's chain is 17500, the rows 14300, the writes 11500, the exchange
+// 5500, the column maxima 3700 (34 -> 28 us a panel of the 7741-column front of a
+// 64000-variable KKT system once no thread walks the columns alone and no CTA
+// writes R for all).  The nbR x nbR diagonal block R
 // is factored first, replicated in every CTA with diagonal pivots assumed,
 // FB_RB columns at a time (one warp factors the diagonal block of the step
 // with shuffles, the rows below it are solved against that block, then a
@@ -603,7 +607,7 @@ __global__ void __launch_bounds__(FB_THREADS) k_wide_panel_blk(float *S, int nro
   extern __shared__ __align__(16) unsigned char fb_raw[];
   __shared__ float rinv[WP_NB];
   __shared__ unsigned cpart[FB_THREADS / WP_NB][WP_NB];
-  __shared__ int s_kept;
+  __shared__ unsigned s_pass[2];
   if (*(volatile int *)&ctl->halt) return;  // queued behind a fast panel that stopped early
   const int nbR = min(nb, w - k0);           // panel columns = rows of R
   float *wsm = reinterpret_cast<float *>(fb_raw);  // [WP_NB][FB_THREADS]: W of the thread's row
@@ -686,9 +690,12 @@ __global__ void __launch_bounds__(FB_THREADS) k_wide_panel_blk(float *S, int nro
       }
     }
     __syncthreads();
-    for (int e = tid; e < mb * mb; e += FB_THREADS) {
-      const int io = e % mb, jo = e / mb;
-      if (io < jo) continue;
+    // lower part: columns a and mb - 1 - a together have mb + 1 entries
+    for (int e = tid; e < (mb + 1) / 2 * (mb + 1); e += FB_THREADS) {
+      const int a = e / (mb + 1), c = e % (mb + 1);
+      const bool first = c < mb - a;
+      if (!first && 2 * a == mb - 1) continue;
+      const int jo = first ? a : mb - 1 - a, io = first ? a + c : jo + c - (mb - a);
       const int i = b + FB_RB + io, jj = b + FB_RB + jo;
       float x = Rc[jj * FB_LD + i];
 #pragma unroll
@@ -737,15 +744,18 @@ __global__ void __launch_bounds__(FB_THREADS) k_wide_panel_blk(float *S, int nro
   unsigned long long *slots = &ctl->mslot[0][0][0];
   const int nvalid = max(0, min(FB_THREADS, min(nrow, w) - (k0 + nbR + (int)blockIdx.x * FB_THREADS)));
   for (int j = wid; j < nbR; j += FB_THREADS / 32) {
+    // every load unconditional, so that they overlap (6000 cycles for the 64
+    // columns when they waited for one another)
     unsigned m = 0u;
-#pragma unroll 4
-    for (int t = lane; t < nvalid; t += 32) {
-      const float a = fabsf(wsm[j * FB_THREADS + t]);
-      if (a == a) m = max(m, __float_as_uint(a));
+#pragma unroll
+    for (int t = lane; t < FB_THREADS; t += 32) {
+      const unsigned a = mag(wsm[j * FB_THREADS + t]);
+      if (t < nvalid && !mag_nan<float>(a)) m = max(m, a);
     }
-    for (int i = j + 1 + lane; i < nbR; i += 32) {
-      const float a = fabsf(Rc[j * FB_LD + i]);
-      if (a == a) m = max(m, __float_as_uint(a));
+#pragma unroll
+    for (int i = lane; i < WP_NB; i += 32) {
+      const unsigned a = mag(Rc[j * FB_LD + i]);
+      if (i > j && i < nbR && !mag_nan<float>(a)) m = max(m, a);
     }
     m = __reduce_max_sync(0xffffffffu, m);
     if (lane == 0)
@@ -802,25 +812,25 @@ __global__ void __launch_bounds__(FB_THREADS) k_wide_panel_blk(float *S, int nro
     if (fail) return;
     __syncthreads();
   }
-  if (tid == 0) {
-    int k = 0;
-    for (; k < nbR; ++k) {
-      unsigned mb = 0u;
+  // columns before the first that needs a pivot search or has a zero or NaN
+  // pivot, a column per thread (one thread walking them took 6500 cycles)
+  if (tid < WP_NB) {
+    unsigned mb = 0u;
 #pragma unroll
-      for (int p = 0; p < FB_THREADS / WP_NB; ++p) mb = max(mb, cpart[p][k]);
-      const float colmax = __uint_as_float(mb);
-      const float absakk = fabsf(Rc[k * FB_LD + k]);
-      if (!(absakk >= alpha * colmax) || absakk == 0.f) break;  // pivot search, zero or NaN pivot
-    }
-    s_kept = k;
+    for (int p = 0; p < FB_THREADS / WP_NB; ++p) mb = max(mb, cpart[p][tid]);
+    const float absakk = fabsf(Rc[tid * FB_LD + tid]);
+    const unsigned bal = __ballot_sync(0xffffffffu, tid < nbR && absakk >= alpha * __uint_as_float(mb) && absakk != 0.f);
+    if (lane == 0) s_pass[wid] = bal;
   }
   __syncthreads();
   // --- global writes of the kept columns
-  const int kept = s_kept;
+  const unsigned long long failed = ~((unsigned long long)s_pass[1] << 32 | s_pass[0]);
+  const int kept = failed ? __ffsll((long long)failed) - 1 : WP_NB;
   // W goes to Wb only where a later kernel reads it there: without packed
   // operands, or for a short panel (its operands are packed again from Wb)
   const bool wb_out = !pack_a || kept < nbR;
   if (own)
+#pragma unroll 8
     for (int j = 0; j < kept; ++j) {
       const float wv = wsm[j * FB_THREADS + tid];
       if (wb_out) Wb[(size_t)j * ldw + r_own] = wv;
@@ -858,28 +868,28 @@ __global__ void __launch_bounds__(FB_THREADS) k_wide_panel_blk(float *S, int nro
     if (pk_bf) pack_row(std::true_type{});
     else pack_row(std::false_type{});
   }
-  if (blockIdx.x == 0) {
-    for (int e = tid; e < kept * nbR; e += FB_THREADS) {
-      const int j = e / nbR, i = e % nbR;
-      if (i < j) continue;
-      const float v = Rc[j * FB_LD + i];
-      const int c = k0 + j;
-      if (wb_out) Wb[(size_t)j * ldw + k0 + i] = v;
-      if (i > j) {
-        S[(k0 + i) + (size_t)c * nrow] = v * rinv[j];
-      } else {
-        S[c + (size_t)c * nrow] = 1.f;
-        Dd[c] = v;
-        De[c] = 0.f;
-      }
+  // the block itself, which every CTA has, dealt to all of them (they all read
+  // it before the exchange)
+  for (int e = blockIdx.x * FB_THREADS + tid; e < kept * nbR; e += gridDim.x * FB_THREADS) {
+    const int j = e / nbR, i = e % nbR;
+    if (i < j) continue;
+    const float v = Rc[j * FB_LD + i];
+    const int c = k0 + j;
+    if (wb_out) Wb[(size_t)j * ldw + k0 + i] = v;
+    if (i > j) {
+      S[(k0 + i) + (size_t)c * nrow] = v * rinv[j];
+    } else {
+      S[c + (size_t)c * nrow] = 1.f;
+      Dd[c] = v;
+      De[c] = 0.f;
     }
-    if (tid == 0) {
-      ctl->kb = kept;
-      ctl->stop = kept < nbR ? 1 : 0;
-      if (slot >= 0) {
-        ctl->kb_log[slot] = kept;
-        if (kept < nbR) ctl->halt = 1;
-      }
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    ctl->kb = kept;
+    ctl->stop = kept < nbR ? 1 : 0;
+    if (slot >= 0) {
+      ctl->kb_log[slot] = kept;
+      if (kept < nbR) ctl->halt = 1;
     }
   }
 }
