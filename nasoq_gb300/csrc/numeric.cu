@@ -460,7 +460,8 @@ __global__ void __launch_bounds__(256) k_bk_global(const int *targets, int n, co
       a[e] = r >= c ? Ls[r + (size_t)c * nrow] : T(0);
     }
     __syncthreads();
-    bk_factor(a, w, w, Dg + c0, Dg + n + c0, perm, status, &piv);
+    const int k0 = bk_blocked(a, w, w, Dg + c0, Dg + n + c0);
+    bk_factor(a, w, w, Dg + c0, Dg + n + c0, perm, status, &piv, k0);
     __syncthreads();
     // strict upper triangle back to 0 (never referenced, kept at 0 like the reference)
     for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
@@ -468,7 +469,8 @@ __global__ void __launch_bounds__(256) k_bk_global(const int *targets, int n, co
       Ls[r + (size_t)c * nrow] = r >= c ? a[e] : T(0);
     }
   } else {
-    bk_factor(Ls, nrow, w, Dg + c0, Dg + n + c0, perm, status, &piv);
+    const int k0 = bk_blocked(Ls, nrow, w, Dg + c0, Dg + n + c0);
+    bk_factor(Ls, nrow, w, Dg + c0, Dg + n + c0, perm, status, &piv, k0);
     // zero the strict upper triangle (never referenced, kept at 0 like the reference)
     for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
       int c = e / w, r = e % w;
