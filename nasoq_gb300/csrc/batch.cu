@@ -2558,11 +2558,20 @@ size_t batch_smem_bytes(const BArgs &a, size_t tsize) {
 
 #endif  // NQG_BATCH_FP64_UNIT
 
-// Raises the kernel's dynamic shared-memory limit to smem_attr (outside any
-// stream capture) and returns how many CTAs of `smem` bytes fit on an SM.
+// Raises the kernel's dynamic shared-memory limit (outside any stream capture) and
+// returns how many CTAs of `smem` bytes fit on an SM.  The limit belongs to the
+// kernel, not to a batch: always the device's largest, so that a batch made later
+// with less shared memory does not take it from an earlier one.
 template <class T> int batch_prepare(int threads, size_t smem_attr, size_t smem, int *blocks_per_sm) {
-  if (cudaFuncSetAttribute(k_nasoq_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_attr) !=
-      cudaSuccess)
+  int dev = 0, most = 0;
+  cudaFuncAttributes fa;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa, k_nasoq_batch<T>) != cudaSuccess)
+    return NQG_ERR_CUDA;
+  most -= (int)fa.sharedSizeBytes;
+  if (smem_attr > (size_t)most ||
+      cudaFuncSetAttribute(k_nasoq_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
     return NQG_ERR_CUDA;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_nasoq_batch<T>, threads, smem) != cudaSuccess)
     return NQG_ERR_CUDA;

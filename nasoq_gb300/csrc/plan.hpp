@@ -72,8 +72,8 @@ struct Plan {
   std::vector<int> pers_ptr;        // per supernode s: range in pers_pair
   std::vector<int> pers_pair;       // pair indices
   std::vector<uint8_t> pair_pers;   // per pair: 1 if it is one of them
-  // target row positions of every pair's rows lb .. nr-1 (formed per factorization
-  // read by the update tiles): offsets per pair
+  // target row positions of every pair's rows lb .. nr-1 (formed once per
+  // factorization, read by the update tiles): offsets per pair
   std::vector<int64_t> pair_moff;
   int64_t map_total = 0;
   int64_t pers_map_ints = 0;        // largest rows + columns of such a pair

@@ -8,7 +8,7 @@
 // (blocked_2by2_solver, src/common/Sym_BLAS.cpp:492-529).  Backward
 // (H2LeveledBlockedLTsolve, Triangular_BCSC.cpp:534-600): per level in
 // reverse, gather x(rows below), x1 -= L21^T x2, then the transposed unit
-// triangle.  Vectors are FP64; factor values are FP64 or FP32 (FP32 values
+// triangle.  Small FP64 plans take solve_small.cu instead.  Vectors are FP64; factor values are FP64 or FP32 (FP32 values
 // are widened before use).
 #include <cuda_runtime.h>
 

@@ -1,9 +1,9 @@
 // The refined solve of a small FP64 plan as one launch: triangular solves, D^-1,
-// residuals and the GMRES loop of gmres_refine (solve.cu), whose
-// level kernels and dot products are hundreds of launches of a few
-// microseconds each on a system of a few thousand columns (a QP's active-set
-// iteration solves one such system per step; 74 tree levels at 576 variables
-// and 284 general rows: 106 level kernels per application, 6 us each).
+// residuals and the GMRES loop of gmres_refine (solve.cu), whose level kernels
+// and dot products are hundreds of launches of a few microseconds each on a
+// system of a few thousand columns (a QP's active-set iteration solves one such
+// system per step; 74 tree levels at 576 variables and 284 general rows: 106
+// level kernels per application, 6 us each).
 //
 // Forward / backward sweeps: reference H2LeveledBlockedLsolve / LTsolve
 // (src/triangularSolve/Triangular_BCSC.cpp:378-446, 534-600); D: 1x1 and 2x2

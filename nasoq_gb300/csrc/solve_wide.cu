@@ -8,7 +8,7 @@
 // is block row q (64 rows of the diagonal block, then 64-row blocks of the rows
 // below); it accumulates L(q, j) x_j over the column blocks j before it, each
 // as soon as block j's ready flag carries this launch's epoch, then solves
-// its 64 x 64 unit-lower diagonal tile in one warp and publishes x_q with a
+// its 64 x 64 unit-lower diagonal tile and publishes x_q with a
 // release store of its flag (rows below scatter L21 x into the ancestors'
 // entries with atomics instead).  Backward: item j is column block j, taken
 // from the last; it gathers L21^T x(rows below) without waiting, then

@@ -13,6 +13,7 @@
 //   k_wide_panel    cooperative launch, G CTAs, rows grid-strided; one grid
 //                   barrier per column when no interchange is needed, three
 //                   when one is.  W holds the updated panel columns (= L D).
+//   k_panel64       FP64 panels whose columns need no pivot search: no exchange.
 //   k_wide_trailing A22 -= L21 W21^T over the remaining columns (lower
 //                   trapezoid incl. all rows below the block), 2-D tiles.
 // Every spin-wait is bounded: on timeout the kernel records ST_TIMEOUT and
