@@ -903,7 +903,7 @@ __global__ void __launch_bounds__(FB_THREADS) k_wide_panel_blk(float *S, int nro
 // the CTA's rows.  W goes to Wb and the column maxima to colkey, nothing to S:
 // k_panel64_finish keeps the columns before the first that needs a pivot search.
 // Entries take the same multiply-adds in the same order as in k_wide_panel.
-// The 26 panels of a 1135-column front: 78 us each, 355 us column by column (an
+// The 26 panels of a 1135-column front: 65 us each, 355 us column by column (an
 // exchange of about 2500 cycles and 32 dependent multiply-adds per column).
 constexpr int P64_THREADS = 256, P64_ROWS = 32, P64_RB = 8, P64_LD = WP_NB;
 constexpr size_t P64_SMEM =
@@ -1043,7 +1043,10 @@ __global__ void __launch_bounds__(P64_THREADS) k_panel64(const double *S, int nr
 }
 
 // L, D of the columns of a block-first panel up to the first whose diagonal fails
-// the Bunch-Kaufman test; kb and stop for the host.
+// the Bunch-Kaufman test; kb and stop for the host.  A CTA has 256 rows of 16
+// columns, all its loads in flight before the first store (one CTA for all
+// columns, each load waiting behind a store: 35 us of the panel's 95).
+constexpr int P64_FIN = 16;
 __global__ void __launch_bounds__(P64_THREADS) k_panel64_finish(double *S, int nrow, int w, int k0, int nb,
                                                                 const double *Wb, int ldw, double *Dd, double *De,
                                                                 WideCtl *ctl) {
@@ -1062,18 +1065,23 @@ __global__ void __launch_bounds__(P64_THREADS) k_panel64_finish(double *S, int n
   __syncthreads();
   const unsigned long long failed = ~((unsigned long long)pass[1] << 32 | pass[0]);
   const int kept = failed ? __ffsll((long long)failed) - 1 : WP_NB;
-  const int r = k0 + blockIdx.x * P64_THREADS + tid;
+  const int r = k0 + blockIdx.x * P64_THREADS + tid, j0 = blockIdx.y * P64_FIN;
+  const double *wr = Wb + min(r, nrow - 1);
+  double v[P64_FIN];
+#pragma unroll
+  for (int q = 0; q < P64_FIN; ++q) v[q] = wr[(size_t)min(j0 + q, nbR - 1) * ldw];
   if (r < nrow) {
     const int below = min(kept, r - k0);  // columns left of the row's diagonal entry
-#pragma unroll 8
-    for (int j = 0; j < below; ++j) S[r + (size_t)(k0 + j) * nrow] = Wb[(size_t)j * ldw + r] * rinv[j];
-    if (r - k0 < kept) {
+#pragma unroll
+    for (int q = 0; q < P64_FIN; ++q)
+      if (j0 + q < below) S[r + (size_t)(k0 + j0 + q) * nrow] = v[q] * rinv[j0 + q];
+    if (blockIdx.y == 0 && r - k0 < kept) {
       S[r + (size_t)r * nrow] = 1.0;
       Dd[r] = Wb[(size_t)(r - k0) * ldw + r];
       De[r] = 0.0;
     }
   }
-  if (blockIdx.x == 0 && tid == 0) {
+  if (blockIdx.x + blockIdx.y == 0 && tid == 0) {
     ctl->kb = kept;
     ctl->stop = kept < nbR ? 1 : 0;
   }
@@ -2286,8 +2294,8 @@ static int run_wide(T *S, int nrow, int w, T *Dd, T *De, int *perm, T *Wb, WideC
         const int below = nrow - k0 - kb_want;
         k_panel64<<<std::max(1, (below + P64_ROWS - 1) / P64_ROWS), P64_THREADS, P64_SMEM, st>>>(
             S, nrow, w, k0, kb_want, Wp, ldw, &ctl->colkey[0]);
-        k_panel64_finish<<<(nrow - k0 + P64_THREADS - 1) / P64_THREADS, P64_THREADS, 0, st>>>(S, nrow, w, k0, kb_want,
-                                                                                           Wp, ldw, Dd, De, ctl);
+        k_panel64_finish<<<dim3((nrow - k0 + P64_THREADS - 1) / P64_THREADS, WP_NB / P64_FIN), P64_THREADS, 0, st>>>(
+            S, nrow, w, k0, kb_want, Wp, ldw, Dd, De, ctl);
         if (cudaGetLastError() != cudaSuccess) return NQG_ERR_CUDA;
         if (P) {
           P->nlaunch += 2;
