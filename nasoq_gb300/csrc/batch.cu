@@ -265,18 +265,22 @@ __device__ void block_select(double &v, int &idx, bool sel_max, double *red, int
 // diagonals as the regularization (find_perturbation,
 // linear_solver_wrapper.cpp:352-363).
 //
-// An FP32 factor also gets a sign-keeping floor reg32 on its diagonal: pivots
-// as small as the 1e-9 regularization create element growth of ~1e9 under
-// Bunch-Kaufman restricted to supernode diagonal blocks, beyond what FP32
-// carries; the factor is only the preconditioner of the FP64 refinement,
-// whose matrix keeps the reference's values.
+// An FP32 factor also gets a floor reg32 on its diagonal: pivots as small as
+// the 1e-9 regularization create element growth of ~1e9 under Bunch-Kaufman
+// restricted to supernode diagonal blocks, beyond what FP32 carries; the
+// factor is only the preconditioner of the FP64 refinement, whose matrix keeps
+// the reference's values.  The floor is negative on the constraints' rows: the
+// Schur complement there is -A H^-1 A^T, which a positive one makes singular
+// wherever an eigenvalue of A H^-1 A^T comes near it, and the refinement then
+// ran out of steps (1 in 8000 uneven MPC problems ended up to 1e-1 off, which
+// ones depending on rounding; with the negative floor none of 121856).
 template <class T> __device__ __forceinline__ double fact_val(const Ctx<T> &c, int vq) {
   const int e = c.ent[vq];
   double v = c.kv[vq];
   if (e >= 0) return c.act[e] ? v : 0.0;
   if (e <= -2) {
     if (c.pert[-2 - e]) v = c.reg;
-    if (sizeof(T) == 4 && fabs(v) < c.reg32) v = v < 0.0 ? -c.reg32 : c.reg32;
+    if (sizeof(T) == 4 && fabs(v) < c.reg32) v = v < 0.0 || -2 - e >= c.n ? -c.reg32 : c.reg32;
   }
   return v;
 }

@@ -88,7 +88,7 @@ struct BProb {
   int64_t o_x, o_y, o_z;     // n, meq, mineq (results; warm start in)
   int64_t o_as;              // mineq ints: final active set (insertion order); warm-start set in
   double reg, zero_thresh, eps_abs, tol_abs, tol_rel;
-  double reg32;              // FP32 factor: sign-keeping floor of its diagonal (3e-5 max |k_ij|)
+  double reg32;              // FP32 factor: floor of its diagonal (3e-5 max |k_ij|), negative on the constraints' rows
 };
 
 // Results of one QP (reference Nasoq fields of the same names).
