@@ -16,14 +16,18 @@ constexpr int BK_SMALL_ROWS = 64;  // rows below that their kernel stages at a t
 
 __device__ __forceinline__ void flag_status(int *st, int bits) { atomicOr(st, bits); }
 
-template <class T> __device__ __forceinline__ T tabs(T v) { return v < T(0) ? -v : v; }
+// Magnitude, the sign bit cleared also for -0 and NaN: the searches below order
+// its bits.
+[[maybe_unused]] __device__ __forceinline__ float tabs(float v) { return fabsf(v); }
+[[maybe_unused]] __device__ __forceinline__ double tabs(double v) { return fabs(v); }
 
 // Warp-wide argmax of |value| with the smallest index winning ties (the
 // LAPACK idamax convention) over the lanes that have one (idx >= 0); every
-// lane returns the winner.  The bits of a non-negative
-// floating-point number order like an integer: two integer reductions and a
-// vote instead of a tree of compares (an FP64 compare holds the FP64 pipe of
-// the SM quarter for 64 cycles).
+// lane returns the winner.  The bits of a floating-point number with a clear
+// sign (v comes from tabs; with its sign bit -0.0 would beat every value) order
+// like an integer: two integer reductions and a vote instead of a tree of
+// compares (an FP64 compare holds the FP64 pipe of the SM quarter for 64
+// cycles).
 [[maybe_unused]] __device__ __forceinline__ void warp_argmax(float &v, int &idx) {
   const unsigned FULL = 0xffffffffu;
   const unsigned key = idx >= 0 ? __float_as_uint(v) + 1u : 0u;
