@@ -69,6 +69,22 @@ template <class T> struct Sh {
   __device__ __forceinline__ Sh at(int n) const { return {off + (unsigned)(n * (int)sizeof(T))}; }
 };
 
+// Patterns of more columns than shared memory has room for with both vectors
+// of the solves keep the second one, the refactorization marks and the levels'
+// items in global memory: a kernel of its own (batch_large.cu), since a pointer
+// that may be either costs a generic access everywhere.  FP64 from 11900
+// columns on (horizon 360 of the MPC families), to 15800; FP32 from 22000 to
+// 23400.  64 problems of horizon 400 (FP64) 87.7 ms, of horizon 700 (FP32) 219.5
+// (the kernel with one vector for the solves, which still held them: 332.7 and
+// 973.5); horizon 300, both vectors shared, 55.6.
+#ifdef NQG_BATCH_LARGE_UNIT
+constexpr bool LARGE = true;
+template <class T> using Spill = T *;
+#else
+constexpr bool LARGE = false;
+template <class T> using Spill = Sh<T>;
+#endif
+
 // The problem that the CTA works on, at the start of its dynamic shared memory.
 template <class T> struct Ctx {
   // pattern (read-only)
@@ -110,7 +126,8 @@ template <class T> struct Ctx {
   T *Z;
   // shared memory
   Sh<int> map;
-  Sh<T> xs, xo;  // vectors of the solves, in the factor's order (xo shares the row map's memory)
+  Sh<T> xs;      // vectors of the solves, in the factor's order (xo shares the row map's memory where it is shared)
+  Spill<T> xo;
   Sh<T> B, rowbuf, Dsm, Esm, Binv;
   Sh<int> lp;
   // per-warp scratch of the level-parallel factorization (WF_WARPS warps,
@@ -123,8 +140,8 @@ template <class T> struct Ctx {
   Sh<uint8_t> vis;  // per supernode: visible (structural, or the column of an active constraint)
   Sh<uint8_t> act;  // per constraint: active
   Sh<int> vseg;     // starts of each level's two groups in vrec (2 nlev + 1), then the length of arow
-  Sh<int4> lvl;     // per level (3): the pattern's items of the solves (see BPat)
-  Sh<uint8_t> mark;  // per supernode: to be refactored
+  Spill<int4> lvl;     // per level (3): the pattern's items of the solves (see BPat)
+  Spill<uint8_t> mark;  // per supernode: to be refactored
   int nmark;    // > 0: edits wait for a refactorization; during one, the length of mlist
   double red[32];
   int redi[32];
@@ -1788,8 +1805,9 @@ template <class T> __device__ __noinline__ void load_state(Ctx<T> &) {
 
 }  // namespace
 
-template <class T>
+template <class T, bool LARGE_PATTERNS>
 __global__ void __launch_bounds__(BT_MAX_THREADS, 2) k_nasoq_batch(BArgs a) {
+  static_assert(LARGE_PATTERNS == LARGE, "one of the two per translation unit");
   __shared__ int s_prob;
   __shared__ int s_int[8];
   __shared__ double s_dbl[8];
@@ -1805,14 +1823,15 @@ __global__ void __launch_bounds__(BT_MAX_THREADS, 2) k_nasoq_batch(BArgs a) {
     sp += (unsigned)((bytes + 15) / 16 * 16);
     return o;
   };
-  const unsigned o_map = take((size_t)a.N_max * sizeof(T));  // the row map of a factorization, xo of the solves
+  // the row map of a factorization, and xo of the solves
+  const unsigned o_map = take((size_t)a.N_max * (LARGE ? sizeof(int) : sizeof(T)));
   const unsigned o_xs = take((size_t)a.N_max * sizeof(T));
   const unsigned o_rowbuf = take(batch_rowbuf(a) * sizeof(T));
   const unsigned o_D = take((size_t)a.w_max * sizeof(T)), o_E = take((size_t)a.w_max * sizeof(T));
   const unsigned o_lp = take((size_t)a.w_max * sizeof(int));
-  const unsigned o_lvl = take((size_t)3 * a.nlev_max * sizeof(int4));
+  const unsigned o_lvl = take(LARGE ? 0 : (size_t)3 * a.nlev_max * sizeof(int4));
   const unsigned o_vseg = take((size_t)(2 * a.nlev_max + 2) * sizeof(int));
-  const unsigned o_vis = take((size_t)a.ns_max), o_mark = take((size_t)a.ns_max), o_act = take((size_t)a.mi_max);
+  const unsigned o_vis = take((size_t)a.ns_max), o_mark = take(LARGE ? 0 : (size_t)a.ns_max), o_act = take((size_t)a.mi_max);
   // blocks of the factorization: the CTA's, or one set per warp in the same memory
   const int wcap = a.warp_factor ? min(a.w_max, 32) : 0, rcap = a.warp_factor ? min(a.nr_max, 32) : 0;
   const int wstride = wcap * (rcap + wcap + 4);
@@ -1908,8 +1927,15 @@ __global__ void __launch_bounds__(BT_MAX_THREADS, 2) k_nasoq_batch(BArgs a) {
       c.perm = reinterpret_cast<int *>(slot + a.slot.o_perm);
       c.iperm = reinterpret_cast<int *>(slot + a.slot.o_iperm);
       c.lperm = reinterpret_cast<int *>(slot + a.slot.o_lperm);
+#ifdef NQG_BATCH_LARGE_UNIT
+      c.mark = slot + a.slot.o_mark;
+      c.lvl = reinterpret_cast<int4 *>(slot + a.slot.o_lvl);
+      c.xo = reinterpret_cast<T *>(slot + a.slot.o_xo);
+#else
       c.mark.off = o_mark;
       c.lvl.off = o_lvl;
+      c.xo.off = o_map;
+#endif
       c.piv = slot + a.slot.o_piv;
       c.alist = reinterpret_cast<int *>(slot + a.slot.o_alist);
       c.vrec = reinterpret_cast<int4 *>(slot + a.slot.o_vrec);
@@ -1927,7 +1953,6 @@ __global__ void __launch_bounds__(BT_MAX_THREADS, 2) k_nasoq_batch(BArgs a) {
       c.tmp = reinterpret_cast<double *>(slot + a.slot.o_tmp);
       c.map.off = o_map;
       c.xs.off = o_xs;
-      c.xo.off = o_map;
       c.B.off = o_B;
       c.rowbuf.off = o_rowbuf;
       c.Dsm.off = o_D;
@@ -2453,10 +2478,11 @@ __global__ void __launch_bounds__(BT_MAX_THREADS, 2) k_nasoq_batch(BArgs a) {
   if (a.prof && tid < PH_N) atomicAdd(a.prof + tid, c.cyc[tid]);
 }
 
-// batch_fp64.cu compiles this file again with NQG_BATCH_FP64_UNIT defined for
-// the FP64 instantiation alone (the two instantiations then build in
-// parallel); the non-template kernels and host functions belong to this unit.
-#ifndef NQG_BATCH_FP64_UNIT
+// batch_fp64.cu and batch_large.cu compile this file again with
+// NQG_BATCH_FP64_UNIT / NQG_BATCH_LARGE_UNIT defined for their instantiations
+// alone (they then build in parallel); the non-template kernels and host
+// functions belong to this unit.
+#if !defined(NQG_BATCH_FP64_UNIT) && !defined(NQG_BATCH_LARGE_UNIT)
 
 // Warm-start sets from per-constraint scores (e.g. the logits of the active-set
 // model): problem i proposes every constraint k with scores[i * ld + k] >
@@ -2555,44 +2581,50 @@ int batch_ws_clear(int nprob, BProb *probs, cudaStream_t st) {
 
 size_t batch_smem_bytes(const BArgs &a, size_t tsize) {
   auto up = [](size_t b) { return (b + 15) / 16 * 16; };
-  return BATCH_CTX_BYTES + 2 * up((size_t)a.N_max * tsize) + up(batch_rowbuf(a) * tsize) + 2 * up((size_t)a.w_max * tsize) +
-         up((size_t)a.w_max * sizeof(int)) + (size_t)a.nlev_max * 48 + up((size_t)(2 * a.nlev_max + 2) * sizeof(int)) +
-         2 * up((size_t)a.ns_max) + up((size_t)a.mi_max) + batch_block_bytes(a, tsize) + (size_t)a.stage_bytes;
+  return BATCH_CTX_BYTES + up((size_t)a.N_max * tsize) + up((size_t)a.N_max * (a.large ? sizeof(int) : tsize)) +
+         up(batch_rowbuf(a) * tsize) + 2 * up((size_t)a.w_max * tsize) + up((size_t)a.w_max * sizeof(int)) +
+         (a.large ? 0 : (size_t)a.nlev_max * 48 + up((size_t)a.ns_max)) + up((size_t)(2 * a.nlev_max + 2) * sizeof(int)) +
+         up((size_t)a.ns_max) + up((size_t)a.mi_max) + batch_block_bytes(a, tsize) + (size_t)a.stage_bytes;
 }
 
-#endif  // NQG_BATCH_FP64_UNIT
+#endif
 
 // Raises the kernel's dynamic shared-memory limit (outside any stream capture) and
 // returns how many CTAs of `smem` bytes fit on an SM.  The limit belongs to the
 // kernel, not to a batch: always the device's largest, so that a batch made later
 // with less shared memory does not take it from an earlier one.
-template <class T> int batch_prepare(int threads, size_t smem_attr, size_t smem, int *blocks_per_sm) {
+template <class T, bool LARGE_PATTERNS>
+int batch_prepare(int threads, size_t smem_attr, size_t smem, int *blocks_per_sm) {
+  const auto kernel = k_nasoq_batch<T, LARGE_PATTERNS>;
   int dev = 0, most = 0;
   cudaFuncAttributes fa;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa, k_nasoq_batch<T>) != cudaSuccess)
+      cudaFuncGetAttributes(&fa, kernel) != cudaSuccess)
     return NQG_ERR_CUDA;
   most -= (int)fa.sharedSizeBytes;
   if (smem_attr > (size_t)most ||
-      cudaFuncSetAttribute(k_nasoq_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
     return NQG_ERR_CUDA;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_nasoq_batch<T>, threads, smem) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kernel, threads, smem) != cudaSuccess)
     return NQG_ERR_CUDA;
   return NQG_OK;
 }
 
-template <class T> int launch_batch(const BArgs &a, int grid, int threads, size_t smem, cudaStream_t st) {
-  k_nasoq_batch<T><<<grid, threads, smem, st>>>(a);
+template <class T, bool LARGE_PATTERNS>
+int launch_batch(const BArgs &a, int grid, int threads, size_t smem, cudaStream_t st) {
+  k_nasoq_batch<T, LARGE_PATTERNS><<<grid, threads, smem, st>>>(a);
   return cudaGetLastError() == cudaSuccess ? NQG_OK : NQG_ERR_CUDA;
 }
 
-#ifdef NQG_BATCH_FP64_UNIT
-template int launch_batch<double>(const BArgs &, int, int, size_t, cudaStream_t);
-template int batch_prepare<double>(int, size_t, size_t, int *);
-#else
-template int launch_batch<float>(const BArgs &, int, int, size_t, cudaStream_t);
-template int batch_prepare<float>(int, size_t, size_t, int *);
+#define NQG_BATCH_INSTANCE(T)                                                           \
+  template int launch_batch<T, LARGE>(const BArgs &, int, int, size_t, cudaStream_t); \
+  template int batch_prepare<T, LARGE>(int, size_t, size_t, int *);
+#if defined(NQG_BATCH_FP64_UNIT) || defined(NQG_BATCH_LARGE_UNIT)
+NQG_BATCH_INSTANCE(double)
+#endif
+#if !defined(NQG_BATCH_FP64_UNIT)
+NQG_BATCH_INSTANCE(float)
 #endif
 
 }  // namespace nqg

@@ -103,6 +103,7 @@ struct BResult {
 // Per-CTA scratch: one problem at a time, sized for the largest pattern.
 struct BSlot {
   int64_t o_L, o_S, o_G, o_D, o_ls, o_perm, o_iperm, o_lperm, o_piv, o_alist, o_vrec, o_arow, o_mlist;
+  int64_t o_mark, o_lvl, o_xo;  // large patterns (BArgs::large)
   int64_t o_Fv, o_Rv;  // factorization / refinement values of K in CSR order (inactive rows zeroed)
   int64_t o_cmask;     // per supernode: bit mask of its active constraint-column descendants
   int64_t o_rhs, o_sol, o_r, o_w, o_V, o_Z, o_tmp;
@@ -129,6 +130,7 @@ struct BArgs {
   unsigned long long *prof;  // per-phase SM cycles summed over CTAs, or null
   int stage_bytes;           // shared memory for the factor and row lists of problems that fit
   int warp_factor;           // level-parallel factorization, a warp per supernode of <= 32 x 32
+  int large;                 // the second vector of the solves, marks and levels in the slot, not in shared memory
   // Problems with identical matrix values (same pattern, values,
   // regularization) share the factorization with every inequality hidden: a
   // launch with mode = 1 computes it once per group into `bases` (one slot
@@ -162,7 +164,10 @@ int batch_ws_clear(int nprob, BProb *probs, cudaStream_t st);
 // given) from a staging buffer into the value pool.
 int batch_scatter_vectors(int nprob, const BProb *probs, const BPat *pats, const int64_t *voff, const double *stage,
                           double *dpool, cudaStream_t st);
-template <class T> int batch_prepare(int threads, size_t smem_attr, size_t smem, int *blocks_per_sm);
-template <class T> int launch_batch(const BArgs &a, int grid, int threads, size_t smem, cudaStream_t st);
+// LARGE_PATTERNS: as BArgs::large
+template <class T, bool LARGE_PATTERNS>
+int batch_prepare(int threads, size_t smem_attr, size_t smem, int *blocks_per_sm);
+template <class T, bool LARGE_PATTERNS>
+int launch_batch(const BArgs &a, int grid, int threads, size_t smem, cudaStream_t st);
 
 }  // namespace nqg

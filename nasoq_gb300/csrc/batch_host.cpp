@@ -580,6 +580,20 @@ void fill_values(nqg_batch *b, int i, std::vector<unsigned char> &pert_pool) {
   P.reg32 = 3e-5 * (amax > 0 ? amax : 1.0);
 }
 
+// The batch's kernel: by precision, and by where its vectors fit.
+int launch_kernel(const nqg_batch *b, const nqg::BArgs &a, int grid, size_t smem, cudaStream_t st) {
+  const auto launch = b->set.qp.precision == NQG_FP32
+                          ? (a.large ? nqg::launch_batch<float, true> : nqg::launch_batch<float, false>)
+                          : (a.large ? nqg::launch_batch<double, true> : nqg::launch_batch<double, false>);
+  return launch(a, grid, b->threads, smem, st);
+}
+int prepare_kernel(const nqg_batch *b, const nqg::BArgs &a, size_t smem_attr, size_t smem, int *bps) {
+  const auto prepare = b->set.qp.precision == NQG_FP32
+                           ? (a.large ? nqg::batch_prepare<float, true> : nqg::batch_prepare<float, false>)
+                           : (a.large ? nqg::batch_prepare<double, true> : nqg::batch_prepare<double, false>);
+  return prepare(b->threads, smem_attr, smem, bps);
+}
+
 // Queue resets and one persistent launch per tier, forked from the batch's
 // stream and joined back into it.
 int launch(nqg_batch *b) {
@@ -589,9 +603,7 @@ int launch(nqg_batch *b) {
     if (cudaStreamWaitEvent(L.stream, b->efork, 0) != cudaSuccess) return NQG_ERR_CUDA;
     if (cudaMemsetAsync(L.args.head, 0, sizeof(int), L.stream) != cudaSuccess) return NQG_ERR_CUDA;
     L.args.prof = b->args.prof;
-    const int rc = b->set.qp.precision == NQG_FP32
-                       ? nqg::launch_batch<float>(L.args, L.grid, b->threads, L.smem, L.stream)
-                       : nqg::launch_batch<double>(L.args, L.grid, b->threads, L.smem, L.stream);
+    const int rc = launch_kernel(b, L.args, L.grid, L.smem, L.stream);
     if (rc) return rc;
     if (cudaEventRecord(L.done, L.stream) != cudaSuccess) return NQG_ERR_CUDA;
     if (cudaStreamWaitEvent(b->stream, L.done, 0) != cudaSuccess) return NQG_ERR_CUDA;
@@ -918,7 +930,22 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
   base_args.mi_max = mi_max;
   base_args.nlev_max = nlev_max;
   base_args.stage_bytes = 0;
-  const size_t static_smem = 8 * 1024;  // the kernel's own __shared__ variables, rounded up
+  size_t static_smem = 8 * 1024;  // the kernel's own __shared__ variables, rounded up
+  // Patterns of too many columns keep part of the state in the slot (the
+  // context, 3 KB, was a __shared__ variable in what that limit allows for);
+  // NASOQ_GB300_BATCH_LARGE=1 asks for it.
+  {
+    const char *e = std::getenv("NASOQ_GB300_BATCH_LARGE");
+    base_args.large = (e && std::string(e) == "1") ||
+                      (int64_t)nqg::batch_smem_bytes(base_args, ts) + (int64_t)static_smem > smem_optin;
+    if (base_args.large) {
+      static_smem -= nqg::BATCH_CTX_BYTES + 1024;
+      sl.o_mark = seg(ns_max);
+      sl.o_lvl = seg((int64_t)nlev_max * 48);
+      sl.o_xo = seg((int64_t)N_max * ts);
+      sl.bytes = off;
+    }
+  }
   // Level-parallel factorization (a warp per supernode of at most 32 x 32)
   // for FP32 factors where its per-warp scratch keeps as many CTAs per SM as
   // the layout without it (FP64 factors measured faster on the CTA path);
@@ -932,10 +959,7 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
       nqg::BArgs with = base_args;
       with.warp_factor = 1;
       const size_t s0 = nqg::batch_smem_bytes(base_args, ts), s1 = nqg::batch_smem_bytes(with, ts);
-      auto occ = [&](size_t sm, int *bps) {
-        return b->set.qp.precision == NQG_FP32 ? nqg::batch_prepare<float>(b->threads, sm, sm, bps)
-                                               : nqg::batch_prepare<double>(b->threads, sm, sm, bps);
-      };
+      auto occ = [&](size_t sm, int *bps) { return prepare_kernel(b, base_args, sm, sm, bps); };
       int b0 = 0, b1 = 0;
       if ((int64_t)s1 + (int64_t)static_smem <= smem_optin && occ(s0, &b0) == NQG_OK && occ(s1, &b1) == NQG_OK &&
           b1 > 0 && b1 >= b0)
@@ -952,7 +976,7 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
     need[i] = ((int64_t)P.lsize * (int64_t)ts + 15) / 16 * 16 + (int64_t)P.sbsize * (int64_t)ts + (int64_t)P.rsize * 4;
   }
   std::vector<int64_t> budgets;
-  if (b->set.stage) {
+  if (b->set.stage && stage_max > 0) {
     for (int64_t kb : {16, 32, 48, 64, 96, 128, 160, 192, 224})
       if (kb * 1024 <= stage_max) budgets.push_back(kb * 1024);
     if (budgets.empty() || budgets.back() < stage_max) budgets.push_back(stage_max / 16 * 16);
@@ -992,8 +1016,7 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
   int64_t nslots = 0;
   for (auto &L : b->tiers) {
     int bps = 0;
-    int rc = b->set.qp.precision == NQG_FP32 ? nqg::batch_prepare<float>(b->threads, smem_top, L.smem, &bps)
-                                            : nqg::batch_prepare<double>(b->threads, smem_top, L.smem, &bps);
+    int rc = prepare_kernel(b, L.args, smem_top, L.smem, &bps);
     if (rc || bps <= 0) return fail(b, NQG_ERR_CUDA, "no resident CTA fits the batched kernel");
     L.bps = bps;
     L.grid = std::min(L.nprob, bps * b->num_sms);
@@ -1068,8 +1091,7 @@ extern "C" int nqg_batch_finalize(nqg_batch *b) {
     BQ_CUDA(cudaMemsetAsync(A.head, 0, sizeof(int), b->stream));
     const int grid = std::min(b->nbase, T0.bps * b->num_sms);
     const size_t smem = base_smem;
-    const int rc = b->set.qp.precision == NQG_FP32 ? nqg::launch_batch<float>(A, grid, b->threads, smem, b->stream)
-                                                   : nqg::launch_batch<double>(A, grid, b->threads, smem, b->stream);
+    const int rc = launch_kernel(b, A, grid, smem, b->stream);
     if (rc) return fail(b, rc, "launch of the shared factorizations failed");
     BQ_CUDA(cudaStreamSynchronize(b->stream));
   }
