@@ -508,11 +508,20 @@ Operand weights(const __nv_bfloat16 *p, int rows, int K) { return {nullptr, p, r
 // tile splits the same rows of A again).
 int tile_columns(int M, int N) { return (long)((M + MT - 1) / MT) * ((N + 63) / 64) > SM_COUNT && N > 64 ? 128 : 64; }
 
+// Shared-memory limits of the kernels below, for the device that a model is
+// made on (they belong to a device, not to the process).
+template <int NB, int NT> cudaError_t allow_smem() {
+  return cudaFuncSetAttribute(k_mlp_tc<NB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem(NB, NT));
+}
+cudaError_t allow_smem_all() {
+  for (cudaError_t e : {allow_smem<1, 64>(), allow_smem<1, 128>(), allow_smem<3, 64>()})
+    if (e != cudaSuccess) return e;
+  return cudaSuccess;
+}
+
 template <int NB, int NT>
 void launch_tc(nqg_mlp *m, int M, int N, int K, const Operand &A, const Operand &B, float *C, int ldc, int epi,
                const float *bias, const float *mask, int parts) {
-  static const cudaError_t attr = cudaFuncSetAttribute(k_mlp_tc<NB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem(NB, NT));
-  (void)attr;  // a failure shows as the launch's error
   const dim3 grid((N + NT - 1) / NT, (M + MT - 1) / MT, parts);
   k_mlp_tc<NB, NT><<<grid, TC_THREADS, tc_smem(NB, NT), m->stream>>>(M, N, K, A, B, C, ldc, (size_t)M * N, epi, bias, mask,
                                                                      m->timeout);
@@ -577,6 +586,7 @@ extern "C" int nqg_mlp_create(int nsizes, const int *sizes, unsigned long long s
   if (!out || nsizes < 2 || !sizes) return NQG_ERR_ARG;
   for (int l = 0; l < nsizes; ++l)
     if (sizes[l] <= 0) return NQG_ERR_ARG;
+  if (allow_smem_all() != cudaSuccess) return NQG_ERR_CUDA;
   auto *m = new nqg_mlp;
   m->sizes.assign(sizes, sizes + nsizes);
   m->L = nsizes - 1;
