@@ -85,7 +85,8 @@ __device__ __forceinline__ void split8(const float *x, uint4 (&part)[3]) {
     for (int e = 0; e < 2; ++e) {
       const float v = x[2 * q + e];
       const uint32_t b = __float_as_uint(v);
-      h[e] = b & 0xffff0000u;
+      // a NaN may have its payload in the low bits alone, which would leave an infinity
+      h[e] = (b & 0x7fffffffu) > 0x7f800000u ? 0x7fff0000u : b & 0xffff0000u;
       const float r = (b & 0x7f800000u) == 0x7f800000u ? 0.f : v - __uint_as_float(h[e]);  // exact; infinities and NaN stay in h
       m[e] = __float_as_uint(r) & 0xffff0000u;
       l[e] = __float_as_uint(r - __uint_as_float(m[e]));
