@@ -147,6 +147,23 @@ __device__ __forceinline__ void load_unit(const Operand &o, int r, int k0, int K
 __host__ __device__ constexpr int tc_stage(int nb, int nt) { return 3 * A_PART + nb * nt * 128; }
 __host__ __device__ constexpr int tc_smem(int nb, int nt) { return 2 * tc_stage(nb, nt) + 1024 + 64; }
 
+// Entry (r, k) of an FP32 operand.
+__device__ __forceinline__ float value(const Operand &o, int r, int k) {
+  return o.across ? o.p[r + (size_t)k * o.ld] : o.p[(size_t)r * o.ld + k];
+}
+// Entry (m, n) of part z of nz of a product of two FP32 operands, by FP32
+// multiply-adds.  A result that is not a number is formed again by it: an
+// infinity times a part of the other value that happens to be zero is no
+// product of the values.
+__device__ __noinline__ float plain_entry(const Operand &A, const Operand &B, int m, int n, int K, int z, int nz) {
+  float s = 0.f;
+#pragma unroll 1
+  for (int k0 = z * KT; k0 < K; k0 += nz * KT)
+#pragma unroll 4
+    for (int k = k0; k < min(k0 + KT, K); ++k) s = fmaf(value(A, m, k), value(B, n, k), s);
+  return s;
+}
+
 // NB: BF16 parts of B (1: BF16 operand, 3: FP32 one).
 template <int NB, int NT>
 __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(int M, int N, int K, Operand A, Operand B, float *C, int ldc, size_t part,
@@ -327,6 +344,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(int M, int N, int K, Oper
         const int n = n0 + h + lane;
         if (n >= N) continue;
         float v = out[r * LDO + h + lane];
+        if (NB == 3 && v != v) v = plain_entry(A, B, m, n, K, blockIdx.z, gridDim.z);
         if (epi == EPI_BIAS_RELU) v = fmaxf(v + bias[n], 0.f);
         else if (epi == EPI_BIAS) v = v + bias[n];
         else if (epi == EPI_RELU_MASK) v = mask[(size_t)m * ldc + n] > 0.f ? v : 0.f;

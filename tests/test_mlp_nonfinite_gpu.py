@@ -23,3 +23,36 @@ def test_nan_of_any_payload_stays(bits):
     _, gw, _ = m.loss_grad(x, np.zeros((3, 70), np.float32))
     assert np.isnan(gw).all()  # the row's logits, and with them its share of every gradient
     m.close()
+
+
+@pytest.mark.parametrize("rows", [4, 300])
+def test_infinite_input_in_gradients(rows):
+    """dL/dW of a single layer is a sum over rows of d x, an FP32 sum in which
+    an infinite x gives an infinity for d != 0 and NaN for d = 0, also where d
+    has few bits (labels and saturated outputs give d = +-1 / rows)."""
+    sizes = (33, 66)
+    rng = np.random.default_rng(rows)
+    m = nq.MLP(sizes, seed=1)
+    m.set_weights(np.where(rng.random(33 * 66) < 0.5, 1.0, -1.0).astype(np.float32), np.zeros(66, np.float32))
+    x = rng.standard_normal((rows, 33)).astype(np.float32)
+    x[1, 7], x[2, 9] = np.inf, -np.inf
+    y = (rng.random((rows, 66)) < 0.5).astype(np.float32)
+    w = m.get_weights()[0].reshape(66, 33).astype(np.float64)
+    z = np.zeros((rows, 66))
+    for k in range(33):
+        z += x[:, k, None].astype(np.float64) * w[None, :, k]
+    assert (m.forward(x)[1:3] == z[1:3]).all()  # +-inf
+    with np.errstate(over="ignore", invalid="ignore"):
+        s = 1.0 / (1.0 + np.exp(-z))
+        d = (s * (2.0 * y + 1.0 - y) - 2.0 * y) / rows
+        want = np.zeros((66, 33))
+        for r in range(rows):
+            want += d[r][:, None] * x[r].astype(np.float64)[None, :]
+    _, gw, gb = m.loss_grad(x, y, pos_weight=2.0)
+    gw = gw.reshape(66, 33)
+    odd = ~np.isfinite(want)
+    assert odd[:, [7, 9]].any() and np.isinf(want).any()
+    assert np.array_equal(gw[odd], want[odd].astype(np.float32), equal_nan=True)
+    # sums of `rows` FP32 terms
+    assert np.abs(gw[~odd] - want[~odd]).max() <= 2.0 ** -23 * (rows + 33) * np.linalg.norm(want[~odd])
+    m.close()
