@@ -389,8 +389,16 @@ int nqg_mlp_get_weights(nqg_mlp *m, float *w_all, float *b_all);
 int nqg_mlp_forward(nqg_mlp *m, int rows, const float *x, float *logits);
 /* Device buffers, enqueued on `stream` (NULL: the model's own stream, and the
  * call waits).  The model's activation buffers serve every call: forwards of
- * one model on different streams must not overlap (use one model per stream). */
+ * one model on different streams must not overlap (use one model per stream).
+ * A tensor-core wait that gives up (NQG_ERR_TIMEOUT) is reported by the call
+ * itself where it waits, else by nqg_mlp_stream_status, to be asked once the
+ * caller has synchronised its stream; the logits are then not valid. */
 int nqg_mlp_forward_device(nqg_mlp *m, int rows, const float *d_x, float *d_logits, void *stream);
+/* NQG_ERR_TIMEOUT if a forward on a caller's stream gave up since the last call, else NQG_OK. */
+int nqg_mlp_stream_status(nqg_mlp *m);
+/* Polls before a tensor-core wait gives up (0: the default, which is the most;
+ * negative: at once). */
+int nqg_mlp_set_wait_limit(nqg_mlp *m, long long polls);
 int nqg_mlp_loss_grad(nqg_mlp *m, int rows, const float *x, const float *y, float pos_weight, double *loss,
                       float *gw_all, float *gb_all);
 int nqg_mlp_set_data(nqg_mlp *m, int n, const float *x, const float *y);

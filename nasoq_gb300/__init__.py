@@ -167,6 +167,8 @@ def lib():
     L.nqg_mlp_get_weights.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
     L.nqg_mlp_forward.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
     L.nqg_mlp_forward_device.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]
+    L.nqg_mlp_stream_status.argtypes = [C.c_void_p]
+    L.nqg_mlp_set_wait_limit.argtypes = [C.c_void_p, C.c_longlong]
     L.nqg_mlp_loss_grad.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_float,
                                     C.POINTER(C.c_double), C.c_void_p, C.c_void_p]
     L.nqg_mlp_set_data.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
@@ -665,6 +667,15 @@ class MLP:
     def forward_device(self, rows, d_x, d_logits, stream=None):
         self._raise(lib().nqg_mlp_forward_device(self._h, int(rows), C.c_void_p(d_x), C.c_void_p(d_logits),
                                                  C.c_void_p(stream) if stream else None), "forward")
+
+    def check_stream(self):
+        """Raises if a forward on a caller's stream, since synchronised, gave
+        up waiting (its logits are not valid)."""
+        self._raise(lib().nqg_mlp_stream_status(self._h), "forward on a caller's stream")
+
+    def set_wait_limit(self, polls):
+        """Polls before a tensor-core wait gives up (0: the default; negative: at once)."""
+        self._raise(lib().nqg_mlp_set_wait_limit(self._h, int(polls)), "set wait limit")
 
     def loss_grad(self, x, y, pos_weight=1.0):
         x = np.ascontiguousarray(x, np.float32)

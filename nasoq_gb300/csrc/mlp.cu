@@ -70,8 +70,8 @@ struct Operand {
 // wide product takes 128 columns at a time (tile_columns).
 //
 // gridDim.z > 1: part z takes every gridDim.z-th chunk of K and stores to
-// C + z * part (plain store).  `timeout` (host memory) is set if an MMA wait
-// gives up.
+// C + z * part (plain store).  If an MMA wait gives up (after wait_limit polls),
+// the tile's entries are NaN and `timeout` (host memory) is set.
 constexpr int MT = 128, KT = 64;      // rows of a tile, K entries per stage
 constexpr int A_PART = MT * 128;     // bytes of one BF16 part of A in a stage
 
@@ -167,7 +167,8 @@ __device__ __noinline__ float plain_entry(const Operand &A, const Operand &B, in
 // NB: BF16 parts of B (1: BF16 operand, 3: FP32 one).
 template <int NB, int NT>
 __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(int M, int N, int K, Operand A, Operand B, float *C, int ldc, size_t part,
-                                                int epi, const float *bias, const float *mask, int *timeout) {
+                                                int epi, const float *bias, const float *mask, int *timeout,
+                                                long long wait_limit) {
   extern __shared__ __align__(16) unsigned char tc_raw[];
   __shared__ int s_fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(int M, int N, int K, Oper
   auto collect = [&](int steps) {
     if (tid == 0)
       for (int s = 0; s < 2; ++s)
-        if (uses[s] > 0 && !t5::mbar_wait(t5::smem_u32(&mbar[s]), (uses[s] - 1) & 1)) s_fail = 1;
+        if (uses[s] > 0 && !t5::mbar_wait(t5::smem_u32(&mbar[s]), (uses[s] - 1) & 1, wait_limit)) s_fail = 1;
     __syncthreads();
     t5::fence_after();
     if (s_fail) return false;
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(int M, int N, int K, Oper
     const int s = it & 1;
     unsigned char *stg = base + s * STAGE;
     if (uses[s] > 0) {  // the MMAs that last read this stage must have completed
-      if (tid == 0 && !t5::mbar_wait(t5::smem_u32(&mbar[s]), (uses[s] - 1) & 1)) s_fail = 1;
+      if (tid == 0 && !t5::mbar_wait(t5::smem_u32(&mbar[s]), (uses[s] - 1) & 1, wait_limit)) s_fail = 1;
       __syncthreads();
       if (s_fail) {
         ok = false;
@@ -333,8 +334,11 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(int M, int N, int K, Oper
       for (int q = 0; q < 32; ++q) out[row * LDO + 64 * h + 32 * (warp >> 2) + q] = sum[h][q];
   }
   __syncthreads();
-  if (ok) {
-    float *Cz = C + blockIdx.z * part;
+  float *Cz = C + blockIdx.z * part;
+  if (!ok) {
+    for (int e = tid; e < MT * NT; e += TC_THREADS)
+      if (m0 + e / NT < M && n0 + e % NT < N) Cz[(size_t)(m0 + e / NT) * ldc + n0 + e % NT] = __int_as_float(0x7fffffff);
+  } else {
 #pragma unroll 4
     for (int r = warp * 16; r < warp * 16 + 16; ++r) {
       const int m = m0 + r;
@@ -468,9 +472,11 @@ struct nqg_mlp {
   int *d_idx = nullptr;
   double *d_loss = nullptr;
   float *d_parts = nullptr;  // parts of a gradient's product (see k_parts)
-  int *timeout = nullptr;    // host memory: set by a kernel whose MMA wait gave up
+  // host memory, set by kernels whose MMA wait gave up: on the model's own stream, on a caller's
+  int *timeout = nullptr;
+  long long wait_limit = t5::WAIT_LIMIT;
   long step = 0;
-  cudaStream_t stream = nullptr;
+  cudaStream_t stream = nullptr, own_stream = nullptr;  // where launches go; the model's own
   std::string err;
 };
 
@@ -542,8 +548,9 @@ template <int NB, int NT>
 void launch_tc(nqg_mlp *m, int M, int N, int K, const Operand &A, const Operand &B, float *C, int ldc, int epi,
                const float *bias, const float *mask, int parts) {
   const dim3 grid((N + NT - 1) / NT, (M + MT - 1) / MT, parts);
+  int *const report = m->timeout + (m->stream == m->own_stream ? 0 : 1);
   k_mlp_tc<NB, NT><<<grid, TC_THREADS, tc_smem(NB, NT), m->stream>>>(M, N, K, A, B, C, ldc, (size_t)M * N, epi, bias, mask,
-                                                                     m->timeout);
+                                                                     report, m->wait_limit);
 }
 
 // B FP32 (NB 3) or BF16 (NB 1).
@@ -592,9 +599,11 @@ void backward(nqg_mlp *m, int rows) {
   }
 }
 
-int mma_status(nqg_mlp *m) {
-  if (!*(volatile int *)m->timeout) return NQG_OK;
-  *(volatile int *)m->timeout = 0;
+// `which`: 0 the model's own stream, 1 callers' streams.
+int mma_status(nqg_mlp *m, int which = 0) {
+  volatile int *t = m->timeout + which;
+  if (!*t) return NQG_OK;
+  *t = 0;
   m->err = "a tensor-core wait timed out";
   return NQG_ERR_TIMEOUT;
 }
@@ -613,6 +622,7 @@ extern "C" int nqg_mlp_create(int nsizes, const int *sizes, unsigned long long s
     delete m;
     return NQG_ERR_CUDA;
   }
+  m->own_stream = m->stream;
   std::mt19937_64 rng(seed);
   for (int l = 0; l < m->L; ++l) {
     const int in = sizes[l], o = sizes[l + 1];
@@ -647,8 +657,8 @@ extern "C" int nqg_mlp_create(int nsizes, const int *sizes, unsigned long long s
   if (cudaMalloc(&m->d_loss, sizeof(double)) != cudaSuccess) return NQG_ERR_CUDA;
   // parts > 1 only while parts x tiles <= SM_COUNT
   if (cudaMalloc(&m->d_parts, (size_t)SM_COUNT * MT * 64 * sizeof(float)) != cudaSuccess) return NQG_ERR_CUDA;
-  if (cudaHostAlloc(&m->timeout, sizeof(int), cudaHostAllocDefault) != cudaSuccess) return NQG_ERR_CUDA;
-  *m->timeout = 0;
+  if (cudaHostAlloc(&m->timeout, 2 * sizeof(int), cudaHostAllocDefault) != cudaSuccess) return NQG_ERR_CUDA;
+  m->timeout[0] = m->timeout[1] = 0;
   if (cudaStreamSynchronize(m->stream) != cudaSuccess) return NQG_ERR_CUDA;
   *out = m;
   return NQG_OK;
@@ -722,6 +732,15 @@ extern "C" int nqg_mlp_forward_device(nqg_mlp *m, int rows, const float *d_x, fl
   MQ(cudaStreamSynchronize(st));
   return mma_status(m);
 }
+
+extern "C" int nqg_mlp_set_wait_limit(nqg_mlp *m, long long polls) {
+  if (!m) return NQG_ERR_ARG;
+  m->wait_limit = polls == 0 ? t5::WAIT_LIMIT : std::clamp(polls, 0ll, t5::WAIT_LIMIT);
+  return NQG_OK;
+}
+
+// What forwards on callers' streams have reported since the last call.
+extern "C" int nqg_mlp_stream_status(nqg_mlp *m) { return m ? mma_status(m, 1) : NQG_ERR_ARG; }
 
 // Host-buffer variant of nqg_mlp_forward_device.
 extern "C" int nqg_mlp_forward(nqg_mlp *m, int rows, const float *x, float *logits) {

@@ -106,8 +106,8 @@ __device__ __forceinline__ bool mbar_test(uint32_t mbar, uint32_t parity) {
   return ok != 0;
 }
 // Bounded wait for phase `parity` of an mbarrier; false on timeout.
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-  for (long long it = 0; it < WAIT_LIMIT; ++it)
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, long long limit = WAIT_LIMIT) {
+  for (long long it = 0; it < limit; ++it)
     if (mbar_test(mbar, parity)) return true;
   return false;
 }
