@@ -220,8 +220,9 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(int M, int N, int K, Oper
   for (int h = 0; h < NT / 64; ++h)
 #pragma unroll
     for (int q = 0; q < 32; ++q) sum[h][q] = 0.f;
-  // adds what the accumulators hold after `steps` K steps, once the MMAs have completed; every thread calls
-  auto collect = [&](int steps) {
+  // adds what the accumulators hold, once the MMAs have completed; every thread calls
+  static_assert(KT / 16 >= NACC, "a chunk has written every accumulator");
+  auto collect = [&]() {
     if (tid == 0)
       for (int s = 0; s < 2; ++s)
         if (uses[s] > 0 && !t5::mbar_wait(t5::smem_u32(&mbar[s]), (uses[s] - 1) & 1, wait_limit)) s_fail = 1;
@@ -232,7 +233,6 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(int M, int N, int K, Oper
     for (int h = 0; h < NT / 64; ++h)
 #pragma unroll 1
       for (int g = NACC; g >= 0; --g) {
-        if (g < NACC && g >= steps) continue;
         uint32_t v[32];
         t5::tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g * NT + 64 * h + 32 * (warp >> 2)), v);
 #pragma unroll
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(int M, int N, int K, Oper
     const bool more = ch + (int)gridDim.z < nchunk;
     if (more) load(ch + gridDim.z);
     if (it % SEG == SEG - 1 || !more)
-      if (!collect((it % SEG + 1) * (KT / 16))) {
+      if (!collect()) {
         ok = false;
         break;
       }
