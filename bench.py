@@ -59,9 +59,8 @@ WS_THRESHOLD = 1.5  # logit above which a constraint is proposed (swept 0..5: 1.
 TRAIN_EPOCHS = 60   # swept 20 / 60: 60 epochs (10 s) cut warm-start drops from 5.0 to 2.9 per QP
 CPU_SAMPLE_PER_PROC = 48
 # DRAM bytes (read + write) of one batch-kernel launch on 4096 warm-started QPs
-# of this family, from a single-pass ncu capture:
-# profiles/ncu_batch_solve_panel_kernels.md
-NCU_BATCH_TRAFFIC = 3_423_730_944 + 2_593_120_768
+# of this family, from a single-pass ncu capture
+NCU_BATCH_TRAFFIC = 3_459_575_552 + 2_581_873_920
 # LBL section: K = [H A^T; A -1e-8 I], H 3D 7-point Laplacian on 64^3, A 20000 x n, 6 N(0,1) per row
 GRID, MCON, PER_ROW, DELTA, SEED = 64, 20000, 6, 1e-8, 0
 TARGET_RELRES = 1e-10
