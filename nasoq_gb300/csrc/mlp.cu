@@ -147,14 +147,14 @@ __device__ __forceinline__ void load_unit(const Operand &o, int r, int k0, int K
 __host__ __device__ constexpr int tc_stage(int nb, int nt) { return 3 * A_PART + nb * nt * 128; }
 __host__ __device__ constexpr int tc_smem(int nb, int nt) { return 2 * tc_stage(nb, nt) + 1024 + 64; }
 
-// Entry (r, k) of an FP32 operand.
+// Entry (r, k) of an operand.
 __device__ __forceinline__ float value(const Operand &o, int r, int k) {
+  if (o.bf) return __bfloat162float(o.bf[(size_t)r * o.ld + k]);
   return o.across ? o.p[r + (size_t)k * o.ld] : o.p[(size_t)r * o.ld + k];
 }
-// Entry (m, n) of part z of nz of a product of two FP32 operands, by FP32
-// multiply-adds.  A result that is not a number is formed again by it: an
-// infinity times a part of the other value that happens to be zero is no
-// product of the values.
+// Entry (m, n) of part z of nz of a product, by FP32 multiply-adds.  A result
+// that is not a number is formed again by it: an infinity times a part of the
+// other value that happens to be zero is no product of the values.
 __device__ __noinline__ float plain_entry(const Operand &A, const Operand &B, int m, int n, int K, int z, int nz) {
   float s = 0.f;
 #pragma unroll 1
@@ -326,14 +326,27 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(int M, int N, int K, Oper
   // global rows are written in whole lines
   float *out = reinterpret_cast<float *>(base);
   constexpr int LDO = NT + 1;
+  bool nan = false;
   if (ok) {
     const int row = (warp & 3) * 32 + lane;
 #pragma unroll
     for (int h = 0; h < NT / 64; ++h)
 #pragma unroll
-      for (int q = 0; q < 32; ++q) out[row * LDO + 64 * h + 32 * (warp >> 2) + q] = sum[h][q];
+      for (int q = 0; q < 32; ++q) {
+        out[row * LDO + 64 * h + 32 * (warp >> 2) + q] = sum[h][q];
+        nan |= sum[h][q] != sum[h][q];
+      }
   }
-  __syncthreads();
+  // a loop of its own: as a call in the epilogue's it cost 8 us of 65 (4096-row forward)
+  if (__syncthreads_or(nan)) {
+#pragma unroll 1
+    for (int e = tid; e < MT * NT; e += TC_THREADS) {
+      const int m = m0 + e / NT, n = n0 + e % NT;
+      float &v = out[(e / NT) * LDO + e % NT];
+      if (m < M && n < N && v != v) v = plain_entry(A, B, m, n, K, blockIdx.z, gridDim.z);
+    }
+    __syncthreads();
+  }
   float *Cz = C + blockIdx.z * part;
   if (!ok) {
     for (int e = tid; e < MT * NT; e += TC_THREADS)
@@ -348,7 +361,6 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(int M, int N, int K, Oper
         const int n = n0 + h + lane;
         if (n >= N) continue;
         float v = out[r * LDO + h + lane];
-        if (NB == 3 && v != v) v = plain_entry(A, B, m, n, K, blockIdx.z, gridDim.z);
         if (epi == EPI_BIAS_RELU) v = fmaxf(v + bias[n], 0.f);
         else if (epi == EPI_BIAS) v = v + bias[n];
         else if (epi == EPI_RELU_MASK) v = mask[(size_t)m * ldc + n] > 0.f ? v : 0.f;

@@ -56,3 +56,34 @@ def test_infinite_input_in_gradients(rows):
     # sums of `rows` FP32 terms
     assert np.abs(gw[~odd] - want[~odd]).max() <= 2.0 ** -23 * (rows + 33) * np.linalg.norm(want[~odd])
     m.close()
+
+
+def test_infinite_weight():
+    """A weight of infinity times an activation of few bits is an infinity (NaN
+    for 0), in the logits and in the gradient of the layer below."""
+    m = nq.MLP((32, 70), seed=1)
+    w = np.ones((70, 32), np.float32)
+    w[5, 3] = np.inf
+    m.set_weights(w.ravel(), np.zeros(70, np.float32))
+    x = np.ones((5, 32), np.float32)
+    x[:, 3] = [1.0, -2.0, 0.0, 0.1, -np.inf]
+    z = m.forward(x)
+    assert np.array_equal(z[:, 5], np.array([np.inf, -np.inf, np.nan, np.inf, -np.inf], np.float32), equal_nan=True)
+    assert np.isfinite(np.delete(z[:4], 5, axis=1)).all()
+    m.close()
+
+    inp, hid, out, rows = 16, 24, 70, 4
+    m = nq.MLP((inp, hid, out), seed=1)
+    w2 = np.ones((out, hid), np.float32)
+    w2[6, 2] = w2[65, 11] = np.inf
+    m.set_weights(np.concatenate([np.ones(hid * inp, np.float32), w2.ravel()]), np.zeros(hid + out, np.float32))
+    x = np.full((rows, inp), 0.5, np.float32)  # every hidden unit is 8
+    y = np.ones((rows, out), np.float32)
+    y[:, 6] = 0.0
+    assert (m.forward(x)[:, [6, 65]] == np.inf).all()
+    _, gw, _ = m.loss_grad(x, y)
+    g1 = gw[:hid * inp].reshape(hid, inp)
+    assert (g1[2] == np.inf).all()  # dlogit 1 / rows there
+    assert np.isnan(g1[11]).all()   # dlogit 0
+    assert np.isfinite(np.delete(g1, [2, 11], axis=0)).all()
+    m.close()
