@@ -48,8 +48,7 @@ def _both(monkeypatch, make):
 
 
 def _agree(out, growth, kappa):
-    (x, steps), (xg, steps_g) = out
-    assert steps == steps_g
+    x, xg = out[0][0], out[1][0]
     # the bar of the comparisons with the reference's solutions: pivots of 1e-9 (the regularization) are taken
     # inside their supernode, the growth of up to 1e9 amplifies the rounding of either solve
     tol = max(1e-9, 1e-14 * kappa, 1e-15 * growth)
@@ -81,6 +80,8 @@ def test_refinement(restarts, steps, tol, refine_only, dense, monkeypatch):
     full[i, cols] = v
     full = full + np.tril(full, -1).T
     _agree(out, growth, np.linalg.cond(full))
+    # with hidden constraints the last step's residual is at rounding level, here it is not
+    assert out[0][1] == out[1][1]
     if tol == 1e6:  # the first residual is below it
         assert out[0][1] == 0
     elif tol == 1e-15:
